@@ -206,8 +206,10 @@ cudaError_t row5_device_table(const uint32_t **out) {
     return cudaSuccess;
 }
 
-// Largest staged scene: the block's dynamic shared memory stays below this.
-constexpr size_t kMaxDynSmem = 200 * 1024;
+// Largest staged scene in bytes (about 1,600 boxes): it shares the block's
+// dynamic shared memory with the warps' scratch, within 200 KB.
+constexpr size_t kMaxSceneBytes = 135008;
+static_assert(kMaxSceneBytes + sizeof(mrpop::WarpScratch) * mrpop::kWarpsPerBlock <= 200 * 1024, "scene and scratch");
 
 }  // namespace
 
@@ -251,7 +253,7 @@ mrpop_status mrpop_scene_create(const mrpop_scene_desc *desc, mrpop_scene **out)
     mrpop::SceneCounts c{(int)desc->num_spheres, (int)desc->num_capsules, (int)desc->num_z_capsules,
                          (int)desc->num_cuboids, (int)desc->num_z_cuboids};
     const mrpop::SceneLayout L = mrpop::scene_layout(c);
-    if ((size_t)L.total * sizeof(float4) + block_scratch_bytes() > kMaxDynSmem)
+    if ((size_t)L.total * sizeof(float4) > kMaxSceneBytes)
         return fail(MRPOP_ERR_UNSUPPORTED, "scene_create: scene too large to stage in shared memory (" +
                                                std::to_string(L.total * 16) + " bytes)");
     std::vector<float4> h((size_t)L.total);
@@ -450,9 +452,6 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
             r = std::fmax(r, std::sqrt((d.x - cx) * (d.x - cx) + (d.y - cy) * (d.y - cy) + (d.z - cz) * (d.z - cz)) + d.r);
         }
         p.grp[gi] = make_float4((float)cx, (float)cy, (float)cz, (float)(r * 1.001 + kCullMargin));
-        const SphereDef &ref = kApprox[grp_ref(gi)];
-        const double ox = cx - ref.x, oy = cy - ref.y, oz = cz - ref.z;
-        p.gofs[gi] = (float)(std::sqrt(ox * ox + oy * oy + oz * oz) * 1.001 + r * 1.001 + kCullMargin);
     }
     // the hand group's three parts (bits of hand_part over spheres kHandFirst..)
     for (int s = 0; s < kHandParts; s++) {
@@ -482,22 +481,23 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
 }
 
 // A 128-byte head with the two work counters, then per edge: flag words,
-// candidate masks, reference-sphere bounds and segment state.  The kernels
+// candidate masks, arm-pair joints and segment state.  The kernels
 // stage the flag words as 32-bit pairs for up to 4 arms, in the first half
 // of their slice (which keeps its 64-bit size).
 int robotset_arms(const mrpop_robotset *robots) { return robots ? robots->n_arms : 0; }
 
 void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int A) {
+    (void)A;
     const int spl = g > 32 ? 2 : 1;
     const size_t flag_bytes = (size_t)n_edges * 32 * spl * 2 * sizeof(uint64_t);
     const size_t mask_bytes = (size_t)n_edges * 2 * sizeof(uint64_t);
-    const size_t bound_bytes = (size_t)n_edges * A * kRefSpheres * sizeof(float4);
+    const size_t pair_bytes = (size_t)n_edges * kPairSlots * sizeof(uint16_t);
     p.work = (unsigned long long *)scratch;
     char *b = (char *)scratch + kSplitScratchHead;
     p.sflags = (uint64_t *)b;
     p.smasks = (uint64_t *)(b + flag_bytes);
-    p.sbounds = (float4 *)(b + flag_bytes + mask_bytes);
-    p.snseg = (int32_t *)(b + flag_bytes + mask_bytes + bound_bytes);
+    p.spairs = (uint16_t *)(b + flag_bytes + mask_bytes);
+    p.snseg = (int32_t *)(b + flag_bytes + mask_bytes + pair_bytes);
     p.sdone = p.snseg + n_edges;
 }
 

@@ -12,7 +12,7 @@
 //                pairs, each screened one pair per lane against swept bounds of
 //                the warp's samples first; the result is a per-(arm, joint)
 //                flag word and per-sample sphere counts, staged in HBM with the
-//                swept bounds for the narrow kernel.
+//                arm pairs those bounds connect for the narrow kernel.
 //   decision     per warp: shuffle reductions give the edge totals; the
 //                reference's proportional 4g-thread split (utils.cuh:476-517)
 //                is evaluated exactly to pick the samples that get a detailed
@@ -82,7 +82,7 @@ static __device__ unsigned long long *g_dev_phase;
 constexpr int kWarpsPerBlock = 6;
 constexpr int kMaxArms = 5;
 constexpr int kMaxDof = 7 * kMaxArms;
-constexpr int kCrossStash = 16;        // per-lane arm-vs-arm candidate spheres
+constexpr int kCrossStash = 8;         // per-lane arm-vs-arm candidate spheres
 constexpr float kCullMargin = 1e-3f;   // metres added to every bounding radius
 constexpr float kApproxMaxR = 0.176f;  // largest broad-phase sphere radius
 
@@ -115,9 +115,6 @@ __host__ __device__ inline SceneLayout scene_layout(const SceneCounts &c) {
     return l;
 }
 
-// Approx spheres whose swept bounds the narrow phase reuses: 0..8 (the
-// reference sphere of every detailed sub-group, see grp_ref).
-constexpr int kRefSpheres = 9;
 // Segmented rules: segments checked by rounds of the split kernels before the
 // fused kernel takes the remaining ones.
 constexpr int kSegRounds = 4;
@@ -144,11 +141,10 @@ struct EdgeParams {
     unsigned long long *phase;  // phase timers (MRPOP_PHASE_TIMERS builds only)
     uint64_t *sflags;           // split pipeline: per-sample {env, self} flag words (32-bit for <= 4 arms)
     uint64_t *smasks;           // split pipeline: per-edge {env, self} candidate masks
-    float4 *sbounds;            // split pipeline: per-edge swept reference-sphere bounds [A][kRefSpheres]
+    uint16_t *spairs;           // split pipeline: per-edge arm-pair joints [SPL][num_pairs(A)] (kPairSlots reserved)
     int32_t *snseg;             // segmented rules: per-edge segment count (-1: too many), from segment 0
     int32_t *sdone;             // segmented rules: per-edge verdict written
     unsigned long long *work;   // split kernels: next-edge counters {broad, narrow}, zero before each launch
-    float gofs[11];             // sub-group g: |group centre - reference sphere centre| + group radius
     float4 grp[11];             // detailed sub-group bounds in their joint frame (+margin)
     float4 hsub[3];             // bounds of the hand group's three parts in the joint-7 frame (+margin)
     const uint32_t *row5;       // forearm-hand rows table (kRow5N6 x kRow5N7 bits), or nullptr
@@ -161,13 +157,6 @@ struct WarpScratch {
     float base[kMaxDof];   // segment start (accumulated for CONNECT)
     float stepg[kMaxDof];  // per-sample step (delta/g or vec/g)
     float delta[kMaxDof];  // per-segment step (B-spline / shortcut accumulation)
-    // bound of the centres of approx spheres 0..kRefSpheres-1 of each arm over
-    // every sample of the segment ({centre, radius}, sphere radius excluded);
-    // written by the broad phase, read by the narrow phase's arm-vs-arm screen
-    float4 rsw[kMaxArms][kRefSpheres];
-    // sub-group bounds over the segment's samples derived from rsw (the
-    // narrow phase's arm-vs-arm screen)
-    float4 gbd[kMaxArms][11];
     union {
         struct {
             float4 swept[kMaxArms][kNumApprox]; // per-arm swept bound of each approx sphere
@@ -177,7 +166,11 @@ struct WarpScratch {
         struct {
             union {
                 float stash[kDetRows][3][32];        // first sphere of each detailed self row
-                float cstash[kCrossStash][4][32];    // arm-vs-arm candidates {x, y, z, r}
+                struct {                             // arm-vs-arm test of one arm pair
+                    float gc[11][3][32];             // the upper arm's sub-group centres
+                    float xs[kCrossStash][4][32];    // the lower arm's candidate spheres {x, y, z, r} ...
+                    uint32_t xm[kCrossStash][32];    // ... and the upper arm's sub-groups each can reach
+                } cross;
             };
         } lanes;
     };
@@ -339,8 +332,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // sphere radius + cull margin.  If the sphere touches something at any of the
 // samples, its swept bound touches it too (the margin covers FP rounding).
 __device__ __forceinline__ void fk_approx_lane(const float *base12, const WarpScratch &W, int rule, int seg,
-                                                   int qarm, int k, float (*dst)[3][32], int lane, float4 *swept,
-                                                   float4 *rsw, bool merge) {
+                                                   int qarm, int k, float (*dst)[3][32], int lane, float4 *swept) {
     float q[7];
     sample_q(W, rule, seg, qarm, k, q);
     ArmSpheres s;
@@ -382,22 +374,6 @@ __device__ __forceinline__ void fk_approx_lane(const float *base12, const WarpSc
             const float dx = bx - ax, dy = by - ay, dz = bz - az;
             swept[i] = make_float4(0.5f * (ax + bx), 0.5f * (ay + by), 0.5f * (az + bz),
                                    0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + c_approx[i].w + kCullMargin);
-        }
-    }
-    __syncwarp();
-    // bounds of the reference spheres' centres for the narrow phase (sphere
-    // radius and margin taken off again, +1e-6 m for the rounding), grown
-    // over the segment's earlier samples when merging
-    if (lane < kRefSpheres) {
-        const float4 sv = swept[lane];
-        const float hd = sv.w - c_approx[lane].w - kCullMargin + 1e-6f;
-        if (!merge) {
-            rsw[lane] = make_float4(sv.x, sv.y, sv.z, hd);
-        } else {
-            const float4 o = rsw[lane];
-            const float ex = sv.x - o.x, ey = sv.y - o.y, ez = sv.z - o.z;
-            const float d = sqrtf(ex * ex + ey * ey + ez * ez) * 1.0001f;
-            rsw[lane] = make_float4(o.x, o.y, o.z, fmaxf(o.w, d + hd) + 1e-6f);
         }
     }
     __syncwarp();
@@ -490,6 +466,55 @@ __device__ __forceinline__ uint32_t env_mask_approx(const float4 *S, const Scene
     return m;
 }
 
+// Arm pairs (a < b) in order: pair index of (a, b), and the count.
+__host__ __device__ __forceinline__ constexpr int pair_index(int a, int b, int A) {
+    return a * (2 * A - a - 1) / 2 + (b - a - 1);
+}
+__host__ __device__ __forceinline__ constexpr int num_pairs(int A) { return A * (A - 1) / 2; }
+
+// Arm pair p (pair_index order): its lower and upper arm.
+template <int A>
+__host__ __device__ __forceinline__ constexpr void pair_arms(int p, int &a, int &b) {
+    a = 0;
+    while (p >= A - 1 - a) {
+        p -= A - 1 - a;
+        a++;
+    }
+    b = a + 1 + p;
+}
+
+// pair_arms inverts pair_index for every pair of up to 5 arms
+template <int A>
+constexpr bool pair_order_round_trips() {
+    for (int p = 0; p < num_pairs(A); p++) {
+        int a = 0, b = 0;
+        pair_arms<A>(p, a, b);
+        if (!(0 <= a && a < b && b < A) || pair_index(a, b, A) != p) return false;
+    }
+    return true;
+}
+static_assert(pair_order_round_trips<2>() && pair_order_round_trips<3>() && pair_order_round_trips<4>() &&
+                  pair_order_round_trips<5>(),
+              "arm pair order");
+
+// Every detailed sphere lies inside an approx sphere of its joint grown by
+// 0.9 mm (0.6 mm in fact), so two arms' joints whose approx spheres' swept
+// bounds (which carry kCullMargin each) do not meet cannot collide.
+constexpr bool approx_cover_detailed() {
+    for (int i = 0; i < kNumDet; i++) {
+        bool in = false;
+        for (int a = 0; a < kNumApprox; a++) {
+            if (approx_joint(a) != det_joint(i)) continue;
+            const double x = (double)kDet[i].x - kApprox[a].x, y = (double)kDet[i].y - kApprox[a].y,
+                         z = (double)kDet[i].z - kApprox[a].z, r = (double)kApprox[a].r + 9e-4 - kDet[i].r;
+            in = in || (r > 0.0 && x * x + y * y + z * z <= r * r);
+        }
+        if (!in) return false;
+    }
+    return true;
+}
+static_assert(kCullMargin >= 1e-3f && approx_cover_detailed(), "approx spheres cover the detailed ones");
+
 // Broad-phase intra-arm rows (panda_multi_geometry.cuh:133-139) as 21 pairs.
 static __constant__ uint8_t c_intra_pairs[21][2] = {
     {0, 5}, {0, 6}, {0, 7}, {0, 8}, {0, 9}, {0, 10}, {1, 5}, {1, 6}, {1, 7}, {1, 8}, {1, 9},
@@ -522,11 +547,12 @@ __device__ __forceinline__ uint32_t intra_flags(const float (*sp)[3][32], const 
 
 template <int A>
 __device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W, const float4 *S,
-                                             const SceneLayout &L, int seg, int k, bool merge, uint64_t &envw,
-                                             uint64_t &selfw) {
+                                             const SceneLayout &L, int seg, int k, uint64_t &envw, uint64_t &selfw,
+                                             uint32_t &pm) {
     const int lane = threadIdx.x & 31;
     envw = 0;
     selfw = 0;
+    pm = 0;
     const bool do_env = P.flags & kEnvBit, do_self = P.flags & kSelfBit;
     auto &cur = W.broad.cur;
     auto &low = W.broad.low;
@@ -534,7 +560,7 @@ __device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W
     for (int b = 0; b < A; b++) {
         MRPOP_PHASE_START();
         float4 *sw = W.broad.swept[b];
-        fk_approx_lane(P.base[b], W, P.rule, seg, P.single ? 0 : b, k, cur, lane, sw, W.rsw[b], merge);
+        fk_approx_lane(P.base[b], W, P.rule, seg, P.single ? 0 : b, k, cur, lane, sw);
         MRPOP_PHASE(P, 0);
         if (do_env) {
             const uint32_t m = env_mask_approx(S, L, P.sc, cur, lane, sw);
@@ -568,8 +594,8 @@ __device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W
                                                   near3(swa[i].x, swa[i].y, swa[i].z, sw[j], swa[i].w));
             }
             if (!(bal[0] | bal[1] | bal[2] | bal[3])) continue;
-            fk_approx_lane(P.base[a], W, P.rule, seg, a, k, low, lane, nullptr, nullptr, false);
-            uint32_t am = 0;
+            fk_approx_lane(P.base[a], W, P.rule, seg, a, k, low, lane, nullptr);
+            uint32_t am = 0, ja = 0, jb = 0;
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 uint32_t q = bal[r];
@@ -577,12 +603,15 @@ __device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W
                     const int t = 32 * r + __ffs(q) - 1;
                     q &= q - 1;
                     const int i = t / kNumApprox, j = t - kNumApprox * i;
+                    ja |= 1u << approx_joint(i);
+                    jb |= 1u << approx_joint(j);
                     if (hit_sphere_sphere(low[i][0][lane], low[i][1][lane], low[i][2][lane], c_approx[i].w,
                                           cur[j][0][lane], cur[j][1][lane], cur[j][2][lane], c_approx[j].w))
                         am |= 1u << approx_joint(i);
                 }
             }
             selfw |= (uint64_t)am << (8 * a);
+            if (lane == pair_index(a, b, A)) pm = ja | jb << 8;
         }
         MRPOP_PHASE(P, 3);
     }
@@ -826,13 +855,22 @@ __device__ __forceinline__ bool row5_apart(const uint32_t *tab, float q6, float 
     return (__ldg(tab + (cell >> 5)) >> (cell & 31)) & 1u;
 }
 
-// Per-lane state of the lane-parallel detailed check of one arm.
+// Per-lane state of the lane-parallel detailed check of one arm.  A lane with
+// em = rm = 0 takes no further part: it has no tests here, its sample has hit,
+// or a lower lane's sample has (only the first colliding sample is reported).
 struct LaneCtx {
     uint32_t em;  // env-flagged joints
     uint32_t rm;  // flagged detailed self rows
     int quirk;
     bool hit;
+    __device__ __forceinline__ void set_hit() {
+        hit = true;
+        em = rm = 0;
+    }
 };
+
+// Lanes 0..lane: a hit on any of them settles the lane's sample.
+__device__ __forceinline__ uint32_t lanes_upto(int lane) { return (2u << lane) - 1u; }
 
 // Joint j of one arm, frame T: env tests of an env-flagged joint, stash of the
 // first spheres of flagged rows, and the row tests whose targets are here
@@ -840,17 +878,17 @@ struct LaneCtx {
 __device__ __forceinline__ void lane_env(int j, const EdgeParams &P, const Xf &T, LaneCtx &c, const float4 *S,
                                          const SceneLayout &L) {
     // every lane takes part in the env screening (warp-wide votes inside)
-    if (__any_sync(kFull, !c.hit && (c.em >> j & 1u))) {
+    if (__any_sync(kFull, c.em >> j & 1u)) {
 #pragma unroll 1
         for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++)
-            if (env_group_warp(S, L, P.sc, T, g, P.grp[g], !c.hit && (c.em >> j & 1u))) c.hit = true;
+            if (env_group_warp(S, L, P.sc, T, g, P.grp[g], c.em >> j & 1u)) c.set_hit();
     }
 }
 
 template <int A>
 __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &T, LaneCtx &c, WarpScratch &W,
                                           const float4 *det_tab, int lane) {
-    if (c.hit || !c.rm) return;
+    if (!c.rm) return;
     uint32_t m1 = c.rm & c_rows.jfirst[c.quirk][j];
     while (m1) {
         const int r = __ffs(m1) - 1;
@@ -918,7 +956,7 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
             }
         }
         if (h) {
-            c.hit = true;
+            c.set_hit();
             return;
         }
     }
@@ -929,7 +967,10 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
 // arm's chain is rebuilt in registers; env tests of env-flagged joints
 // (screened warp-wide per sub-group) and the intra-arm rows of self-flagged
 // joints run as the frames stream by (the first sphere of each row is stashed
-// until its targets come).  Returns true if a test fired.
+// until its targets come).  Once a lane's test has fired, the lanes above it
+// stop: random edges that collide mostly do so at their first samples, and
+// the rest of such an edge's tests is not needed.  Returns true if a test
+// fired.
 // ONE: only arm one_arm's chain (the arm-per-warp kernel).
 template <int A, bool ONE = false>
 __device__ __forceinline__ bool narrow_lane(const EdgeParams &P, WarpScratch &W, const float4 *S,
@@ -942,7 +983,7 @@ __device__ __forceinline__ bool narrow_lane(const EdgeParams &P, WarpScratch &W,
     MRPOP_PHASE_START();
 #pragma unroll 1
     for (int a = ONE ? one_arm : 0; a < (ONE ? one_arm + 1 : A); a++) {
-        if (__all_sync(kFull, c.hit || !(de || ds))) break;
+        if (!__any_sync(kFull, de || ds)) break;
         c.em = de ? (uint32_t)(envw >> (8 * a)) & 0xffu : 0u;
         const uint32_t sm = ds ? (uint32_t)(selfw >> (8 * a)) & 0xffu : 0u;
         c.rm = sm ? row_mask(sm, c.quirk != 0) : 0u;
@@ -951,7 +992,8 @@ __device__ __forceinline__ bool narrow_lane(const EdgeParams &P, WarpScratch &W,
             row5_apart(P.row5, sample_q1(W, P.rule, seg, qa + 5, k), sample_q1(W, P.rule, seg, qa + 6, k)))
             c.rm &= ~row5_rows(c.quirk);
         // the arm's chain is walked only if some lane has env or row tests on it
-        if (!__any_sync(kFull, !c.hit && (c.em | c.rm))) continue;
+        if (!__any_sync(kFull, c.em | c.rm)) continue;
+        const uint32_t before = __ballot_sync(kFull, c.hit);
         Xf T;
         load_base(T, P.base[a]);
 #pragma unroll 1
@@ -962,63 +1004,83 @@ __device__ __forceinline__ bool narrow_lane(const EdgeParams &P, WarpScratch &W,
             MRPOP_PHASE(P, 9);
             lane_rows<A>(j, P, T, c, W, det_tab, lane);
             MRPOP_PHASE(P, 10);
+            const uint32_t hb = __ballot_sync(kFull, c.hit);
+            if (hb != before) {
+                if (hb & lanes_upto(lane)) {
+                    c.em = c.rm = 0;
+                    de = ds = false;
+                }
+                if (!__any_sync(kFull, c.em | c.rm)) break;
+            }
         }
     }
     return c.hit;
 }
 
-// Arm a, joint j: stash the flagged spheres (index >= from) that can reach
-// bound bb, until the stash is full; `next` receives the first sphere left out.
-__device__ __forceinline__ void stash_joint(int j, const Xf &T, uint32_t sma, uint32_t qa, int from, int &n,
+// Lower arm, joint j (flagged for this lane): its spheres from index `from` on
+// that can reach one of the upper arm's sub-groups gb (bounds, centres in
+// W.lanes.cross.gc) go to the lane's stash with the sub-groups they reach;
+// `next` receives the first sphere left out when the stash is full.
+__device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf &T, uint32_t gb, int from, int &n,
                                             int &next, WarpScratch &W, int lane) {
-    if (next >= 0 || !(sma >> j & 1u) || det_first(j + 1) <= from) return;
+    auto &X = W.lanes.cross;
 #pragma unroll 1
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
-        if (!(qa >> g & 1u) || grp_first(g + 1) <= from) continue;
+        if (grp_first(g + 1) <= from) continue;
+        const float4 gl = P.grp[g];
+        const float3 gc = place_reg(T, gl);
+        uint32_t near = 0;
+        for (uint32_t m = gb; m; m &= m - 1) {
+            const int t = __ffs(m) - 1;
+            if (near3(gc.x, gc.y, gc.z, make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], P.grp[t].w),
+                      gl.w))
+                near |= 1u << t;
+        }
+        if (!near) continue;
 #pragma unroll 1
         for (int i = max(grp_first(g), from); i < grp_first(g + 1); i++) {
             const float4 sd = c_det[i];
             const float3 p = place_reg(T, sd);
+            uint32_t nm = 0;
+            for (uint32_t m = near; m; m &= m - 1) {
+                const int t = __ffs(m) - 1;
+                if (near3(p.x, p.y, p.z, make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], P.grp[t].w),
+                          sd.w))
+                    nm |= 1u << t;
+            }
+            if (!nm) continue;
             if (n == kCrossStash) {
                 next = i;
                 return;
             }
-            W.lanes.cstash[n][0][lane] = p.x;
-            W.lanes.cstash[n][1][lane] = p.y;
-            W.lanes.cstash[n][2][lane] = p.z;
-            W.lanes.cstash[n][3][lane] = sd.w;
+            X.xs[n][0][lane] = p.x;
+            X.xs[n][1][lane] = p.y;
+            X.xs[n][2][lane] = p.z;
+            X.xs[n][3][lane] = sd.w;
+            X.xm[n][lane] = nm;
             n++;
         }
     }
 }
 
-// Arm b, joint j: its spheres against the stashed spheres, by sub-group.
-__device__ __forceinline__ void probe_joint(int j, const EdgeParams &P, const Xf &T, uint32_t qb, int n, bool &hit,
-                                            WarpScratch &W, int lane) {
-    if (hit) return;
+// Upper arm, joint j: its spheres against the stashed spheres that reach their
+// sub-group.
+__device__ __forceinline__ void probe_joint(int j, const Xf &T, int n, bool &hit, WarpScratch &W, int lane) {
+    auto &X = W.lanes.cross;
 #pragma unroll 1
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
-        if (!(qb >> g & 1u)) continue;
-        const float4 gl = P.grp[g];
-        const float3 gc = place_reg(T, gl);
-        const float4 gb = make_float4(gc.x, gc.y, gc.z, gl.w);
-        uint32_t near = 0;
-        for (int e = 0; e < n; e++)
-            if (near3(W.lanes.cstash[e][0][lane], W.lanes.cstash[e][1][lane], W.lanes.cstash[e][2][lane], gb,
-                      W.lanes.cstash[e][3][lane]))
-                near |= 1u << e;
-        if (!near) continue;
+        uint32_t em = 0;
+        for (int e = 0; e < n; e++) em |= (X.xm[e][lane] >> g & 1u) << e;
+        if (!em) continue;
         bool h = false;
         for (int i = grp_first(g); i < grp_first(g + 1); i++) {
             const float4 sd = c_det[i];
             const float3 p = place_reg(T, sd);
-            uint32_t m = near;
-            while (m) {
+            for (uint32_t m = em; m; m &= m - 1) {
                 const int e = __ffs(m) - 1;
-                m &= m - 1;
                 // sphere_1 = the lower arm's sphere (panda_four.cuh:441-443)
-                h |= hit_sphere_sphere(W.lanes.cstash[e][0][lane], W.lanes.cstash[e][1][lane],
-                                       W.lanes.cstash[e][2][lane], W.lanes.cstash[e][3][lane], p.x, p.y, p.z, sd.w);
+                h |= hit_sphere_sphere(X.xs[e][0][lane], X.xs[e][1][lane], X.xs[e][2][lane], X.xs[e][3][lane], p.x,
+                                       p.y, p.z, sd.w);
             }
         }
         if (h) {
@@ -1028,88 +1090,79 @@ __device__ __forceinline__ void probe_joint(int j, const EdgeParams &P, const Xf
     }
 }
 
-// Joint of detailed sub-group g.
-__device__ __forceinline__ constexpr int grp_joint(int g) { return g < 5 ? g : g < 8 ? 5 : g < 9 ? 6 : 7; }
-// Reference approx sphere of sub-group g: an approx sphere on the same joint
-// (the nearest one for the hand), so that the group's centre is at a fixed
-// distance from it (EdgeParams::gofs adds that distance and the group radius).
-__host__ __device__ __forceinline__ constexpr int grp_ref(int g) {
-    return g < 5 ? g : g < 8 ? 5 : g < 9 ? 6 : g < 10 ? 7 : 8;
+// Sub-groups of the joints in jm.
+__device__ __forceinline__ uint32_t joint_groups(uint32_t jm) {
+    return (jm & 0x1fu) | (jm >> 5 & 1u) * 0xe0u | (jm >> 6 & 1u) << 8 | (jm >> 7 & 1u) * 0x600u;
 }
 
-// Arm pairs (a < b) in order: pair index of (a, b), and the count.
-__host__ __device__ __forceinline__ constexpr int pair_index(int a, int b, int A) {
-    return a * (2 * A - a - 1) / 2 + (b - a - 1);
-}
-__host__ __device__ __forceinline__ constexpr int num_pairs(int A) { return A * (A - 1) / 2; }
-
-// Arm-vs-arm detailed test (panda_four.cuh:415-453) of this lane's sample;
-// every lane of the warp calls it, lanes with act set take part.  For each arm
-// pair (a, b) the 121 sub-group pairs are screened warp-wide, one per lane,
-// with bounds over the segment's samples (the swept bound of the group's
-// reference approx sphere, W.rsw, grown by EdgeParams::gofs; groups of a
-// restricted to joints some active lane has self-flagged).  Pairs with no
-// surviving group pair are skipped by the whole warp.  Otherwise each active
-// lane stashes arm a's flagged spheres of the surviving groups that can reach
-// arm b's bound (chunks of kCrossStash) and streams arm b's surviving groups
-// against them.  Returns true if a test fired.
-// SEL: only the arm pairs whose bit (pair_index) is set in `pairs`.
-template <int A, bool SEL = false>
-__device__ __forceinline__ bool cross_swept(const EdgeParams &P, WarpScratch &W, int seg, int k, uint64_t selfw,
-                                            bool act, uint32_t pairs = 0) {
+// Arm-vs-arm detailed test (panda_four.cuh:415-453) of arms a < b for this
+// lane's sample; every lane of the warp calls it.  sma: the lane's self-flagged
+// joints of arm a to test (0: the lane only keeps the others company), jb: the
+// joints of arm b.  Both are already cut to the joints that some approx sphere
+// pair's swept bounds connect in these 32 samples (the broad phase's screen):
+// a joint's detailed spheres lie inside its approx spheres but for 0.6 mm, and
+// those bounds carry 1 mm each.  Arm b's sub-group centres are placed first;
+// arm a's spheres are then tested against them by sub-group and one by one,
+// so that only spheres that can reach arm b are stashed (most lanes stash
+// none, and arm b's chain is walked again only if some lane did).  Returns
+// true if a test fired.
+// Bound by instruction issue.  Against one that screened all 121 sub-group
+// pairs of every arm pair and stashed every flagged sphere 16 at a time (with
+// the lanes above a hit going on): 262144 5-arm edges x 64 samples 11.90 ->
+// 10.26 ms, 65536 shortcut edges 7.36 -> 6.37 ms, 128 uneven instances 15.4 ->
+// 12.5 ms, 300 5-arm extend checks 120 -> 104 us.
+__device__ __forceinline__ bool cross_pair(const EdgeParams &P, WarpScratch &W, int seg, int k, int a, int b,
+                                           uint32_t sma, uint32_t jb) {
     const int lane = threadIdx.x & 31;
-    bool hit = false;
+    const uint32_t uj = __reduce_or_sync(kFull, sma);
+    if (!uj) return false;
+    const int top_a = 31 - __clz(uj), top_b = 31 - __clz(jb);
+    const uint32_t gb = joint_groups(jb);
+    {
+        Xf T;
+        load_base(T, P.base[b]);
 #pragma unroll 1
-    for (int a = 0; a < A - 1; a++) {
-        const uint32_t sma = act ? (uint32_t)(selfw >> (8 * a)) & 0xffu : 0u;
-        const uint32_t uj = __reduce_or_sync(kFull, sma);
-        if (!uj) continue;
+        for (int j = 0;; j++) {
+            if (jb >> j & 1u) {
 #pragma unroll 1
-        for (int b = a + 1; b < A; b++) {
-            if (SEL && !(pairs >> pair_index(a, b, A) & 1u)) continue;
-            uint32_t qa = 0, qb = 0;
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int t = 32 * r + lane;
-                const int ga = t / kNumGroups, gb = t - kNumGroups * ga;
-                bool pass = false;
-                if (t < kNumGroups * kNumGroups && (uj >> grp_joint(ga) & 1u)) {
-                    const float4 u = W.gbd[a][ga];
-                    pass = near3(u.x, u.y, u.z, W.gbd[b][gb], u.w);
-                }
-                uint32_t bal = __ballot_sync(kFull, pass);
-                while (bal) {
-                    const int tt = 32 * r + __ffs(bal) - 1;
-                    bal &= bal - 1;
-                    qa |= 1u << (tt / kNumGroups);
-                    qb |= 1u << (tt % kNumGroups);
+                for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
+                    const float3 c = place_reg(T, P.grp[g]);
+                    W.lanes.cross.gc[g][0][lane] = c.x;
+                    W.lanes.cross.gc[g][1][lane] = c.y;
+                    W.lanes.cross.gc[g][2][lane] = c.z;
                 }
             }
-            if (!qa || !act || hit) continue;
-            int from = 0;
-            while (from >= 0 && !hit) {
-                int n = 0, next = -1;
-                {
-                    Xf T;
-                    load_base(T, P.base[a]);
-#pragma unroll 1
-                    for (int j = 0; j < kNumJoints; j++) {
-                        if (j > 0) joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * a + j - 1, k), j);
-                        stash_joint(j, T, sma, qa, from, n, next, W, lane);
-                    }
-                }
-                from = next;
-                if (n == 0) break;
-                Xf T;
-                load_base(T, P.base[b]);
-#pragma unroll 1
-                for (int j = 0; j < kNumJoints; j++) {
-                    if (j > 0) joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * b + j - 1, k), j);
-                    probe_joint(j, P, T, qb, n, hit, W, lane);
-                }
-            }
+            if (j == top_b) break;
+            joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * b + j, k), j + 1);
         }
     }
+    bool hit = false;
+    int from = sma ? 0 : kNumDet;
+    do {
+        int n = 0, next = kNumDet;
+        {
+            Xf T;
+            load_base(T, P.base[a]);
+#pragma unroll 1
+            for (int j = 0;; j++) {
+                if ((sma >> j & 1u) && next == kNumDet && from < det_first(j + 1))
+                    stash_joint(j, P, T, gb, from, n, next, W, lane);
+                if (j == top_a) break;
+                joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * a + j, k), j + 1);
+            }
+        }
+        if (__any_sync(kFull, n > 0)) {
+            Xf T;
+            load_base(T, P.base[b]);
+#pragma unroll 1
+            for (int j = 0;; j++) {
+                if ((jb >> j & 1u) && !hit && n > 0) probe_joint(j, T, n, hit, W, lane);
+                if (j == top_b) break;
+                joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * b + j, k), j + 1);
+            }
+        }
+        from = hit ? kNumDet : next;
+    } while (__any_sync(kFull, from < kNumDet));
     return hit;
 }
 
@@ -1221,8 +1274,8 @@ __device__ __forceinline__ void thread_split(bool exact, int g, int lane, const 
 template <int A, int SPL>
 __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W, const float4 *S,
                                              const SceneLayout &L, int seg, int g, int lane, uint64_t (&envw)[SPL],
-                                             uint64_t (&selfw)[SPL], uint64_t &cand_env, uint64_t &cand_self,
-                                             double &tally) {
+                                             uint64_t (&selfw)[SPL], uint32_t (&pm)[SPL], uint64_t &cand_env,
+                                             uint64_t &cand_self, double &tally) {
     MRPOP_PHASE_START();
     int envc[SPL], selfc[SPL];
     int tot_env = 0, tot_self = 0;
@@ -1232,17 +1285,20 @@ __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W
     for (int s = 0; s < SPL; s++) {
         const int k = lane + 1 + 32 * s;
         uint64_t ew, sw;
-        broad_sample<A>(P, W, S, L, seg, k <= g ? k : g, s > 0, ew, sw);
+        uint32_t pw;
+        broad_sample<A>(P, W, S, L, seg, k <= g ? k : g, ew, sw, pw);
         if (k > g) ew = sw = 0;
         const int ec = flag_count(ew), sc = flag_count(sw);
         if (s == 0) {
             envw[0] = ew;
             selfw[0] = sw;
+            pm[0] = pw;
             envc[0] = ec;
             selfc[0] = sc;
         } else {
             envw[SPL - 1] = ew;
             selfw[SPL - 1] = sw;
+            pm[SPL - 1] = pw;
             envc[SPL - 1] = ec;
             selfc[SPL - 1] = sc;
         }
@@ -1283,15 +1339,9 @@ template <int A, int SPL>
 __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &W, const float4 *S,
                                               const SceneLayout &L, const float4 *det_tab, int seg, int lane,
                                               const uint64_t (&envw)[SPL], const uint64_t (&selfw)[SPL],
-                                              uint64_t cand_env, uint64_t cand_self, int k0 = 0) {
+                                              const uint32_t (&pm)[SPL], uint64_t cand_env, uint64_t cand_self,
+                                              int k0 = 0) {
     MRPOP_PHASE_START();
-    // sub-group bounds over the segment's samples, from the reference-sphere bounds
-    for (int t = lane; t < A * kNumGroups; t += 32) {
-        const int a = t / kNumGroups, g = t - kNumGroups * a;
-        const float4 u = W.rsw[a][grp_ref(g)];
-        W.gbd[a][g] = make_float4(u.x, u.y, u.z, u.w + P.gofs[g]);
-    }
-    __syncwarp();
     uint64_t hits = 0;
     // one copy of the per-sample code for both slots (not unrolled)
 #pragma unroll 1
@@ -1306,9 +1356,24 @@ __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &
         bool h = narrow_lane<A>(P, W, S, L, det_tab, seg, k, ew, sw, dE, dS);
         MRPOP_PHASE(P, 5);
         MRPOP_COUNT_LANES(14, dE || dS);
-        if (A > 1 && __any_sync(kFull, dS && !h)) {
-            MRPOP_COUNT_W(15, 1);
-            h |= cross_swept<A>(P, W, seg, k, sw, dS && !h);
+        if (A > 1) {
+            // the arm pairs that the broad phase's swept bounds connect
+            // (every vote is a statement of its own: all lanes take part)
+            const uint32_t pms = s == 0 ? pm[0] : pm[SPL - 1];
+            uint32_t pairs = __ballot_sync(kFull, pms != 0);
+            uint32_t hb = __ballot_sync(kFull, h);
+            bool act = dS && !(hb & lanes_upto(lane));
+            while (pairs && __any_sync(kFull, act)) {
+                MRPOP_COUNT_W(15, 1);
+                const int p = __ffs(pairs) - 1;
+                pairs &= pairs - 1;
+                const uint32_t m = __shfl_sync(kFull, pms, p);
+                int a, b;
+                pair_arms<A>(p, a, b);
+                h |= cross_pair(P, W, seg, k, a, b, act ? (uint32_t)(sw >> (8 * a)) & m & 0xffu : 0u, m >> 8);
+                hb = __ballot_sync(kFull, h);
+                act = act && !(hb & lanes_upto(lane));
+            }
         }
         MRPOP_PHASE(P, 6);
         hits |= (uint64_t)__ballot_sync(kFull, h) << (32 * s);
@@ -1361,8 +1426,10 @@ __device__ __forceinline__ void fused_edge(const EdgeParams &P, WarpScratch &W, 
     if (P.rule == kRuleConnect && P.seg0 > 0) connect_advance(W, dof, P.seg0, lane);
     for (int seg = P.seg0; seg < nseg_run && first == 0; seg++) {
         uint64_t envw[SPL], selfw[SPL], cand_env, cand_self;
-        if (broad_decide<A, SPL>(P, W, S, L, seg, g, lane, envw, selfw, cand_env, cand_self, tally)) {
-            const int fb = narrow_segment<A, SPL>(P, W, S, L, det_tab, seg, lane, envw, selfw, cand_env, cand_self);
+        uint32_t pm[SPL];
+        if (broad_decide<A, SPL>(P, W, S, L, seg, g, lane, envw, selfw, pm, cand_env, cand_self, tally)) {
+            const int fb =
+                narrow_segment<A, SPL>(P, W, S, L, det_tab, seg, lane, envw, selfw, pm, cand_env, cand_self);
             if (fb < 64) first = seg * g + fb + 1;
         }
         if (P.rule == kRuleConnect) {
@@ -1393,9 +1460,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 // `half` of a pair takes samples 32 * half + 1 .. 32 * half + 32 of every
 // segment, so an edge takes the time of one 32-sample slot instead of two.
 // The thread split's totals and shares are summed over the pair (integers,
-// so in any order), the segment's swept bounds merged with the single-warp
-// kernel's formula, and both warps leave a segment together at its first
-// hit: the verdicts are those of the one-warp kernels.
+// so in any order), and both warps leave a segment together at its first hit:
+// the verdicts are those of the one-warp kernels.
 // ---------------------------------------------------------------------------
 struct PairShare {
     int tot[2][2];  // [half] env, self flag totals of the slot
@@ -1406,8 +1472,7 @@ struct PairShare {
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
 template <int A>
-__device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch &W, const WarpScratch &Wo,
-                                                const float4 *S, const SceneLayout &L, const float4 *det_tab,
+__device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch &W, const float4 *S, const SceneLayout &L, const float4 *det_tab,
                                                 long long e, int dof, int g, int lane, int half, PairShare &X,
                                                 int bar_id, bool staged) {
     if (!staged) {
@@ -1424,7 +1489,8 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
     int first = 0;
     for (int seg = 0; seg < nseg_run && first == 0; seg++) {
         uint64_t ew, sw;
-        broad_sample<A>(P, W, S, L, seg, k <= g ? k : g, false, ew, sw);
+        uint32_t pw;
+        broad_sample<A>(P, W, S, L, seg, k <= g ? k : g, ew, sw, pw);
         if (k > g) ew = sw = 0;
         const int ec = flag_count(ew), sc = flag_count(sw);
         int te = ec, ts = sc;
@@ -1437,27 +1503,13 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
             X.tot[half][0] = te;
             X.tot[half][1] = ts;
         }
-        pair_sync(bar_id);  // A: both slots' totals and swept bounds written
+        pair_sync(bar_id);  // A: both slots' totals written
         const int tot_env = X.tot[0][0] + X.tot[1][0], tot_self = X.tot[0][1] + X.tot[1][1];
         if (tot_env > 0 || tot_self > 0) {
-            // the segment's bounds: slot 0's grown by slot 1's (fk_approx_lane's merge)
-            const WarpScratch &W0 = half == 0 ? W : Wo, &W1 = half == 0 ? Wo : W;
-            float4 mg[2];
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const int t = lane + 32 * r;
-                if (t < A * kRefSpheres) {
-                    const float4 o = (&W0.rsw[0][0])[t], sv = (&W1.rsw[0][0])[t];
-                    const float ex = sv.x - o.x, ey = sv.y - o.y, ez = sv.z - o.z;
-                    const float d = sqrtf(ex * ex + ey * ey + ez * ez) * 1.0001f;
-                    mg[r] = make_float4(o.x, o.y, o.z, fmaxf(o.w, d + sv.w) + 1e-6f);
-                }
-            }
             bool cE, cS;
             if (P.flags & kExactBit) {
                 cE = ec > 0;
                 cS = sc > 0;
-                pair_sync(bar_id);  // B (both warps read the bounds)
             } else {
                 int de = k <= g ? ref_share(ec, tot_env, g) : 0, ds = k <= g ? ref_share(sc, tot_self, g) : 0;
                 int se = de, ss = ds;
@@ -1470,7 +1522,7 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
                     X.sum[half][0] = se;
                     X.sum[half][1] = ss;
                 }
-                pair_sync(bar_id);  // B: shares written, bounds read
+                pair_sync(bar_id);  // B: shares written
                 if (k == g) {  // the remainder goes to the last sample
                     de += 4 * g - (X.sum[0][0] + X.sum[1][0]);
                     ds += 4 * g - (X.sum[0][1] + X.sum[1][1]);
@@ -1478,17 +1530,13 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
                 cE = tot_env > 0 && de > 0;
                 cS = tot_self > 0 && ds > 0;
             }
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                const int t = lane + 32 * r;
-                if (t < A * kRefSpheres) (&W.rsw[0][0])[t] = mg[r];
-            }
             const uint64_t cand_env = __ballot_sync(kFull, cE), cand_self = __ballot_sync(kFull, cS);
             __syncwarp();
             const uint64_t envw[1] = {ew}, selfw[1] = {sw};
+            const uint32_t pm[1] = {pw};
             const int fb = (cand_env | cand_self)
-                               ? narrow_segment<A, 1>(P, W, S, L, det_tab, seg, lane, envw, selfw, cand_env, cand_self,
-                                                      32 * half)
+                               ? narrow_segment<A, 1>(P, W, S, L, det_tab, seg, lane, envw, selfw, pm, cand_env,
+                                                      cand_self, 32 * half)
                                : 64;
             if (lane == 0) X.fb[half] = fb;
             pair_sync(bar_id);  // C: both slots' first hits written
@@ -1517,12 +1565,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     MRPOP_KERNEL_PROLOGUE()
     static_assert(kWarpsPerBlock % 2 == 0, "warps come in pairs");
     __shared__ PairShare X[kWarpsPerBlock / 2];
-    const WarpScratch &Wo = Wall[warp ^ 1];
     const int pair = warp >> 1, half = warp & 1;
     (void)nwarps;
     for (long long e = (long long)blockIdx.x * (kWarpsPerBlock / 2) + pair; e < P.n_edges;
          e += (long long)gridDim.x * (kWarpsPerBlock / 2))
-        fused_edge_pair<A>(P, W, Wo, S, L, det_tab, e, dof, g, lane, half, X[pair], 1 + pair, staged);
+        fused_edge_pair<A>(P, W, S, L, det_tab, e, dof, g, lane, half, X[pair], 1 + pair, staged);
 }
 
 // ---------------------------------------------------------------------------
@@ -1539,6 +1586,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 struct ArmShare {
     unsigned long long env[2][32], self[2][32];  // [slot][lane] flag words of the segment
     unsigned int hits[2];                        // [slot] lanes whose sample collided
+    unsigned int pm[2][num_pairs(kMaxArms)];     // [slot][pair] joints connected by swept bounds
     unsigned int next[3];                        // arm pairs handed out: broad, narrow slot 0, slot 1
 };
 
@@ -1548,31 +1596,6 @@ __device__ __forceinline__ int take_pair(unsigned int *c, int lane) {
     if (lane == 0) p = atomicAdd(c, 1u);
     return (int)__shfl_sync(kFull, p, 0);
 }
-
-// Arm pair p (pair_index order): its lower and upper arm.
-template <int A>
-__host__ __device__ __forceinline__ constexpr void pair_arms(int p, int &a, int &b) {
-    a = 0;
-    while (p >= A - 1 - a) {
-        p -= A - 1 - a;
-        a++;
-    }
-    b = a + 1 + p;
-}
-
-// pair_arms inverts pair_index for every pair of up to 5 arms
-template <int A>
-constexpr bool pair_order_round_trips() {
-    for (int p = 0; p < num_pairs(A); p++) {
-        int a = 0, b = 0;
-        pair_arms<A>(p, a, b);
-        if (!(0 <= a && a < b && b < A) || pair_index(a, b, A) != p) return false;
-    }
-    return true;
-}
-static_assert(pair_order_round_trips<2>() && pair_order_round_trips<3>() && pair_order_round_trips<4>() &&
-                  pair_order_round_trips<5>(),
-              "arm pair order");
 
 template <int A, int SPL>
 __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char *wbase, const float4 *S,
@@ -1606,8 +1629,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
             const int k = lane + 1 + 32 * s;
             float(*sp)[3][32] = s == 0 ? W.broad.cur : W.broad.low;
             float4 *sw = W.broad.swept[s];
-            fk_approx_lane(P.base[arm], W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, sp, lane, sw, W.rsw[arm],
-                           s > 0);
+            fk_approx_lane(P.base[arm], W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, sp, lane, sw);
             uint32_t em = 0, im = 0;
             if (do_env) {
                 const uint32_t m = env_mask_approx(S, L, P.sc, sp, lane, sw);
@@ -1643,10 +1665,13 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                         bal[r] = __ballot_sync(kFull, t < kNumApprox * kNumApprox &&
                                                           near3(swa[i].x, swa[i].y, swa[i].z, swb[j], swa[i].w));
                     }
-                    if (!(bal[0] | bal[1] | bal[2] | bal[3])) continue;
+                    if (!(bal[0] | bal[1] | bal[2] | bal[3])) {
+                        if (lane == 0) X.pm[s][p] = 0;
+                        continue;
+                    }
                     const float(*low)[3][32] = s == 0 ? Wa[a].broad.cur : Wa[a].broad.low;
                     const float(*cur)[3][32] = s == 0 ? Wa[b].broad.cur : Wa[b].broad.low;
-                    uint32_t am = 0;
+                    uint32_t am = 0, ja = 0, jb = 0;
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
                         uint32_t q = bal[r];
@@ -1654,6 +1679,8 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                             const int t = 32 * r + __ffs(q) - 1;
                             q &= q - 1;
                             const int i = t / kNumApprox, j = t - kNumApprox * i;
+                            ja |= 1u << approx_joint(i);
+                            jb |= 1u << approx_joint(j);
                             if (hit_sphere_sphere(low[i][0][lane], low[i][1][lane], low[i][2][lane],
                                                   c_approx[i].w, cur[j][0][lane], cur[j][1][lane],
                                                   cur[j][2][lane], c_approx[j].w))
@@ -1661,8 +1688,9 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                         }
                     }
                     if (am && k <= g) atomicOr(&X.self[s][lane], (unsigned long long)am << (8 * a));
+                    if (lane == 0) X.pm[s][p] = ja | jb << 8;
                 }
-                }
+            }
         }
         __syncthreads();
         // the thread split, from the ORed words (every warp alike)
@@ -1686,30 +1714,42 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
             uint64_t cand_env = 0, cand_self = 0;
             thread_split<SPL>((P.flags & kExactBit) != 0, g, lane, envc, selfc, tot_env, tot_self, cand_env,
                               cand_self);
-            // the segment's sub-group bounds for the arm-vs-arm screens, from
-            // every arm's reference-sphere bounds (each warp's own row)
-            const WarpScratch *Wa = reinterpret_cast<const WarpScratch *>(wbase);
-            for (int t = lane; t < A * kNumGroups; t += 32) {
-                const int a = t / kNumGroups, gg = t - kNumGroups * a;
-                const float4 u = Wa[a].rsw[a][grp_ref(gg)];
-                W.gbd[a][gg] = make_float4(u.x, u.y, u.z, u.w + P.gofs[gg]);
-            }
-            __syncwarp();
 #pragma unroll 1
             for (int s = 0; s < SPL; s++) {
+                // hits found so far by any warp: a hit in an earlier slot
+                // settles the edge, one at or below a lane settles that lane
+                // (a stale read only costs tests that are not needed).  Other
+                // warps, and this warp's lane 0, write the words meanwhile, so
+                // the branch takes lane 0's reading for the whole warp
+                const volatile unsigned int *hits = X.hits;
+                if (s > 0 && __shfl_sync(kFull, hits[0], 0)) break;
                 const int bit = lane + 32 * s;
                 const bool dE = cand_env >> bit & 1ull, dS = cand_self >> bit & 1ull;
                 const int k = bit + 1 <= g ? bit + 1 : g;
-                bool h = narrow_lane<A, true>(P, W, S, L, det_tab, seg, k, envw[s], selfw[s], dE, dS, arm);
-                // the slot's arm pairs, one at a time to whichever warp is free
+                const uint64_t ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
+                const bool open = !(hits[s] & lanes_upto(lane));
+                unsigned int hb = __ballot_sync(
+                    kFull, narrow_lane<A, true>(P, W, S, L, det_tab, seg, k, ew, sw, dE && open, dS && open, arm));
+                if (lane == 0 && hb) atomicOr(&X.hits[s], hb);
+                // the slot's connected arm pairs, one at a time to whichever
+                // warp is free
                 if (A > 1 && __any_sync(kFull, dS)) {
                     unsigned int *next = &X.next[1 + s];
-                    for (int p = take_pair(next, lane); p < num_pairs(A); p = take_pair(next, lane))
-                        if (__any_sync(kFull, dS && !h))
-                            h |= cross_swept<A, true>(P, W, seg, k, selfw[s], dS && !h, 1u << p);
+                    const uint32_t live = __ballot_sync(kFull, lane < num_pairs(A) && X.pm[s][lane] != 0);
+                    for (int t = take_pair(next, lane); t < __popc(live); t = take_pair(next, lane)) {
+                        const bool act = dS && !((hits[s] | hb) & lanes_upto(lane));
+                        uint32_t rest = live;
+                        for (int i = 0; i < t; i++) rest &= rest - 1;
+                        const int p = __ffs(rest) - 1;
+                        const uint32_t m = X.pm[s][p];
+                        int a, b;
+                        pair_arms<A>(p, a, b);
+                        const uint32_t sma = act ? (uint32_t)(sw >> (8 * a)) & m & 0xffu : 0u;
+                        const unsigned int h2 = __ballot_sync(kFull, cross_pair(P, W, seg, k, a, b, sma, m >> 8));
+                        if (lane == 0 && h2) atomicOr(&X.hits[s], h2);
+                        hb |= h2;
+                    }
                 }
-                const unsigned int hb = __ballot_sync(kFull, h);
-                if (lane == 0 && hb) atomicOr(&X.hits[s], hb);
             }
             __syncthreads();
             const uint64_t hits = (uint64_t)X.hits[0] | (SPL > 1 ? (uint64_t)X.hits[1] << 32 : 0ull);
@@ -1729,8 +1769,13 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
     }
 }
 
+// CTAs of the arm-per-warp kernels that fit an SM beside a 51-box scene (their
+// scratch is 11.6 KB per warp).  Given as a launch bound because ptxas, left to
+// choose, cuts 5 arms at 64 samples to 72 registers and spills.
+__host__ __device__ constexpr int armwise_min_blocks(int A) { return A >= 5 ? 3 : A == 4 ? 4 : 5; }
+
 template <int A, int SPL>
-__global__ void __launch_bounds__(32 * A) armwise_kernel(const __grid_constant__ EdgeParams P) {
+__global__ void __launch_bounds__(32 * A, armwise_min_blocks(A)) armwise_kernel(const __grid_constant__ EdgeParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ float4 det_tab[kNumDet];
@@ -1749,9 +1794,9 @@ __global__ void __launch_bounds__(32 * A) armwise_kernel(const __grid_constant__
 
 // ---------------------------------------------------------------------------
 // split pipeline for single-segment edges: the broad kernel writes every
-// sample's flag words, each edge's candidate masks and reference-sphere
-// bounds to HBM (P.sflags, P.smasks, P.sbounds); the narrow kernel runs the
-// detailed phase of edges with candidates.  Each kernel's code fits the
+// sample's flag words, each edge's candidate masks and the joints that swept
+// bounds connect per arm pair to HBM (P.sflags, P.smasks, P.spairs); the narrow
+// kernel runs the detailed phase of edges with candidates.  Each kernel's code fits the
 // instruction cache on its own.  broad_edge / narrow_edge are one warp's work
 // on edge e, shared by the plain kernels and the batch kernels.
 // ---------------------------------------------------------------------------
@@ -1821,12 +1866,15 @@ __device__ __forceinline__ void broad_edge(const EdgeParams &P, WarpScratch &W, 
         (void)nseg;
     }
     uint64_t envw[SPL], selfw[SPL], cand_env, cand_self;
+    uint32_t pm[SPL];
     double tally = 0.0;
-    const bool any = broad_decide<A, SPL>(P, W, S, L, r, g, lane, envw, selfw, cand_env, cand_self, tally);
+    const bool any = broad_decide<A, SPL>(P, W, S, L, r, g, lane, envw, selfw, pm, cand_env, cand_self, tally);
     if (any) {
 #pragma unroll
-        for (int s = 0; s < SPL; s++) store_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
-        for (int t = lane; t < A * kRefSpheres; t += 32) P.sbounds[e * (A * kRefSpheres) + t] = (&W.rsw[0][0])[t];
+        for (int s = 0; s < SPL; s++) {
+            store_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
+            if (lane < num_pairs(A)) P.spairs[(e * SPL + s) * num_pairs(A) + lane] = (uint16_t)pm[s];
+        }
     }
     if (lane == 0) {
         P.smasks[2 * e] = cand_env;
@@ -1861,11 +1909,13 @@ __device__ __forceinline__ void narrow_edge(const EdgeParams &P, WarpScratch &W,
     const int nseg = edge_setup(P, W, e, dof, g, lane, too_many);
     if (SEG && P.rule == kRuleConnect && r > 0) connect_advance(W, dof, r, lane);
     uint64_t envw[SPL], selfw[SPL];
+    uint32_t pm[SPL];
 #pragma unroll
-    for (int s = 0; s < SPL; s++) load_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
-    for (int t = lane; t < A * kRefSpheres; t += 32) (&W.rsw[0][0])[t] = P.sbounds[e * (A * kRefSpheres) + t];
-    __syncwarp();
-    const int fb = narrow_segment<A, SPL>(P, W, S, L, det_tab, r, lane, envw, selfw, cand_env, cand_self);
+    for (int s = 0; s < SPL; s++) {
+        load_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
+        pm[s] = lane < num_pairs(A) ? P.spairs[(e * SPL + s) * num_pairs(A) + lane] : 0u;
+    }
+    const int fb = narrow_segment<A, SPL>(P, W, S, L, det_tab, r, lane, envw, selfw, pm, cand_env, cand_self);
     if (lane == 0) {
         if (fb < 64) {
             P.valid[e] = 0;
@@ -2030,7 +2080,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 // launch's counter, stages each instance's parameters and scene as
 // batch_kernel does, and runs the arm-per-warp body on every edge of the chunk.
 template <int A, int SPL>
-__global__ void __launch_bounds__(32 * A) batch_armwise_kernel(const __grid_constant__ BatchParams B) {
+__global__ void __launch_bounds__(32 * A, armwise_min_blocks(A)) batch_armwise_kernel(const __grid_constant__ BatchParams B) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ float4 det_tab[kNumDet];

@@ -62,15 +62,16 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
 size_t warp_scratch_bytes();
 
 // Scratch of the single-segment pipeline (staged flags, candidate masks and
-// reference-sphere bounds): its size, and its slices in p.  Two work counters
+// arm-pair joints): its size, and its slices in p.  Two work counters
 // in a 128-byte head (every edge's flag words start on an L2 line), then per
 // edge: 32 * spl samples x {env, self} flag words, {env, self} candidate
-// masks, A arms' reference-sphere bounds and the segment state.
+// masks, kPairSlots arm-pair words and the segment state.
 constexpr size_t kSplitScratchHead = 128;
-constexpr size_t split_scratch_bytes(int64_t n_edges, int g, int A) {
+constexpr int kPairSlots = 2 * num_pairs(kMaxArms);
+constexpr size_t split_scratch_bytes(int64_t n_edges, int g, [[maybe_unused]] int A) {
     return kSplitScratchHead +
            (size_t)n_edges * (32 * (g > 32 ? 2 : 1) * 2 * sizeof(uint64_t) + 2 * sizeof(uint64_t) +
-                              (size_t)A * kRefSpheres * sizeof(float4) + 2 * sizeof(int32_t));
+                              kPairSlots * sizeof(uint16_t) + 2 * sizeof(int32_t));
 }
 void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int A);
 
