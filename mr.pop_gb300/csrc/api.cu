@@ -391,6 +391,20 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots) {
 
 namespace {
 
+// True for a rotation (rows orthonormal to 1e-4) and a translation within
+// 16 m (FP32 positions then err by a few micrometres).
+bool rigid_base(const float *m) {
+    for (int r = 0; r < 3; r++) {
+        for (int c = r; c < 3; c++) {
+            double dot = 0.0;
+            for (int i = 0; i < 3; i++) dot += (double)m[4 * r + i] * m[4 * c + i];
+            if (!(std::fabs(dot - (r == c ? 1.0 : 0.0)) < 1e-4)) return false;
+        }
+        if (!(std::fabs((double)m[4 * r + 3]) <= 16.0)) return false;
+    }
+    return true;
+}
+
 }  // namespace
 
 namespace mrpop {
@@ -475,6 +489,7 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
     A = arm >= 0 ? 1 : robots->n_arms;
     for (int a = 0; a < A; a++)
         for (int i = 0; i < 12; i++) p.base[a][i] = robots->base[arm >= 0 ? arm : a][i];
+    for (int a = 0; a < A; a++) p.rigid |= (int)rigid_base(p.base[a]) << a;
     p.fbp = broad_flops_per_sample(A, scene->env_test_flops, flags);
     smem = (size_t)scene->total_f4 * sizeof(float4) + block_scratch_bytes();
     return MRPOP_OK;

@@ -126,6 +126,7 @@ struct EdgeParams {
     int g;           // samples per segment
     int flags;       // MRPOP_CHECK_* | MRPOP_MODE_EXACT
     int single;      // 1: single-arm (fkcc_single_buffer_mr) semantics
+    int rigid;       // bit a: arm a's base is a rigid transform near the origin (see kRegularRad)
     int rule;        // MRPOP_RULE_*
     int seg0;        // segmented rules: the segment this launch checks (split kernels) or starts at (fused)
     float range;
@@ -325,13 +326,35 @@ __device__ __forceinline__ float warp_max(float v) {
     return r;
 }
 
+// Three-input float min / max (sm_100 family); NaN inputs are ignored, as
+// fminf / fmaxf do.
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Facts that hold for every pose of the arm (link lengths, distances between
+// spheres that depend on a joint or two) are used only where the joint frames
+// are accurate: joint values that add up to at most this many radians, where
+// __sinf / __cosf err by about 1e-5 at most (beyond, or with a NaN, the
+// computed frames need not be rotations), on a base that is a rigid transform
+// (EdgeParams::rigid).  FP32 positions then err by far less than a millimetre.
+constexpr float kRegularRad = 64.0f;
+
 // FK of one arm for this lane's sample; the 11 approx centres go to column
 // `lane` of dst.  With swept != nullptr it also writes, for every approx
 // sphere, a bound of that sphere over the warp's 32 samples: the centre of
 // the box around its 32 centres, radius = half the box diagonal (+0.4 %) +
 // sphere radius + cull margin.  If the sphere touches something at any of the
 // samples, its swept bound touches it too (the margin covers FP rounding).
-__device__ __forceinline__ void fk_approx_lane(const float *base12, const WarpScratch &W, int rule, int seg,
+// Returns whether the joint values are within kRegularRad.
+__device__ __forceinline__ bool fk_approx_lane(const float *base12, const WarpScratch &W, int rule, int seg,
                                                    int qarm, int k, float (*dst)[3][32], int lane, float4 *swept) {
     float q[7];
     sample_q(W, rule, seg, qarm, k, q);
@@ -343,40 +366,47 @@ __device__ __forceinline__ void fk_approx_lane(const float *base12, const WarpSc
         dst[i][1][lane] = s.y[i];
         dst[i][2][lane] = s.z[i];
     }
-    if (!swept) return;
+    if (!swept) return false;
     __syncwarp();
     {
         // spheres 1..10: lane t < 30 takes coordinate t % 3 of sphere 1 + t / 3
-        // over the 32 columns (start skewed by lane: conflict-free banks);
-        // sphere 0 (the base frame's) by warp reductions
+        // over the 32 columns, four at a time (start skewed by lane: each
+        // quarter warp reads eight different 16-byte bank groups) and three
+        // values per min / max: 8 loads and 32 min / max in place of 31 loads
+        // and 62 (with the pairs of sphere 5 left out below, the broad kernel
+        // on 65536 4-arm edges: 531 -> 470 us); sphere 0 sits on the base and
+        // does not move
         float lo = 0.0f, hi = 0.0f;
         if (lane < 30) {
-            const float *col = &dst[1 + lane / 3][lane % 3][0];
-            lo = hi = col[lane];
-#pragma unroll 8
-            for (int l = 1; l < 32; l++) {
-                const float v = col[(l + lane) & 31];
-                lo = fminf(lo, v);
-                hi = fmaxf(hi, v);
+            const float4 *col = reinterpret_cast<const float4 *>(&dst[1][0][0] + 32 * lane);
+            const float4 f = col[lane & 7];
+            lo = fminf(min3(f.x, f.y, f.z), f.w);
+            hi = fmaxf(max3(f.x, f.y, f.z), f.w);
+#pragma unroll
+            for (int l = 1; l < 8; l++) {
+                const float4 v = col[(l + lane) & 7];
+                lo = min3(min3(lo, v.x, v.y), v.z, v.w);
+                hi = max3(max3(hi, v.x, v.y), v.z, v.w);
             }
         }
         const float ly = __shfl_down_sync(kFull, lo, 1), hy = __shfl_down_sync(kFull, hi, 1);
         const float lz = __shfl_down_sync(kFull, lo, 2), hz = __shfl_down_sync(kFull, hi, 2);
-        const float l0x = warp_min(s.x[0]), h0x = warp_max(s.x[0]);
-        const float l0y = warp_min(s.y[0]), h0y = warp_max(s.y[0]);
-        const float l0z = warp_min(s.z[0]), h0z = warp_max(s.z[0]);
         const bool own = lane < 30 && lane % 3 == 0;
         const int i = own ? 1 + lane / 3 : 0;
         if (own || lane == 30) {
-            const float ax = own ? lo : l0x, bx = own ? hi : h0x;
-            const float ay = own ? ly : l0y, by = own ? hy : h0y;
-            const float az = own ? lz : l0z, bz = own ? hz : h0z;
+            const float ax = own ? lo : s.x[0], bx = own ? hi : s.x[0];
+            const float ay = own ? ly : s.y[0], by = own ? hy : s.y[0];
+            const float az = own ? lz : s.z[0], bz = own ? hz : s.z[0];
             const float dx = bx - ax, dy = by - ay, dz = bz - az;
             swept[i] = make_float4(0.5f * (ax + bx), 0.5f * (ay + by), 0.5f * (az + bz),
                                    0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + c_approx[i].w + kCullMargin);
         }
     }
     __syncwarp();
+    float sum = 0.0f;  // NaN if any is
+#pragma unroll
+    for (int d = 0; d < 7; d++) sum += fabsf(q[d]);
+    return sum <= kRegularRad;
 }
 
 // ---------------------------------------------------------------------------
@@ -526,14 +556,19 @@ static __constant__ uint8_t c_intra_pairs[21][2] = {
 // pairs, one per lane, screened by the swept bounds sw of the warp's samples;
 // exact per-sample tests for the survivors.  Returns the lane's flag bits (by
 // joint of the pair's first sphere).
-__device__ __forceinline__ uint32_t intra_flags(const float (*sp)[3][32], const float4 *sw, int lane) {
+// regular (warp-uniform): the pairs of sphere 5 are not tested, its joint is
+// flagged.  Pair (5, 8) overlaps in every pose: sphere 8 lies on joint 7's axis
+// at (0.088, -0.129) from joint 6's, 0.156 m, and sphere 5 0.111 m from joint
+// 6's axis and 0.037 m along it, so their centres are at most
+// sqrt(0.267^2 + 0.037^2) = 0.270 m apart with radii adding up to 0.280 m.
+__device__ __forceinline__ uint32_t intra_flags(const float (*sp)[3][32], const float4 *sw, int lane, bool regular) {
     // pair `lane` of c_intra_pairs, computed rather than read per lane
     const int p1 = lane < 6 ? 0 : lane < 12 ? 1 : lane < 17 ? 2 : 5;
     const int p2 = lane < 12 ? 5 + lane % 6 : lane == 12 ? 5 : lane < 17 ? lane - 6 : lane - 10;
     const float4 u1 = sw[p1];
-    const bool c = lane < 21 && near3(u1.x, u1.y, u1.z, sw[p2], u1.w);
+    const bool c = lane < (regular ? 17 : 21) && near3(u1.x, u1.y, u1.z, sw[p2], u1.w);
     uint32_t bal = __ballot_sync(kFull, c);
-    uint32_t jm = 0;
+    uint32_t jm = regular ? 1u << approx_joint(5) : 0u;
     while (bal) {
         const int t = __ffs(bal) - 1;
         bal &= bal - 1;
@@ -560,7 +595,7 @@ __device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W
     for (int b = 0; b < A; b++) {
         MRPOP_PHASE_START();
         float4 *sw = W.broad.swept[b];
-        fk_approx_lane(P.base[b], W, P.rule, seg, P.single ? 0 : b, k, cur, lane, sw);
+        const bool reg = fk_approx_lane(P.base[b], W, P.rule, seg, P.single ? 0 : b, k, cur, lane, sw);
         MRPOP_PHASE(P, 0);
         if (do_env) {
             const uint32_t m = env_mask_approx(S, L, P.sc, cur, lane, sw);
@@ -574,7 +609,8 @@ __device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W
         if (!do_self) continue;
         // intra-arm pairs: one pair per lane screened by swept bounds, exact
         // per-sample tests for the survivors
-        const uint32_t jm = intra_flags(cur, sw, lane);
+        const bool regular = __all_sync(kFull, reg) && (P.rigid >> b & 1);
+        const uint32_t jm = intra_flags(cur, sw, lane, regular);
         selfw |= (uint64_t)jm << (8 * b);
         MRPOP_PHASE(P, 2);
         if (A == 1) continue;
@@ -1629,7 +1665,9 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
             const int k = lane + 1 + 32 * s;
             float(*sp)[3][32] = s == 0 ? W.broad.cur : W.broad.low;
             float4 *sw = W.broad.swept[s];
-            fk_approx_lane(P.base[arm], W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, sp, lane, sw);
+            const bool reg =
+                fk_approx_lane(P.base[arm], W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, sp, lane, sw);
+            const bool regular = __all_sync(kFull, reg) && (P.rigid >> arm & 1);
             uint32_t em = 0, im = 0;
             if (do_env) {
                 const uint32_t m = env_mask_approx(S, L, P.sc, sp, lane, sw);
@@ -1637,7 +1675,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                 for (int i = 1; i < kNumApprox; i++)
                     if (m >> i & 1u) em |= 1u << approx_joint(i);
             }
-            if (do_self) im = intra_flags(sp, sw, lane);
+            if (do_self) im = intra_flags(sp, sw, lane, regular);
             if (k <= g) {
                 if (em) atomicOr(&X.env[s][lane], (unsigned long long)em << (8 * arm));
                 if (im) atomicOr(&X.self[s][lane], (unsigned long long)im << (8 * arm));
