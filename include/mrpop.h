@@ -124,10 +124,11 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots);
  * sample index of the first sample whose detailed check fired (-1 if valid).
  * Replaces one fkcc_single_buffer* call per edge (see flags above).
  * Launch form: a call of more than the fused-edge limit runs the split
- * pipeline (a broad and a narrow kernel; for segmented rules, segment rounds
- * of both and a fused tail); a smaller call runs as one fused launch (both
+ * pipeline (a broad and a narrow kernel, and for more than one arm a rows
+ * kernel; for segmented rules, segment rounds of them and a fused tail); a smaller call runs as one fused launch (both
  * phases per edge in one warp, from segment 0), which saves the launches and
  * the staging that dominate small calls.  Verdicts are the same either way.
+ * Segmented calls (mrpop_validate_segments) have 5/2 of the limit.
  * mrpop_set_fused_edges sets the limit for the process (0: the default, 2048
  * edges; -1: every call split) and returns the previous one.
  */

@@ -107,7 +107,9 @@ cudaError_t timed_launch(int arms, mrpop::KernelKind kind, const mrpop::EdgePara
     }
     if (!on) return mrpop::launch_validate(arms, kind, p, smem, stream);
     TimedLaunch t{nullptr, nullptr,
-                  (int)(kind == mrpop::kFusedPair || kind == mrpop::kArmwise ? mrpop::kFused : kind)};
+                  (int)(kind == mrpop::kFusedPair || kind == mrpop::kArmwise ? mrpop::kFused
+                        : kind == mrpop::kRows                               ? mrpop::kNarrow
+                                                                             : kind)};
     cudaError_t e = cudaEventCreate(&t.start);
     if (e == cudaSuccess) e = cudaEventCreate(&t.stop);
     if (e == cudaSuccess) e = cudaEventRecord(t.start, stream);
@@ -495,7 +497,7 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
     return MRPOP_OK;
 }
 
-// A 128-byte head with the two work counters, then per edge: flag words,
+// A 128-byte head with the three work counters, then per edge: flag words,
 // candidate masks, arm-pair joints and segment state.  The kernels
 // stage the flag words as 32-bit pairs for up to 4 arms, in the first half
 // of their slice (which keeps its 64-bit size).
@@ -521,6 +523,18 @@ void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int
 // library's stream-ordered pool.
 // Calls of at most this many edges run as one fused launch (mrpop_set_fused_edges).
 constexpr int64_t kFusedEdgesDefault = 2048;
+constexpr int64_t kMaxFusedEdges = (int64_t)1 << 40;  // (beyond any call; keeps the product below in range)
+
+// The limit of segmented calls: the split pipeline runs 4 rounds of two or
+// three launches and a fused tail, each as long as its slowest edge, so one
+// fused launch is the faster form up to about two edges per resident warp.
+// Measured, split against fused in us: 3 arms x 24 B-spline 2800 edges 609 /
+// 250, 4096 569 / 422, 8000 641 / 750; 5 arms x 64 shortcut 4096 edges 1058 /
+// 773, 8000 1251 / 1480; 4 arms x 32 connect 4096 576 / 381, 8000 737 / 763.
+// (Single-segment calls, 4 arms x 32: 2000 edges 171 / 207, 2800 224 / 191,
+// 4096 240 / 322; 5 arms x 64: 2000 327 / 246, 4096 395 / 463.)
+constexpr int64_t fused_segment_edges(int64_t limit) { return limit < 0 ? limit : limit * 5 / 2; }
+
 std::atomic<int64_t> g_fused_edges{kFusedEdgesDefault};
 
 mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robots, const float *q0,
@@ -547,7 +561,8 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     // more arms one warp per arm, else above 32 samples per segment two warps
     // per edge (one per 32-sample slot), unless the flop tally is wanted
     cudaError_t err;
-    if (n_edges <= g_fused_edges.load(std::memory_order_relaxed)) {
+    const int64_t limit = g_fused_edges.load(std::memory_order_relaxed);
+    if (n_edges <= (rule == MRPOP_RULE_PLAIN || limit > kMaxFusedEdges ? limit : fused_segment_edges(limit))) {
         p.seg0 = 0;
         err = timed_launch(A, flops ? kFused : A >= 3 ? kArmwise : g > 32 ? kFusedPair : kFused, p, smem, stream);
         if (tmp_valid) cudaFreeAsync(tmp_valid, stream);
@@ -557,7 +572,7 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     }
     // split pipeline: staged flags, masks, bounds and segment state in
     // stream-ordered scratch.  Single-segment edges: one broad and one narrow
-    // launch.  Segmented rules: segment r of every undecided edge per round
+    // launch (and one of rows for more than one arm).  Segmented rules: segment r of every undecided edge per round
     // (broad + narrow), kSegRounds rounds, then the fused kernel for the edges
     // that still have segments left, from segment kSegRounds on.
     void *scratch = ext_scratch;
@@ -573,9 +588,10 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
         const int rounds = rule == MRPOP_RULE_PLAIN ? 1 : kSegRounds;
         for (int r = 0; r < rounds && err == cudaSuccess; r++) {
             p.seg0 = r;
-            err = cudaMemsetAsync(p.work, 0, 2 * sizeof(unsigned long long), stream);
+            err = cudaMemsetAsync(p.work, 0, 3 * sizeof(unsigned long long), stream);
             if (err == cudaSuccess) err = timed_launch(A, kBroad, p, smem, stream);
             if (err == cudaSuccess) err = timed_launch(A, kNarrow, p, smem, stream);
+            if (err == cudaSuccess && A > 1) err = timed_launch(A, kRows, p, smem, stream);
         }
         if (err == cudaSuccess && rule != MRPOP_RULE_PLAIN) {
             p.seg0 = kSegRounds;

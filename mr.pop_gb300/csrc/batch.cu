@@ -8,7 +8,8 @@
 // parameter blocks, a chunk table (up to `chunk` edges of one instance per
 // chunk, instances in order) and work counters; batch_kernel<A, SPL, MODE,
 // SEG> hands chunks to CTAs and edges to warps.  A group's run is a broad and
-// a narrow launch (each after its counter reset); a segmented group runs them
+// a narrow launch, and for more than one arm a rows launch (each after its
+// counter reset); a segmented group runs them
 // for kSegRounds rounds and then the fused kernel.  The captured graph runs
 // each group on its own branch so small groups overlap.
 //
@@ -33,7 +34,7 @@ struct mrpop_batch {
         mrpop::EdgeParams *d_items = nullptr;
         int4 *d_chunks = nullptr;
         int n_chunks = 0;
-        unsigned long long *d_work = nullptr;  // chunk counters of the broad, narrow and fused launches
+        unsigned long long *d_work = nullptr;  // chunk counters of the broad, narrow, fused and rows launches
         size_t scene_bytes = 0;       // largest staged scene of the group's instances
         std::vector<int64_t> edges;   // per instance
         int chunk = 0;                // edges per chunk
@@ -72,7 +73,8 @@ void release(mrpop_batch *b) {
 
 // One kernel of a group (mode kBatchBroad / kBatchNarrow / kBatchFused; seg0:
 // the round, or the first segment of the fused launch): its chunk counter is
-// zeroed first (in stream order).
+// zeroed first (in stream order).  The narrow kernel of a composite group is
+// followed by the rows kernel, in the same shape.
 cudaError_t launch_group(const mrpop_batch::Group &g, int mode, int grid, int seg0, cudaStream_t s) {
     mrpop::BatchParams p;
     p.items = g.d_items;
@@ -82,6 +84,12 @@ cudaError_t launch_group(const mrpop_batch::Group &g, int mode, int grid, int se
     p.work = g.d_work + mode;
     cudaError_t err = cudaMemsetAsync(p.work, 0, sizeof(unsigned long long), s);
     if (err == cudaSuccess) err = mrpop::launch_batch(g.arms, mode, g.seg, g.spl, p, g.smem(mode), grid, g.warps[mode], s);
+    if (mode == mrpop::kBatchNarrow && g.arms > 1) {
+        p.work = g.d_work + 3;
+        if (err == cudaSuccess) err = cudaMemsetAsync(p.work, 0, sizeof(unsigned long long), s);
+        if (err == cudaSuccess)
+            err = mrpop::launch_batch(g.arms, mrpop::kBatchRows, g.seg, g.spl, p, g.smem(mode), grid, g.warps[mode], s);
+    }
     return err;
 }
 
@@ -108,7 +116,10 @@ cudaError_t set_chunks(mrpop_batch::Group &g, int chunk) {
 cudaError_t max_grid(const mrpop_batch::Group &g, int mode, int warps, int sms, int *out) {
     int nb = 0;
     const size_t smem = g.scene_bytes + (size_t)warps * mrpop::warp_scratch_bytes();
-    const cudaError_t err = mrpop::batch_occupancy(g.arms, mode, g.seg, g.spl, smem, warps, &nb);
+    cudaError_t err = cudaSuccess;
+    if (mode == mrpop::kBatchNarrow && g.arms > 1)  // (raises the rows kernel's shared-memory limit too)
+        err = mrpop::batch_occupancy(g.arms, mrpop::kBatchRows, g.seg, g.spl, smem, warps, &nb);
+    if (err == cudaSuccess) err = mrpop::batch_occupancy(g.arms, mode, g.seg, g.spl, smem, warps, &nb);
     *out = (int)std::max(1LL, std::min<long long>((long long)sms * std::max(nb, 1), g.n_chunks));
     return err;
 }
@@ -200,7 +211,7 @@ mrpop_status mrpop_batch_create(const mrpop_batch_item *items, int64_t n_items, 
             if (ps.empty()) continue;
             g.n_items = (int64_t)ps.size();
             err = cudaMalloc(&g.d_items, ps.size() * sizeof(mrpop::EdgeParams));
-            if (err == cudaSuccess) err = cudaMalloc(&g.d_work, 3 * sizeof(unsigned long long));
+            if (err == cudaSuccess) err = cudaMalloc(&g.d_work, 4 * sizeof(unsigned long long));
             if (err == cudaSuccess)
                 err = cudaMemcpy(g.d_items, ps.data(), ps.size() * sizeof(mrpop::EdgeParams), cudaMemcpyHostToDevice);
             if (err == cudaSuccess) err = set_chunks(g, kChunkEdges);

@@ -145,7 +145,7 @@ struct EdgeParams {
     uint16_t *spairs;           // split pipeline: per-edge arm-pair joints [SPL][num_pairs(A)] (kPairSlots reserved)
     int32_t *snseg;             // segmented rules: per-edge segment count (-1: too many), from segment 0
     int32_t *sdone;             // segmented rules: per-edge verdict written
-    unsigned long long *work;   // split kernels: next-edge counters {broad, narrow}, zero before each launch
+    unsigned long long *work;   // split kernels: next-edge counters {broad, narrow, rows}, zero before each launch
     float4 grp[11];             // detailed sub-group bounds in their joint frame (+margin)
     float4 hsub[3];             // bounds of the hand group's three parts in the joint-7 frame (+margin)
     const uint32_t *row5;       // forearm-hand rows table (kRow5N6 x kRow5N7 bits), or nullptr
@@ -729,6 +729,15 @@ __device__ __forceinline__ uint32_t row_mask(uint32_t sm, bool quirk) {
     return m;
 }
 
+// Rows whose targets are the forearm's spheres alone.
+constexpr uint32_t forearm_rows() {
+    uint32_t m = 0;
+    for (int r = 0; r < kDetRows; r++)
+        if (det_joint(det_row_hi(r)) == 5) m |= 1u << r;
+    return m;
+}
+constexpr uint32_t kForearmRows = forearm_rows();
+
 // Row bookkeeping of the detailed self check, per sphere index i:
 //   first[q][i]  rows whose first-read sphere is i (q = 1: the composite
 //                robots' reading, sphere r; q = 0: sphere first(r))
@@ -908,9 +917,9 @@ struct LaneCtx {
 // Lanes 0..lane: a hit on any of them settles the lane's sample.
 __device__ __forceinline__ uint32_t lanes_upto(int lane) { return (2u << lane) - 1u; }
 
-// Joint j of one arm, frame T: env tests of an env-flagged joint, stash of the
-// first spheres of flagged rows, and the row tests whose targets are here
-// (screened by the target group's bound).
+// Joint j of one arm, frame T: env tests of an env-flagged joint (lane_env);
+// stash of the first spheres of flagged rows, and the row tests whose targets
+// are here, screened by the target group's bound (lane_rows).
 __device__ __forceinline__ void lane_env(int j, const EdgeParams &P, const Xf &T, LaneCtx &c, const float4 *S,
                                          const SceneLayout &L) {
     // every lane takes part in the env screening (warp-wide votes inside)
@@ -998,59 +1007,202 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
     }
 }
 
-// Lane-parallel detailed check of this lane's sample, called by every lane of
-// the warp (de = ds = false for a lane without a candidate sample): every
-// arm's chain is rebuilt in registers; env tests of env-flagged joints
-// (screened warp-wide per sub-group) and the intra-arm rows of self-flagged
-// joints run as the frames stream by (the first sphere of each row is stashed
-// until its targets come).  Once a lane's test has fired, the lanes above it
-// stop: random edges that collide mostly do so at their first samples, and
-// the rest of such an edge's tests is not needed.  Returns true if a test
-// fired.
-// ONE: only arm one_arm's chain (the arm-per-warp kernel).
-template <int A, bool ONE = false>
-__device__ __forceinline__ bool narrow_lane(const EdgeParams &P, WarpScratch &W, const float4 *S,
-                                                const SceneLayout &L, const float4 *det_tab, int seg, int k,
-                                                uint64_t envw, uint64_t selfw, bool de, bool ds, int one_arm = 0) {
-    const int lane = threadIdx.x & 31;
-    LaneCtx c;
-    c.quirk = (!P.single && !(P.flags & kExactBit)) ? 1 : 0;
-    c.hit = false;
-    MRPOP_PHASE_START();
-#pragma unroll 1
-    for (int a = ONE ? one_arm : 0; a < (ONE ? one_arm + 1 : A); a++) {
-        if (!__any_sync(kFull, de || ds)) break;
-        c.em = de ? (uint32_t)(envw >> (8 * a)) & 0xffu : 0u;
-        const uint32_t sm = ds ? (uint32_t)(selfw >> (8 * a)) & 0xffu : 0u;
-        c.rm = sm ? row_mask(sm, c.quirk != 0) : 0u;
-        const int qa = 7 * (P.single ? 0 : a);
-        if (P.row5 && (c.rm & row5_rows(c.quirk)) &&
-            row5_apart(P.row5, sample_q1(W, P.rule, seg, qa + 5, k), sample_q1(W, P.rule, seg, qa + 6, k)))
-            c.rm &= ~row5_rows(c.quirk);
-        // the arm's chain is walked only if some lane has env or row tests on it
-        if (!__any_sync(kFull, c.em | c.rm)) continue;
-        const uint32_t before = __ballot_sync(kFull, c.hit);
-        Xf T;
-        load_base(T, P.base[a]);
-#pragma unroll 1
-        for (int j = 0; j < kNumJoints; j++) {
-            if (j > 0) joint_step_rt(T, sample_q1(W, P.rule, seg, qa + j - 1, k), j);
-            MRPOP_PHASE(P, 8);
-            lane_env(j, P, T, c, S, L);
-            MRPOP_PHASE(P, 9);
-            lane_rows<A>(j, P, T, c, W, det_tab, lane);
-            MRPOP_PHASE(P, 10);
-            const uint32_t hb = __ballot_sync(kFull, c.hit);
-            if (hb != before) {
-                if (hb & lanes_upto(lane)) {
-                    c.em = c.rm = 0;
-                    de = ds = false;
-                }
-                if (!__any_sync(kFull, c.em | c.rm)) break;
-            }
+// ---------------------------------------------------------------------------
+// Screen of the detailed intra-arm rows whose first sphere is on joints 0..4
+// (the "low" rows: 0..16 in the composite reading, 0..12 by sphere index).
+// They are flagged whenever the arm's big approx spheres overlap, in most
+// edges, and hardly ever fire; finding that out by walking the chain costs a
+// row x sub-group test per lane and joint.  Here one pass covers every arm
+// with low rows flagged: the warp's lanes are (arm, sub-interval of the slot's
+// samples), each evaluates the arm at its sub-interval's middle and tests each
+// low row's first sphere against the target sub-groups' bounds, grown by how
+// far the joints between can move the target within the sub-interval.  The
+// target centres are carried inward frame by frame (F_j Rz(q_j) from joint 7
+// to joint 2), so that the first spheres are compile-time constants of their
+// own frames and the base and joint 1 do not enter.  Of the arms with low rows
+// flagged, five in six (5 arms) to half (one arm) need no walk after it.
+// Measured with the rows in a kernel of their own, detailed phase: 262144
+// 5-arm edges x 64 samples 4.47 -> 3.35 ms, 65536 shortcut edges 3.82 -> 2.55
+// ms, 65536 4-arm edges 505 -> 457 us, 30011 one-arm edges 147 -> 139 us.
+// ---------------------------------------------------------------------------
+struct RowScreen {
+    uint32_t rows;  // this lane's (arm, sub-interval): rows that may fire
+    uint32_t arms;  // arms screened, in lane order
+    int sub;        // sub-intervals per arm
+};
+
+// Largest distance of the centre of target sub-group 5 + t from joint j's
+// axis (2..7) over all poses, in metres, rounded up; 0 where joint j does not
+// move it against joints 0..4.  In frame 4 a target of joint 5 at (rho, c_z)
+// from axis 5 is within hypot(0.0825, 0.384 + c_z) + rho of the origin, one
+// further out within 0.393 m plus its distance from joint 6's origin; every
+// frame inward adds its translation (0.0825, 0.316).
+__host__ __device__ __forceinline__ constexpr float row_reach(int t, int j) {
+    constexpr float kReach[6][6] = {
+        //  j = 2   3       4       5       6       7
+        {0.860f, 0.544f, 0.461f, 0.067f, 0.000f, 0.000f},  // 5
+        {0.630f, 0.313f, 0.230f, 0.027f, 0.000f, 0.000f},  // 6
+        {0.790f, 0.473f, 0.391f, 0.089f, 0.000f, 0.000f},  // 7
+        {0.837f, 0.520f, 0.437f, 0.044f, 0.044f, 0.000f},  // 8
+        {0.955f, 0.638f, 0.556f, 0.162f, 0.162f, 0.044f},  // 9
+        {0.981f, 0.664f, 0.581f, 0.188f, 0.188f, 0.002f}}; // 10
+    return kReach[t][j - 2];
+}
+
+// Target centre p through joint J: F_J Rz(q) p (see joint_step for F_J).
+template <int J>
+__device__ __forceinline__ void carry_inward(float3 &p, float c, float s) {
+    const float x = c * p.x - s * p.y, y = s * p.x + c * p.y;
+    if constexpr (J == 2) p = make_float3(x, p.z, -y);
+    else if constexpr (J == 5) p = make_float3(x - 0.0825f, p.z + 0.384f, -y);
+    else if constexpr (J == 3) p = make_float3(x, -p.z - 0.316f, y);
+    else if constexpr (J == 4) p = make_float3(x + 0.0825f, -p.z, y);
+    else if constexpr (J == 6) p = make_float3(x, -p.z, y);
+    else p = make_float3(x + 0.088f, -p.z, y);  // J == 7
+}
+
+// The targets' centres and squared reaches (bound + the row's sphere radius +
+// motion) in the current frame.
+struct RowTargets {
+    float3 c[6];   // sub-groups 5..10
+    float mv[6];   // motion within the sub-interval against the current frame
+    float rr[6];   // (bound + first sphere's radius + motion)^2 for the current joint
+    template <int J>
+    __device__ __forceinline__ void step(float cq, float sq, float dq) {
+#pragma unroll
+        for (int t = 0; t < 6; t++) {
+            if (row_reach(t, J) == 0.0f) continue;
+            carry_inward<J>(c[t], cq, sq);
+            mv[t] = fmaf(dq, row_reach(t, J), mv[t]);
         }
     }
-    return c.hit;
+    __device__ __forceinline__ void reach(const EdgeParams &P, float r) {
+#pragma unroll
+        for (int t = 0; t < 6; t++) {
+            const float v = P.grp[5 + t].w + r + mv[t];
+            rr[t] = v * v;
+        }
+    }
+    // some sub-group of t0..t1 within reach of a sphere at (x, y, z)
+    template <int T0, int T1>
+    __device__ __forceinline__ bool near(float x, float y, float z) const {
+        bool n = false;
+#pragma unroll
+        for (int t = T0 - 5; t <= T1 - 5; t++) {
+            const float dx = c[t].x - x, dy = c[t].y - y, dz = c[t].z - z;
+            n |= dx * dx + dy * dy + dz * dz < rr[t];
+        }
+        return n;
+    }
+};
+
+// Every lane of the warp calls it.  sw: the lane's self flag words (0 for a
+// lane without a self candidate); arms_in: arms to screen.
+template <int A>
+__device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const WarpScratch &W, int seg, int k0, uint64_t sw,
+                                                 int quirk, uint32_t arms_in) {
+    const int lane = threadIdx.x & 31;
+    RowScreen out;
+    out.rows = kFull;
+    out.arms = 0;
+    out.sub = 32;
+    const uint32_t lo = __reduce_or_sync(kFull, (uint32_t)sw & 0x1f1f1f1fu);
+    const uint32_t hi = A > 4 ? __reduce_or_sync(kFull, (uint32_t)(sw >> 32) & 0x1fu) : 0u;
+    uint32_t joints = 0;
+#pragma unroll
+    for (int a = 0; a < A; a++) {
+        const uint32_t u = a < 4 ? lo >> (8 * a) & 0x1fu : hi;
+        if (u && (P.rigid & arms_in) >> a & 1) {
+            out.arms |= 1u << a;
+            joints |= u;
+        }
+    }
+    if (!out.arms) return out;
+    int arm = 0, sub = lane;
+    if (A > 1) {
+        const int n = __popc(out.arms);
+        out.sub = n == 1 ? 32 : n == 2 ? 16 : n == 3 ? 10 : n == 4 ? 8 : 6;
+        int ai = min(lane / out.sub, n - 1);
+        sub = min(lane - ai * out.sub, out.sub - 1);
+        uint32_t m = out.arms;
+        for (; ai > 0; ai--) m &= m - 1;
+        arm = __ffs(m) - 1;
+    }
+    // lanes ilo..ihi of the slot (lane i belongs to sub-interval i * sub / 32)
+    const int ilo = (32 * sub + out.sub - 1) / out.sub, ihi = (32 * (sub + 1) + out.sub - 1) / out.sub - 1;
+    const int klo = min(k0 + 1 + ilo, P.g), khi = min(k0 + 1 + ihi, P.g);
+    const float mid = 0.5f * (float)(klo + khi), half = 0.5f * (float)(khi - klo);
+    float q[7], dq[7], sum = 0.0f;  // joint 1 enters only the range check
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+        const int i = 7 * (P.single ? 0 : arm) + j;
+        q[j] = fmaf(mid, W.stepg[i], W.base[i]);
+        if (P.rule == kRuleBspline || P.rule == kRuleShortcut) q[j] = fmaf((float)seg, W.delta[i], q[j]);
+        dq[j] = fmaf(half, fabsf(W.stepg[i]), 1e-5f);
+        sum += fabsf(q[j]) + dq[j];
+    }
+    RowTargets t;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        t.c[i] = make_float3(P.grp[5 + i].x, P.grp[5 + i].y, P.grp[5 + i].z);
+        t.mv[i] = 0.0f;
+    }
+    uint32_t rows = quirk ? ~0x1ffffu : ~0x1fffu;
+    t.step<7>(__cosf(q[6]), __sinf(q[6]), dq[6]);
+    t.step<6>(__cosf(q[5]), __sinf(q[5]), dq[5]);
+    t.step<5>(__cosf(q[4]), __sinf(q[4]), dq[4]);
+#define MRPOP_NEAR(i, T0, T1) t.near<T0, T1>(kDet[i].x, kDet[i].y, kDet[i].z)
+    // composite reading: row r reads sphere r (first radii 0.06 at most)
+    if (quirk && joints >> 4) {
+        t.reach(P, 0.06f);
+        if (MRPOP_NEAR(13, 9, 10)) rows |= 1u << 13;
+        if (MRPOP_NEAR(14, 9, 10)) rows |= 1u << 14;
+        if (MRPOP_NEAR(15, 9, 10)) rows |= 1u << 15;
+        if (MRPOP_NEAR(16, 9, 10)) rows |= 1u << 16;
+    }
+    t.step<4>(__cosf(q[3]), __sinf(q[3]), dq[3]);
+    if (quirk && (joints >> 3 & 1)) {
+        t.reach(P, 0.06f);
+        if (MRPOP_NEAR(9, 5, 7)) rows |= 1u << 9;
+        if (MRPOP_NEAR(10, 9, 10)) rows |= 1u << 10;
+        if (MRPOP_NEAR(11, 5, 7)) rows |= 1u << 11;
+        if (MRPOP_NEAR(12, 9, 10)) rows |= 1u << 12;
+    }
+    t.step<3>(__cosf(q[2]), __sinf(q[2]), dq[2]);
+    if (joints >> 2 & 1) {
+        t.reach(P, 0.06f);
+        if (quirk) {
+            if (MRPOP_NEAR(5, 5, 7)) rows |= 1u << 5;
+            if (MRPOP_NEAR(6, 9, 10)) rows |= 1u << 6;
+            if (MRPOP_NEAR(7, 5, 7)) rows |= 1u << 7;
+            if (MRPOP_NEAR(8, 9, 10)) rows |= 1u << 8;
+        } else {  // spheres 5..8, a forearm and a hand row each
+            if (MRPOP_NEAR(5, 5, 7)) rows |= 1u << 5;
+            if (MRPOP_NEAR(5, 9, 10)) rows |= 1u << 6;
+            if (MRPOP_NEAR(6, 5, 7)) rows |= 1u << 7;
+            if (MRPOP_NEAR(6, 9, 10)) rows |= 1u << 8;
+            if (MRPOP_NEAR(7, 5, 7)) rows |= 1u << 9;
+            if (MRPOP_NEAR(7, 9, 10)) rows |= 1u << 10;
+            if (MRPOP_NEAR(8, 5, 7)) rows |= 1u << 11;
+            if (MRPOP_NEAR(8, 9, 10)) rows |= 1u << 12;
+        }
+    }
+    t.step<2>(__cosf(q[1]), __sinf(q[1]), dq[1]);
+    if (joints >> 1 & 1) {
+        t.reach(P, 0.06f);
+        if (MRPOP_NEAR(1, 5, 10)) rows |= 1u << 1;
+        if (MRPOP_NEAR(2, 5, 10)) rows |= 1u << 2;
+        if (MRPOP_NEAR(3, 5, 10)) rows |= 1u << 3;
+        if (MRPOP_NEAR(4, 5, 10)) rows |= 1u << 4;
+    }
+    if (joints & 1u) {
+        t.reach(P, 0.08f);
+        // sphere 0 of the base lies on joint 1's axis, 0.283 m below its frame
+        if (t.near<5, 10>(0.0f, 0.0f, kDet[0].z - 0.333f)) rows |= 1u;
+    }
+#undef MRPOP_NEAR
+    if (sum <= kRegularRad) out.rows = rows;  // (false for NaN)
+    return out;
 }
 
 // Lower arm, joint j (flagged for this lane): its spheres from index `from` on
@@ -1131,75 +1283,198 @@ __device__ __forceinline__ uint32_t joint_groups(uint32_t jm) {
     return (jm & 0x1fu) | (jm >> 5 & 1u) * 0xe0u | (jm >> 6 & 1u) << 8 | (jm >> 7 & 1u) * 0x600u;
 }
 
-// Arm-vs-arm detailed test (panda_four.cuh:415-453) of arms a < b for this
-// lane's sample; every lane of the warp calls it.  sma: the lane's self-flagged
-// joints of arm a to test (0: the lane only keeps the others company), jb: the
-// joints of arm b.  Both are already cut to the joints that some approx sphere
-// pair's swept bounds connect in these 32 samples (the broad phase's screen):
-// a joint's detailed spheres lie inside its approx spheres but for 0.6 mm, and
-// those bounds carry 1 mm each.  Arm b's sub-group centres are placed first;
-// arm a's spheres are then tested against them by sub-group and one by one,
-// so that only spheres that can reach arm b are stashed (most lanes stash
-// none, and arm b's chain is walked again only if some lane did).  Returns
-// true if a test fired.
-// Bound by instruction issue.  Against one that screened all 121 sub-group
-// pairs of every arm pair and stashed every flagged sphere 16 at a time (with
-// the lanes above a hit going on): 262144 5-arm edges x 64 samples 11.90 ->
-// 10.26 ms, 65536 shortcut edges 7.36 -> 6.37 ms, 128 uneven instances 15.4 ->
-// 12.5 ms, 300 5-arm extend checks 120 -> 104 us.
-__device__ __forceinline__ bool cross_pair(const EdgeParams &P, WarpScratch &W, int seg, int k, int a, int b,
-                                           uint32_t sma, uint32_t jb) {
+// Shared words of a CTA whose warps take one arm each (armwise_kernel).
+struct ArmShare {
+    unsigned long long env[2][32], self[2][32];  // [slot][lane] flag words of the segment
+    unsigned int hits[2];                        // [slot] lanes whose sample collided
+    unsigned int pm[2][num_pairs(kMaxArms)];     // [slot][pair] joints connected by swept bounds
+    unsigned int next[3];                        // arm pairs handed out: broad, narrow slot 0, slot 1
+};
+
+// The next arm pair for this warp from counter *c (lane 0 takes it).
+__device__ __forceinline__ int take_pair(unsigned int *c, int lane) {
+    unsigned int p = 0;
+    if (lane == 0) p = atomicAdd(c, 1u);
+    return (int)__shfl_sync(kFull, p, 0);
+}
+
+// Detailed check of one slot: this lane's sample is k0 + lane + 1 (lanes past
+// the segment's last sample keep the others company on it, so that the warp's
+// merged bounds stay on real samples); dE, dS: it is an env / self candidate.
+// Every lane of the warp calls it.  Returns the lanes whose test fired, of
+// which the lowest counts: once a lane's test has fired the lanes above it
+// stop.
+//
+// Every test is a walk along one arm's joint chain with all lanes in step, and
+// one loop runs them all (a job each), so that the kernel holds the chain step
+// once and its code stays within the instruction cache.
+//   arm      obstacles against the env-flagged joints (warp-wide screens), and
+//            the intra-arm rows left by screen_rows and the forearm-hand table
+//   centres, stash, probe
+//            one arm pair a < b (panda_four.cuh:415-453), cut to the joints
+//            that some approx sphere pair's swept bounds connect in the slot
+//            (pms: lane p holds pair p's; a joint's detailed spheres lie inside
+//            its approx spheres but for 0.6 mm, and those bounds carry 1 mm
+//            each).  Arm b's sub-group centres are placed first; arm a's
+//            spheres are tested against them by sub-group and one by one, so
+//            that only spheres that can reach arm b are stashed; arm b is
+//            walked again only if some lane stashed any.
+// Bound by instruction issue.  Against the first form of the arm-pair test
+// (all 121 sub-group pairs of every arm pair screened, every flagged sphere
+// stashed, lanes above a hit going on): 262144 5-arm edges x 64 samples 11.90
+// -> 10.26 ms, 65536 shortcut edges 7.36 -> 6.37 ms.
+//
+// STAGE: which tests this kernel runs.  The split pipeline's composite kernels
+// run the rows, which seldom fire, in a kernel of their own after the others
+// (rows_kernel): with all of them the narrow kernel's code, 51 KB, missed the
+// SM's instruction cache (15 times the misses of a 45 KB build; 65536 4-arm
+// edges 505 -> 603 us), and random edges that collide mostly do so with an
+// obstacle or another arm at their first samples.
+// ONE (armwise_kernel): only arm one_arm's env and row tests, then the slot's
+// arm pairs one at a time to whichever warp of the CTA is free (X->next); hits
+// are shared through X->hits (a stale read only costs tests).
+constexpr int kStageAll = 0, kStageEnvPairs = 1, kStageRows = 2;
+
+template <int A, bool ONE = false, int STAGE = kStageAll>
+__device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch &W, const float4 *S,
+                                                const SceneLayout &L, const float4 *det_tab, int seg, int k0,
+                                                uint64_t ew, uint64_t sw, bool dE, bool dS, uint32_t pms,
+                                                int one_arm = 0, ArmShare *X = nullptr, int slot = 0) {
     const int lane = threadIdx.x & 31;
-    const uint32_t uj = __reduce_or_sync(kFull, sma);
-    if (!uj) return false;
-    const int top_a = 31 - __clz(uj), top_b = 31 - __clz(jb);
-    const uint32_t gb = joint_groups(jb);
-    {
-        Xf T;
-        load_base(T, P.base[b]);
+    const int k = min(k0 + lane + 1, P.g);
+    static_assert(!ONE || STAGE == kStageAll, "the arm-per-warp kernel runs every test");
+    constexpr bool with_env = STAGE != kStageRows, with_rows = STAGE != kStageEnvPairs;
+    constexpr bool with_pairs = A > 1 && STAGE != kStageRows;
+    constexpr int kArm = 0, kCentres = 1, kStash = 2, kProbe = 3;  // jobs
+    const int arm0 = ONE ? one_arm : 0, arm1 = ONE ? one_arm + 1 : A;
+    LaneCtx c;
+    c.quirk = (!P.single && !(P.flags & kExactBit)) ? 1 : 0;
+    c.hit = false;
+    bool act = dE || dS;  // this lane's sample is not settled
+    bool pair_phase = false;
+    int arm_next = arm0;
+    RowScreen rs = {kFull, 0u, 32};
+    if (with_rows) rs = screen_rows<A>(P, W, seg, k0, dS ? sw : 0, c.quirk, ONE ? 1u << one_arm : kFull);
+    // the arm pair in hand: its state (0: none, 1: centres placed, 2: stashed,
+    // 3: probed), arms, joints, and the lane's stash
+    int xs = 0, pa = 0, pb = 0, from = 0, n = 0, next = 0;
+    uint32_t pairs = with_pairs && !ONE ? __ballot_sync(kFull, pms != 0) : 0u, jb = 0, uj = 0, sma = 0;
 #pragma unroll 1
-        for (int j = 0;; j++) {
-            if (jb >> j & 1u) {
-#pragma unroll 1
-                for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
-                    const float3 c = place_reg(T, P.grp[g]);
-                    W.lanes.cross.gc[g][0][lane] = c.x;
-                    W.lanes.cross.gc[g][1][lane] = c.y;
-                    W.lanes.cross.gc[g][2][lane] = c.z;
+    for (;;) {
+        // the next job: its kind, arm and last joint (the same in every lane)
+        int job, arm, top;
+        if (with_pairs && pair_phase) {
+            if (xs == 2 && __any_sync(kFull, act && n > 0)) {
+                job = kProbe;
+                xs = 3;
+            } else {
+                if (xs >= 2) {  // this stash is done: the spheres left out, if any
+                    from = act ? next : kNumDet;
+                    xs = __any_sync(kFull, from < kNumDet) ? 1 : 0;
+                }
+                if (xs == 1) {
+                    job = kStash;
+                    xs = 2;
+                    n = 0;
+                    next = kNumDet;
+                } else {
+                    uint32_t m = 0, rest = pairs;
+                    if (ONE) {
+                        const int t = take_pair(&X->next[1 + slot], lane);
+                        for (int i = 0; i < t && rest; i++) rest &= rest - 1;
+                    }
+                    if (!rest) break;
+                    const int p = __ffs(rest) - 1;
+                    if (!ONE) pairs &= pairs - 1;
+                    m = ONE ? X->pm[slot][p] : __shfl_sync(kFull, pms, p);
+                    pair_arms<A>(p, pa, pb);
+                    jb = m >> 8;
+                    sma = act && dS ? (uint32_t)(sw >> (8 * pa)) & m & 0xffu : 0u;
+                    uj = __reduce_or_sync(kFull, sma);
+                    if (!uj) continue;
+                    from = sma ? 0 : kNumDet;
+                    job = kCentres;
+                    xs = 1;
                 }
             }
-            if (j == top_b) break;
-            joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * b + j, k), j + 1);
+            arm = job == kStash ? pa : pb;
+            top = 31 - __clz(job == kStash ? uj : jb);
+        } else {
+            if (arm_next == arm1) {
+                if (!with_pairs) break;
+                pair_phase = true;
+                if (ONE) pairs = __ballot_sync(kFull, lane < num_pairs(A) && X->pm[slot][lane] != 0);
+                continue;
+            }
+            arm = arm_next++;
+            c.em = c.rm = 0;
+            top = -1;
+            if (with_env) {
+                if (act && dE) c.em = (uint32_t)(ew >> (8 * arm)) & 0xffu;
+                const uint32_t u = __reduce_or_sync(kFull, c.em);
+                if (u) top = 31 - __clz(u);
+            }
+            if (with_rows) {
+                const uint32_t sm = act && dS ? (uint32_t)(sw >> (8 * arm)) & 0xffu : 0u;
+                if (sm) c.rm = row_mask(sm, c.quirk != 0);
+                const int q6 = 7 * (P.single ? 0 : arm) + 5;
+                if (P.row5 && (c.rm & row5_rows(c.quirk)) &&
+                    row5_apart(P.row5, sample_q1(W, P.rule, seg, q6, k), sample_q1(W, P.rule, seg, q6 + 1, k)))
+                    c.rm &= ~row5_rows(c.quirk);
+                if (rs.arms >> arm & 1u)
+                    c.rm &= __shfl_sync(kFull, rs.rows,
+                                        __popc(rs.arms & ((1u << arm) - 1u)) * rs.sub + (lane * rs.sub >> 5));
+                const uint32_t u = __reduce_or_sync(kFull, c.rm);
+                if (u) top = max(top, u & ~kForearmRows ? 7 : 5);
+            }
+            if (top < 0) continue;
+            job = kArm;
         }
+        // walk the arm's chain
+        const uint32_t before = __ballot_sync(kFull, c.hit);
+        const uint32_t gb = joint_groups(jb);
+        Xf T;
+        load_base(T, P.base[arm]);
+#pragma unroll 1
+        for (int j = 0;; j++) {
+            if (with_pairs && job != kArm) {
+                if (job == kStash) {
+                    if ((sma >> j & 1u) && next == kNumDet && from < det_first(j + 1))
+                        stash_joint(j, P, T, gb, from, n, next, W, lane);
+                } else if (jb >> j & 1u) {
+                    if (job == kCentres) {
+#pragma unroll 1
+                        for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
+                            const float3 ctr = place_reg(T, P.grp[g]);
+                            W.lanes.cross.gc[g][0][lane] = ctr.x;
+                            W.lanes.cross.gc[g][1][lane] = ctr.y;
+                            W.lanes.cross.gc[g][2][lane] = ctr.z;
+                        }
+                    } else if (act && !c.hit && n > 0) {
+                        probe_joint(j, T, n, c.hit, W, lane);
+                    }
+                }
+            } else {
+                if (with_env) lane_env(j, P, T, c, S, L);
+                if (with_rows) lane_rows<A>(j, P, T, c, W, det_tab, lane);
+                const uint32_t hb = __ballot_sync(kFull, c.hit);
+                if (hb != before) {
+                    if (hb & lanes_upto(lane)) c.em = c.rm = 0;
+                    if (!__any_sync(kFull, c.em | c.rm)) break;
+                }
+            }
+            if (j == top) break;
+            joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * (P.single ? 0 : arm) + j, k), j + 1);
+        }
+        uint32_t hb = __ballot_sync(kFull, c.hit);
+        if (ONE) {
+            if (lane == 0 && hb != before) atomicOr(&X->hits[slot], hb);
+            hb |= *(const volatile unsigned int *)&X->hits[slot];
+        }
+        act = act && !(hb & lanes_upto(lane));
+        if (!__any_sync(kFull, act)) break;
     }
-    bool hit = false;
-    int from = sma ? 0 : kNumDet;
-    do {
-        int n = 0, next = kNumDet;
-        {
-            Xf T;
-            load_base(T, P.base[a]);
-#pragma unroll 1
-            for (int j = 0;; j++) {
-                if ((sma >> j & 1u) && next == kNumDet && from < det_first(j + 1))
-                    stash_joint(j, P, T, gb, from, n, next, W, lane);
-                if (j == top_a) break;
-                joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * a + j, k), j + 1);
-            }
-        }
-        if (__any_sync(kFull, n > 0)) {
-            Xf T;
-            load_base(T, P.base[b]);
-#pragma unroll 1
-            for (int j = 0;; j++) {
-                if ((jb >> j & 1u) && !hit && n > 0) probe_joint(j, T, n, hit, W, lane);
-                if (j == top_b) break;
-                joint_step_rt(T, sample_q1(W, P.rule, seg, 7 * b + j, k), j + 1);
-            }
-        }
-        from = hit ? kNumDet : next;
-    } while (__any_sync(kFull, from < kNumDet));
-    return hit;
+    return __ballot_sync(kFull, c.hit);
 }
 
 // ---------------------------------------------------------------------------
@@ -1371,7 +1646,7 @@ __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W
 // Detailed phase of one segment: every candidate sample in parallel, one lane
 // each (samples k0 + 1 ..; k0 = 32 for the second warp of a pair).  Returns
 // the 0-based index (from k0) of the first colliding sample, or 64.
-template <int A, int SPL>
+template <int A, int SPL, int STAGE = kStageAll>
 __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &W, const float4 *S,
                                               const SceneLayout &L, const float4 *det_tab, int seg, int lane,
                                               const uint64_t (&envw)[SPL], const uint64_t (&selfw)[SPL],
@@ -1385,34 +1660,9 @@ __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &
         const int bit = lane + 32 * s;
         const bool dE = cand_env >> bit & 1ull, dS = cand_self >> bit & 1ull;
         const uint64_t ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
-        // every lane walks the arms (warp-wide screening inside); lanes
-        // without a candidate sample keep the others company on sample
-        // min(k, g), so that the warp's merged bounds stay on real samples
-        const int k = k0 + bit + 1 <= P.g ? k0 + bit + 1 : P.g;
-        bool h = narrow_lane<A>(P, W, S, L, det_tab, seg, k, ew, sw, dE, dS);
-        MRPOP_PHASE(P, 5);
-        MRPOP_COUNT_LANES(14, dE || dS);
-        if (A > 1) {
-            // the arm pairs that the broad phase's swept bounds connect
-            // (every vote is a statement of its own: all lanes take part)
-            const uint32_t pms = s == 0 ? pm[0] : pm[SPL - 1];
-            uint32_t pairs = __ballot_sync(kFull, pms != 0);
-            uint32_t hb = __ballot_sync(kFull, h);
-            bool act = dS && !(hb & lanes_upto(lane));
-            while (pairs && __any_sync(kFull, act)) {
-                MRPOP_COUNT_W(15, 1);
-                const int p = __ffs(pairs) - 1;
-                pairs &= pairs - 1;
-                const uint32_t m = __shfl_sync(kFull, pms, p);
-                int a, b;
-                pair_arms<A>(p, a, b);
-                h |= cross_pair(P, W, seg, k, a, b, act ? (uint32_t)(sw >> (8 * a)) & m & 0xffu : 0u, m >> 8);
-                hb = __ballot_sync(kFull, h);
-                act = act && !(hb & lanes_upto(lane));
-            }
-        }
-        MRPOP_PHASE(P, 6);
-        hits |= (uint64_t)__ballot_sync(kFull, h) << (32 * s);
+        const uint32_t hb = narrow_slot<A, false, STAGE>(P, W, S, L, det_tab, seg, k0 + 32 * s, ew, sw, dE, dS,
+                                                         s == 0 ? pm[0] : pm[SPL - 1]);
+        hits |= (uint64_t)hb << (32 * s);
         if (hits) break; // later slots hold only later samples
     }
     return hits ? __ffsll((long long)hits) - 1 : 64;
@@ -1619,20 +1869,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 // verdicts are those of the one-warp kernels.  The lower arm's spheres of a
 // pair are read from the warp that placed them instead of being placed again.
 // ---------------------------------------------------------------------------
-struct ArmShare {
-    unsigned long long env[2][32], self[2][32];  // [slot][lane] flag words of the segment
-    unsigned int hits[2];                        // [slot] lanes whose sample collided
-    unsigned int pm[2][num_pairs(kMaxArms)];     // [slot][pair] joints connected by swept bounds
-    unsigned int next[3];                        // arm pairs handed out: broad, narrow slot 0, slot 1
-};
-
-// The next arm pair for this warp from counter *c (lane 0 takes it).
-__device__ __forceinline__ int take_pair(unsigned int *c, int lane) {
-    unsigned int p = 0;
-    if (lane == 0) p = atomicAdd(c, 1u);
-    return (int)__shfl_sync(kFull, p, 0);
-}
-
 template <int A, int SPL>
 __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char *wbase, const float4 *S,
                                              const SceneLayout &L, const float4 *det_tab, long long e, int dof,
@@ -1754,40 +1990,14 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                               cand_self);
 #pragma unroll 1
             for (int s = 0; s < SPL; s++) {
-                // hits found so far by any warp: a hit in an earlier slot
-                // settles the edge, one at or below a lane settles that lane
-                // (a stale read only costs tests that are not needed).  Other
-                // warps, and this warp's lane 0, write the words meanwhile, so
-                // the branch takes lane 0's reading for the whole warp
-                const volatile unsigned int *hits = X.hits;
-                if (s > 0 && __shfl_sync(kFull, hits[0], 0)) break;
+                // a hit that some warp found in an earlier slot settles the
+                // edge.  Other warps write the word meanwhile, so the branch
+                // takes lane 0's reading for the whole warp
+                if (s > 0 && __shfl_sync(kFull, *(const volatile unsigned int *)&X.hits[0], 0)) break;
                 const int bit = lane + 32 * s;
                 const bool dE = cand_env >> bit & 1ull, dS = cand_self >> bit & 1ull;
-                const int k = bit + 1 <= g ? bit + 1 : g;
                 const uint64_t ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
-                const bool open = !(hits[s] & lanes_upto(lane));
-                unsigned int hb = __ballot_sync(
-                    kFull, narrow_lane<A, true>(P, W, S, L, det_tab, seg, k, ew, sw, dE && open, dS && open, arm));
-                if (lane == 0 && hb) atomicOr(&X.hits[s], hb);
-                // the slot's connected arm pairs, one at a time to whichever
-                // warp is free
-                if (A > 1 && __any_sync(kFull, dS)) {
-                    unsigned int *next = &X.next[1 + s];
-                    const uint32_t live = __ballot_sync(kFull, lane < num_pairs(A) && X.pm[s][lane] != 0);
-                    for (int t = take_pair(next, lane); t < __popc(live); t = take_pair(next, lane)) {
-                        const bool act = dS && !((hits[s] | hb) & lanes_upto(lane));
-                        uint32_t rest = live;
-                        for (int i = 0; i < t; i++) rest &= rest - 1;
-                        const int p = __ffs(rest) - 1;
-                        const uint32_t m = X.pm[s][p];
-                        int a, b;
-                        pair_arms<A>(p, a, b);
-                        const uint32_t sma = act ? (uint32_t)(sw >> (8 * a)) & m & 0xffu : 0u;
-                        const unsigned int h2 = __ballot_sync(kFull, cross_pair(P, W, seg, k, a, b, sma, m >> 8));
-                        if (lane == 0 && h2) atomicOr(&X.hits[s], h2);
-                        hb |= h2;
-                    }
-                }
+                narrow_slot<A, true>(P, W, S, L, det_tab, seg, 32 * s, ew, sw, dE, dS, 0u, arm, &X, s);
             }
             __syncthreads();
             const uint64_t hits = (uint64_t)X.hits[0] | (SPL > 1 ? (uint64_t)X.hits[1] << 32 : 0ull);
@@ -1928,38 +2138,56 @@ __device__ __forceinline__ void broad_edge(const EdgeParams &P, WarpScratch &W, 
     __syncwarp();
 }
 
-template <int A, int SPL, bool SEG>
+// The detailed phase of edge e.  One arm: all of it, in one kernel.  Composite
+// checks: the obstacles and arm pairs (STAGE kStageEnvPairs, narrow_kernel),
+// then the intra-arm rows (kStageRows, rows_kernel) of the samples below the
+// first hit; between the two P.smasks[2 * e] says whether a sample has hit and
+// P.smasks[2 * e + 1] which samples are left.
+template <int A, int SPL, bool SEG, int STAGE>
 __device__ __forceinline__ void narrow_edge(const EdgeParams &P, WarpScratch &W, const float4 *S, const SceneLayout &L,
                                             const float4 *det_tab, long long e, int dof, int g, int lane,
                                             bool staged) {
-    const uint64_t cand_env = P.smasks[2 * e], cand_self = P.smasks[2 * e + 1];
-    if (!(cand_env | cand_self)) return; // verdict written by the broad kernel
+    constexpr bool first_stage = STAGE == kStageEnvPairs, rows = STAGE == kStageRows;
+    const uint64_t m0 = P.smasks[2 * e], cand_self = P.smasks[2 * e + 1];
+    const uint64_t cand_env = rows ? 0ull : m0;
+    if (!(cand_env | cand_self)) return; // verdict written by an earlier kernel
     if (!staged) {
         if (lane == 0) {
             P.valid[e] = 0;
             P.first_hit[e] = -2;
+            if (first_stage) P.smasks[2 * e] = P.smasks[2 * e + 1] = 0;
         }
         return;
     }
+    uint64_t envw[SPL], selfw[SPL];
+    uint32_t pm[SPL];
+    uint32_t any_pair = 0;
+#pragma unroll
+    for (int s = 0; s < SPL; s++) {
+        pm[s] = !rows && lane < num_pairs(A) ? P.spairs[(e * SPL + s) * num_pairs(A) + lane] : 0u;
+        any_pair |= pm[s];
+    }
+    if (first_stage && !cand_env && !__any_sync(kFull, any_pair)) return; // rows alone
     const int r = SEG ? P.seg0 : 0;
     constexpr bool segmented = SEG;
     bool too_many;
     const int nseg = edge_setup(P, W, e, dof, g, lane, too_many);
     if (SEG && P.rule == kRuleConnect && r > 0) connect_advance(W, dof, r, lane);
-    uint64_t envw[SPL], selfw[SPL];
-    uint32_t pm[SPL];
 #pragma unroll
-    for (int s = 0; s < SPL; s++) {
-        load_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
-        pm[s] = lane < num_pairs(A) ? P.spairs[(e * SPL + s) * num_pairs(A) + lane] : 0u;
-    }
-    const int fb = narrow_segment<A, SPL>(P, W, S, L, det_tab, r, lane, envw, selfw, pm, cand_env, cand_self);
+    for (int s = 0; s < SPL; s++) load_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
+    const int fb =
+        narrow_segment<A, SPL, STAGE>(P, W, S, L, det_tab, r, lane, envw, selfw, pm, cand_env, cand_self);
     if (lane == 0) {
+        const uint64_t left = first_stage ? (fb < 64 ? cand_self & ((1ull << fb) - 1ull) : cand_self) : 0ull;
+        if (first_stage) {
+            P.smasks[2 * e] = fb < 64 ? 1ull : 0ull;
+            P.smasks[2 * e + 1] = left;
+        }
         if (fb < 64) {
             P.valid[e] = 0;
             P.first_hit[e] = r * g + fb + 1;
             if (segmented) P.sdone[e] = 1;
-        } else if (!segmented || r == nseg - 1) {
+        } else if (left == 0 && !(rows && m0) && (!segmented || r == nseg - 1)) {
             P.valid[e] = 1;
             P.first_hit[e] = -1;
             if (segmented) P.sdone[e] = 1;
@@ -1998,7 +2226,24 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     // visible) before reading its output
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (long long e = next_edge(P.work + 1, lane); e < P.n_edges; e = next_edge(P.work + 1, lane))
-        narrow_edge<A, SPL, SEG>(P, W, S, L, det_tab, e, dof, g, lane, staged);
+        narrow_edge<A, SPL, SEG, A == 1 ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, g, lane, staged);
+    if (A > 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the rows kernel
+}
+
+// Composite checks: the intra-arm rows, after the narrow kernel.
+template <int A, int SPL, bool SEG>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
+    rows_kernel(const __grid_constant__ EdgeParams P) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ float4 det_tab[kNumDet];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WarpScratch &W = reinterpret_cast<WarpScratch *>(smem_raw)[warp];  // no scene
+    for (int i = threadIdx.x; i < kNumDet; i += blockDim.x) det_tab[i] = c_det[i];
+    __syncthreads();
+    const SceneLayout L{};
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (long long e = next_edge(P.work + 2, lane); e < P.n_edges; e = next_edge(P.work + 2, lane))
+        narrow_edge<A, SPL, SEG, kStageRows>(P, W, nullptr, L, det_tab, e, 7 * A, P.g, lane, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -2027,6 +2272,8 @@ constexpr int kBatchBroad = 0, kBatchNarrow = 1, kBatchFused = 2;
 // Batch mode of the arm-per-warp kernel (whole edges from segment 0, a CTA of
 // A warps per edge): batch_armwise_kernel.
 constexpr int kBatchArmwise = 3;
+// The rows kernel of composite groups, after kBatchNarrow.
+constexpr int kBatchRows = 4;
 
 // One bulk copy of `bytes` from global to shared memory, completed on `bar`
 // in phase `parity`; bounded wait.  Every thread of the CTA calls it after a
@@ -2088,7 +2335,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
             }
             const uint32_t bytes = (uint32_t)(scene_layout(Ps.sc).total * sizeof(float4));
             staged = true;
-            if (bytes) {
+            if (bytes && MODE != kBatchRows) {
                 staged = stage_bulk(reinterpret_cast<float4 *>(smem_raw), Ps.scene, bytes, &bar, parity, Ps.status);
                 parity ^= 1u;
             }
@@ -2107,7 +2354,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
             if ((int)k >= ch.z) break;
             const long long e = (long long)ch.y + k;
             if (MODE == kBatchBroad) broad_edge<A, SPL, SEG>(P, W, S, L, e, dof, P.g, lane, staged);
-            else if (MODE == kBatchNarrow) narrow_edge<A, SPL, SEG>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
+            else if (MODE == kBatchNarrow)
+                narrow_edge<A, SPL, SEG, A == 1 ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
+            else if (MODE == kBatchRows)
+                narrow_edge<A, SPL, SEG, kStageRows>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
             else fused_edge<A, SPL>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
         }
         __syncthreads(); // every warp is done with this chunk (and instance)

@@ -11,7 +11,9 @@ namespace mrpop {
 // kFusedPair: the fused kernel with two warps per edge (granularity above 32);
 // timed as kFused.
 // kArmwise: the fused kernel with one warp per arm; timed as kFused.
-enum KernelKind { kFused = 0, kBroad = 1, kNarrow = 2, kFusedPair = 3, kArmwise = 4 };
+// kRows: the rows kernel that follows kNarrow for more than one arm; timed as
+// kNarrow.
+enum KernelKind { kFused = 0, kBroad = 1, kNarrow = 2, kFusedPair = 3, kArmwise = 4, kRows = 5 };
 
 // Launch a validator kernel for `arms` arms (1..5).  smem_bytes: dynamic
 // shared memory (staged scene + per-warp scratch).  Returns the launch error.
@@ -21,7 +23,7 @@ template <int A>
 cudaError_t launch_validate_arms(KernelKind kind, const EdgeParams &p, size_t smem_bytes, cudaStream_t stream);
 
 // Batch kernels (BatchParams: the instances of one arm count, samples per
-// lane and segmentation kind; mode = kBatchBroad / kBatchNarrow / kBatchFused,
+// lane and segmentation kind; mode = kBatchBroad / kBatchNarrow / kBatchRows / kBatchFused,
 // seg = segmented instances): resident CTAs per SM at a shared-memory size
 // and CTA size (warps of 32 threads, 1..kWarpsPerBlock), and a launch on
 // `grid` CTAs of `warps` warps.  The dispatchers switch on the arm count
@@ -62,7 +64,7 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
 size_t warp_scratch_bytes();
 
 // Scratch of the single-segment pipeline (staged flags, candidate masks and
-// arm-pair joints): its size, and its slices in p.  Two work counters
+// arm-pair joints): its size, and its slices in p.  Three work counters
 // in a 128-byte head (every edge's flag words start on an L2 line), then per
 // edge: 32 * spl samples x {env, self} flag words, {env, self} candidate
 // masks, kPairSlots arm-pair words and the segment state.

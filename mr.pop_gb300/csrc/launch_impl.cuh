@@ -69,6 +69,9 @@ const void *kernel_fn(KernelKind kind, bool seg) {
     switch (kind) {
     case kBroad: return seg ? (const void *)broad_kernel<A, SPL, true> : (const void *)broad_kernel<A, SPL, false>;
     case kNarrow: return seg ? (const void *)narrow_kernel<A, SPL, true> : (const void *)narrow_kernel<A, SPL, false>;
+    case kRows:
+        if constexpr (A > 1) return seg ? (const void *)rows_kernel<A, SPL, true> : (const void *)rows_kernel<A, SPL, false>;
+        return nullptr;
     case kFusedPair: return (const void *)pair_kernel<A>;
     case kArmwise: return (const void *)armwise_kernel<A, SPL>;
     default: return (const void *)validate_kernel<A, SPL>;
@@ -82,12 +85,14 @@ const void *batch_fn(int mode, bool seg) {
         switch (mode) {
         case kBatchBroad: return (const void *)batch_kernel<A, SPL, kBatchBroad, false>;
         case kBatchNarrow: return (const void *)batch_kernel<A, SPL, kBatchNarrow, false>;
+        case kBatchRows: return (const void *)batch_kernel<A, SPL, kBatchRows, false>;
         default: return (const void *)batch_kernel<A, SPL, kBatchFused, false>;
         }
     }
     switch (mode) {
     case kBatchBroad: return (const void *)batch_kernel<A, SPL, kBatchBroad, true>;
     case kBatchNarrow: return (const void *)batch_kernel<A, SPL, kBatchNarrow, true>;
+    case kBatchRows: return (const void *)batch_kernel<A, SPL, kBatchRows, true>;
     default: return (const void *)batch_kernel<A, SPL, kBatchFused, true>;
     }
 }
@@ -116,6 +121,8 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
         }
         kind = p.g > 32 ? kFusedPair : kFused;
     }
+    // the rows kernel reads no scene
+    if (kind == kRows) smem_bytes = (size_t)kWarpsPerBlock * sizeof(WarpScratch);
     const int spl = p.g > 32 ? 2 : 1;
     const bool seg = p.rule != 0;
     const void *fn = spl == 2 ? kernel_fn<A, 2>(kind, seg) : kernel_fn<A, 1>(kind, seg);
@@ -131,11 +138,11 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
     if (need < grid) grid = need;
     if (grid < 1) grid = 1;
     void *args[] = {(void *)&p};
-    if (kind != kNarrow)
+    if (kind != kNarrow && kind != kRows)
         return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(32 * kWarpsPerBlock), args, smem_bytes, stream);
-    // the narrow kernel follows the broad one as a programmatic dependent: its
-    // CTAs start (and stage the scene) while the broad kernel's last warps
-    // finish, and wait for it in griddepcontrol.wait
+    // the narrow kernel follows the broad one, and the rows kernel the narrow
+    // one, as a programmatic dependent: its CTAs start (and stage the scene)
+    // while the last warps before it finish, and wait in griddepcontrol.wait
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(32 * kWarpsPerBlock);

@@ -52,10 +52,10 @@ constexpr int64_t kFusedEdgesDefault = 4096;
 // arm-per-warp kernel (a CTA of A warps per edge; about as many edges as its
 // CTAs resident on the device at 5 arms).
 constexpr int64_t kArmwiseEdges = 456;
-// Work counters per group and wave: one per launch (split rounds + fused
+// Work counters per group and wave: one per launch (three per split round, fused
 // tail), zeroed together with the parameter upload so that no launch needs a
 // memset of its own.
-constexpr int kCountersPerGroup = 2 * mrpop::kSegRounds + 1;
+constexpr int kCountersPerGroup = 3 * mrpop::kSegRounds + 1;
 constexpr int kGroupKeys = 4 * MRPOP_MAX_ARMS;
 constexpr size_t kAlign = 256;
 
@@ -294,15 +294,18 @@ cudaError_t launch_wave(mrpop_server *s, mrpop_server::Slot &slot) {
         }
         const int rounds = seg ? mrpop::kSegRounds : 1;
         for (int rd = 0; rd < rounds && err == cudaSuccess; rd++) {
-            err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchBroad, rd, items, chunks, r.nc, work + 2 * rd,
+            err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchBroad, rd, items, chunks, r.nc, work + 3 * rd,
                              slot.stream);
             if (err == cudaSuccess)
                 err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchNarrow, rd, items, chunks, r.nc,
-                                 work + 2 * rd + 1, slot.stream);
+                                 work + 3 * rd + 1, slot.stream);
+            if (err == cudaSuccess && arms > 1)
+                err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchRows, rd, items, chunks, r.nc,
+                                 work + 3 * rd + 2, slot.stream);
         }
         if (err == cudaSuccess && seg)
             err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchFused, mrpop::kSegRounds, items, chunks, r.nc,
-                             work + 2 * rounds, slot.stream);
+                             work + 3 * rounds, slot.stream);
     }
     return err;
 }
