@@ -31,6 +31,8 @@
 // exact test is skipped only where the bounds prove it cannot fire, so the
 // set of tests that can fire -- and therefore every verdict -- is unchanged.
 #pragma once
+#include <type_traits>
+
 #include "panda_model.cuh"
 
 namespace mrpop {
@@ -38,6 +40,9 @@ namespace mrpop {
 #ifndef MRPOP_MIN_BLOCKS
 #define MRPOP_MIN_BLOCKS 3
 #endif
+// CTAs per SM of the broad kernels, whose warps need half the scratch: 24 warps
+// per SM at 80 registers in place of 18.
+constexpr int kBroadMinBlocks = 4;
 // Optional per-phase warp timers (development builds with
 // -DMRPOP_PHASE_TIMERS; compiled out otherwise): clock64() deltas of lane 0
 // accumulated into P.phase[i].
@@ -84,7 +89,6 @@ constexpr int kMaxArms = 5;
 constexpr int kMaxDof = 7 * kMaxArms;
 constexpr int kCrossStash = 8;         // per-lane arm-vs-arm candidate spheres
 constexpr float kCullMargin = 1e-3f;   // metres added to every bounding radius
-constexpr float kApproxMaxR = 0.176f;  // largest broad-phase sphere radius
 
 struct SceneCounts {
     int n_sph, n_cap, n_zcap, n_cub, n_zcub;
@@ -152,30 +156,43 @@ struct EdgeParams {
     float base[kMaxArms][12];   // row-major 3x4 per arm of this check
 };
 
-// Per-warp shared scratch.  The broad-phase and narrow-phase parts are never
-// live at the same time and share storage.
-struct WarpScratch {
+// Per-warp shared scratch: the edge's segment start and steps, and the broad
+// phase's or the narrow phase's storage (never live at the same time).
+struct EdgeScratch {
     float base[kMaxDof];   // segment start (accumulated for CONNECT)
     float stepg[kMaxDof];  // per-sample step (delta/g or vec/g)
     float delta[kMaxDof];  // per-segment step (B-spline / shortcut accumulation)
+};
+
+struct BroadPart {
+    float4 swept[kMaxArms][kNumApprox]; // per-arm swept bound of each approx sphere
+    float cur[kNumApprox][3][32];       // per-lane approx spheres of the current arm
+};
+
+// Scratch of the split pipeline's broad kernel, half of WarpScratch.
+struct BroadScratch : EdgeScratch {
+    BroadPart broad;
+};
+
+struct WarpScratch : EdgeScratch {
     union {
-        struct {
-            float4 swept[kMaxArms][kNumApprox]; // per-arm swept bound of each approx sphere
-            float cur[kNumApprox][3][32];   // per-lane approx spheres of the current arm
-            float low[kNumApprox][3][32];   // per-lane approx spheres of a lower arm
-        } broad;
-        struct {
-            union {
-                float stash[kDetRows][3][32];        // first sphere of each detailed self row
-                struct {                             // arm-vs-arm test of one arm pair
-                    float gc[11][3][32];             // the upper arm's sub-group centres
-                    float xs[kCrossStash][4][32];    // the lower arm's candidate spheres {x, y, z, r} ...
-                    uint32_t xm[kCrossStash][32];    // ... and the upper arm's sub-groups each can reach
-                } cross;
-            };
-        } lanes;
+        BroadPart broad;
+        struct {                                // arm-per-warp kernel: the warp's own arm, both slots
+            float4 swept[2][kNumApprox];
+            float sp[2][kNumApprox][3][32];
+        } arm;
+        float stash[kDetRows][3][32];           // first sphere of each detailed self row
+        struct {                                // arm-vs-arm test of one arm pair
+            float gc[11][3][32];                // the upper arm's sub-group centres
+            float xs[kCrossStash][4][32];       // the lower arm's candidate spheres {x, y, z, r} ...
+            uint32_t xm[kCrossStash][32];       // ... and the upper arm's sub-groups each can reach
+        } cross;
     };
 };
+
+// Flag words of one sample: 8 bits (joints) per arm.
+template <int A>
+using Flags = std::conditional_t<(A > 4), uint64_t, uint32_t>;
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kEnvBit = 1, kSelfBit = 2, kExactBit = 16;
@@ -292,7 +309,7 @@ __device__ __forceinline__ void fk_approx_arm(const float *base12, const float (
 
 // Joint values of arm `a` for sample k of segment `seg` (call-site formulas,
 // see the rule constants).
-__device__ __forceinline__ void sample_q(const WarpScratch &W, int rule, int seg, int a, int k, float (&q)[7]) {
+__device__ __forceinline__ void sample_q(const EdgeScratch &W, int rule, int seg, int a, int k, float (&q)[7]) {
     const float fk = (float)k;
 #pragma unroll
     for (int d = 0; d < 7; d++) {
@@ -305,7 +322,7 @@ __device__ __forceinline__ void sample_q(const WarpScratch &W, int rule, int seg
 }
 
 // One joint value (dof index i) of sample k of segment `seg`.
-__device__ __forceinline__ float sample_q1(const WarpScratch &W, int rule, int seg, int i, int k) {
+__device__ __forceinline__ float sample_q1(const EdgeScratch &W, int rule, int seg, int i, int k) {
     float v = __fmaf_rn((float)k, W.stepg[i], W.base[i]);
     if (rule == kRuleBspline || rule == kRuleShortcut)
         for (int s = 0; s < seg; s++) v = __fadd_rn(v, W.delta[i]);
@@ -347,153 +364,179 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // (EdgeParams::rigid).  FP32 positions then err by far less than a millimetre.
 constexpr float kRegularRad = 64.0f;
 
-// FK of one arm for this lane's sample; the 11 approx centres go to column
-// `lane` of dst.  With swept != nullptr it also writes, for every approx
-// sphere, a bound of that sphere over the warp's 32 samples: the centre of
-// the box around its 32 centres, radius = half the box diagonal (+0.4 %) +
-// sphere radius + cull margin.  If the sphere touches something at any of the
-// samples, its swept bound touches it too (the margin covers FP rounding).
-// Returns whether the joint values are within kRegularRad.
-__device__ __forceinline__ bool fk_approx_lane(const float *base12, const WarpScratch &W, int rule, int seg,
-                                                   int qarm, int k, float (*dst)[3][32], int lane, float4 *swept) {
-    float q[7];
-    sample_q(W, rule, seg, qarm, k, q);
-    ArmSpheres s;
-    fk_approx_arm(base12, q, s);
+// The approx spheres s of one arm for this lane's sample go to column `lane` of
+// dst, and a bound of every sphere over the warp's 32 samples to swept: the
+// centre of the box around its 32 centres, radius = half the box diagonal
+// (+0.4 %) + sphere radius + cull margin.  If the sphere touches something at
+// any of the samples, its swept bound touches it too (the margin covers FP
+// rounding).
+__device__ __forceinline__ void store_swept(const ArmSpheres &s, float (*dst)[3][32], int lane, float4 *swept) {
 #pragma unroll
     for (int i = 0; i < kNumApprox; i++) {
         dst[i][0][lane] = s.x[i];
         dst[i][1][lane] = s.y[i];
         dst[i][2][lane] = s.z[i];
     }
-    if (!swept) return false;
     __syncwarp();
-    {
-        // spheres 1..10: lane t < 30 takes coordinate t % 3 of sphere 1 + t / 3
-        // over the 32 columns, four at a time (start skewed by lane: each
-        // quarter warp reads eight different 16-byte bank groups) and three
-        // values per min / max: 8 loads and 32 min / max in place of 31 loads
-        // and 62 (with the pairs of sphere 5 left out below, the broad kernel
-        // on 65536 4-arm edges: 531 -> 470 us); sphere 0 sits on the base and
-        // does not move
-        float lo = 0.0f, hi = 0.0f;
-        if (lane < 30) {
-            const float4 *col = reinterpret_cast<const float4 *>(&dst[1][0][0] + 32 * lane);
-            const float4 f = col[lane & 7];
-            lo = fminf(min3(f.x, f.y, f.z), f.w);
-            hi = fmaxf(max3(f.x, f.y, f.z), f.w);
+    // spheres 1..10: lane t < 30 takes coordinate t % 3 of sphere 1 + t / 3
+    // over the 32 columns, four at a time (start skewed by lane: each
+    // quarter warp reads eight different 16-byte bank groups) and three
+    // values per min / max: 8 loads and 32 min / max in place of 31 loads
+    // and 62 (with the pairs of sphere 5 left out below, the broad kernel
+    // on 65536 4-arm edges: 531 -> 470 us); sphere 0 sits on the base and
+    // does not move
+    float lo = 0.0f, hi = 0.0f;
+    if (lane < 30) {
+        const float4 *col = reinterpret_cast<const float4 *>(&dst[1][0][0] + 32 * lane);
+        const float4 f = col[lane & 7];
+        lo = fminf(min3(f.x, f.y, f.z), f.w);
+        hi = fmaxf(max3(f.x, f.y, f.z), f.w);
 #pragma unroll
-            for (int l = 1; l < 8; l++) {
-                const float4 v = col[(l + lane) & 7];
-                lo = min3(min3(lo, v.x, v.y), v.z, v.w);
-                hi = max3(max3(hi, v.x, v.y), v.z, v.w);
-            }
-        }
-        const float ly = __shfl_down_sync(kFull, lo, 1), hy = __shfl_down_sync(kFull, hi, 1);
-        const float lz = __shfl_down_sync(kFull, lo, 2), hz = __shfl_down_sync(kFull, hi, 2);
-        const bool own = lane < 30 && lane % 3 == 0;
-        const int i = own ? 1 + lane / 3 : 0;
-        if (own || lane == 30) {
-            const float ax = own ? lo : s.x[0], bx = own ? hi : s.x[0];
-            const float ay = own ? ly : s.y[0], by = own ? hy : s.y[0];
-            const float az = own ? lz : s.z[0], bz = own ? hz : s.z[0];
-            const float dx = bx - ax, dy = by - ay, dz = bz - az;
-            swept[i] = make_float4(0.5f * (ax + bx), 0.5f * (ay + by), 0.5f * (az + bz),
-                                   0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + c_approx[i].w + kCullMargin);
+        for (int l = 1; l < 8; l++) {
+            const float4 v = col[(l + lane) & 7];
+            lo = min3(min3(lo, v.x, v.y), v.z, v.w);
+            hi = max3(max3(hi, v.x, v.y), v.z, v.w);
         }
     }
+    const float ly = __shfl_down_sync(kFull, lo, 1), hy = __shfl_down_sync(kFull, hi, 1);
+    const float lz = __shfl_down_sync(kFull, lo, 2), hz = __shfl_down_sync(kFull, hi, 2);
+    const bool own = lane < 30 && lane % 3 == 0;
+    const int i = own ? 1 + lane / 3 : 0;
+    if (own || lane == 30) {
+        const float ax = own ? lo : s.x[0], bx = own ? hi : s.x[0];
+        const float ay = own ? ly : s.y[0], by = own ? hy : s.y[0];
+        const float az = own ? lz : s.z[0], bz = own ? hz : s.z[0];
+        const float dx = bx - ax, dy = by - ay, dz = bz - az;
+        swept[i] = make_float4(0.5f * (ax + bx), 0.5f * (ay + by), 0.5f * (az + bz),
+                               0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + c_approx[i].w + kCullMargin);
+    }
     __syncwarp();
+}
+
+// Joint values of one arm within kRegularRad.
+__device__ __forceinline__ bool regular_pose(const float (&q)[7]) {
     float sum = 0.0f;  // NaN if any is
 #pragma unroll
     for (int d = 0; d < 7; d++) sum += fabsf(q[d]);
     return sum <= kRegularRad;
 }
 
+// Exact env test of one sphere against obstacle o (index over all classes in
+// the bound order cuboids, z-cuboids, capsules, z-capsules, spheres).
+__device__ __forceinline__ bool env_exact(const float4 *S, const SceneLayout &L, const SceneCounts &C, int o, float x,
+                                          float y, float z, float r) {
+    if (o < C.n_cub) {
+        const float4 *c = S + L.cub + 4 * o;
+        return hit_cuboid(c[0], c[1], c[2], c[3], x, y, z, __fmul_rn(r, r));
+    }
+    o -= C.n_cub;
+    if (o < C.n_zcub) {
+        const float4 *c = S + L.zcub + 4 * o;
+        return hit_zcuboid(c[0], c[1], c[2], x, y, z, __fmul_rn(r, r));
+    }
+    o -= C.n_zcub;
+    if (o < C.n_cap) return hit_capsule(S[L.cap + 2 * o], S[L.cap + 2 * o + 1], x, y, z, r);
+    o -= C.n_cap;
+    if (o < C.n_zcap) return hit_zcapsule(S[L.zcap + 2 * o], S[L.zcap + 2 * o + 1], x, y, z, r);
+    o -= C.n_zcap;
+    const float4 c0 = S[L.sph + o];
+    return hit_sphere_sphere(c0.x, c0.y, c0.z, c0.w, x, y, z, r);
+}
+
 // ---------------------------------------------------------------------------
 // broad phase: approx spheres 1..10 of one arm (lane column `lane` of sp)
-// against the scene.  Returns a bitmask over sphere index (bit i = sphere i
-// of this lane's sample touches some obstacle).  The obstacles of each class
-// are screened one per lane against the 10 spheres' swept bounds (sw, shared
-// by the warp): the obstacle's bounding sphere, then for cuboids with
-// orthonormal axes the exact sphere-cuboid test (both conservative; for
-// spheres the record is its own bound).  Exact per-sample tests then run, for
-// the whole warp, only for the (sphere, obstacle) pairs that survive.
+// against the scene.  Returns this lane's joints with a sphere that touches an
+// obstacle.  The obstacles of all classes, in one order, are screened one per
+// lane against the 10 spheres' swept bounds (sw, shared by the warp): the
+// obstacle's bounding sphere, then for cuboids with orthonormal axes the exact
+// sphere-cuboid test (both conservative).  Exact per-sample tests then run, for
+// the whole warp, only for the (sphere, obstacle) pairs that survive, and only
+// while some lane's joint is not flagged yet.
 // ---------------------------------------------------------------------------
-template <typename BoundFn, typename RefineFn, typename ExactFn>
-__device__ __forceinline__ void env_class(int n, int lane, const float4 *sw, const float (*sp)[3][32], uint32_t &m,
-                                          BoundFn bound, RefineFn refine, ExactFn exact) {
+__device__ __forceinline__ uint32_t env_joints(const float4 *S, const SceneLayout &L, const SceneCounts &C,
+                                               const float (*sp)[3][32], int lane, const float4 *sw) {
+    const int n_obst = C.n_cub + C.n_zcub + C.n_cap + C.n_zcap + C.n_sph;
+    uint32_t jm = 0;
+    uint32_t open = 0x7feu;  // spheres whose joint some lane has not flagged (the same in every lane)
 #pragma unroll 1
-    for (int o0 = 0; o0 < n; o0 += 32) {
+    for (int o0 = 0; o0 < n_obst && open; o0 += 32) {
         // one obstacle per lane: which swept sphere bounds reach it
         const int o = o0 + lane;
         uint32_t cand = 0;
-        if (o < n) {
-            const float4 bs = bound(o);
+        if (o < n_obst) {
+            const float4 bs = S[L.b_cub + o];
 #pragma unroll
             for (int i = 1; i < kNumApprox; i++) {
                 const float4 u = sw[i];
                 if (near3(u.x, u.y, u.z, bs, u.w)) cand |= 1u << i;
             }
-            for (uint32_t c = cand; c; c &= c - 1) {
-                const int i = __ffs(c) - 1;
-                if (!refine(o, bs, sw[i])) cand &= ~(1u << i);
+            cand &= open;
+            if (o < C.n_cub + C.n_zcub && bs.w <= 1e17f) {
+#pragma unroll 1
+                for (uint32_t c = cand; c; c &= c - 1) {
+                    const int i = __ffs(c) - 1;
+                    const float4 u = sw[i];
+                    bool in;
+                    if (o < C.n_cub) {
+                        const float4 *r = S + L.cub + 4 * o;
+                        in = hit_cuboid(r[0], r[1], r[2], r[3], u.x, u.y, u.z, u.w * u.w);
+                    } else {
+                        const float4 *r = S + L.zcub + 4 * (o - C.n_cub);
+                        in = hit_zcuboid(r[0], r[1], r[2], u.x, u.y, u.z, u.w * u.w);
+                    }
+                    if (!in) cand &= ~(1u << i);
+                }
             }
         }
         // exact per-sample tests of the surviving (sphere, obstacle) pairs
         uint32_t obal = __ballot_sync(kFull, cand != 0);
+#pragma unroll 1
         while (obal) {
             const int src = __ffs(obal) - 1;
             obal &= obal - 1;
-            uint32_t cm = __shfl_sync(kFull, cand, src);
-            while (cm) {
-                const int i = __ffs(cm) - 1;
-                cm &= cm - 1;
-                if (exact(o0 + src, sp[i][0][lane], sp[i][1][lane], sp[i][2][lane], c_approx[i].w)) m |= 1u << i;
+            uint32_t cm = __shfl_sync(kFull, cand, src) & open;
+            // the spheres cm against one obstacle, whose record stays in registers
+            auto spheres = [&](auto hit) {
+#pragma unroll 1
+                while (cm) {
+                    const int i = __ffs(cm) - 1;
+                    const uint32_t jb = 1u << approx_joint(i);
+                    if (hit(sp[i][0][lane], sp[i][1][lane], sp[i][2][lane], c_approx[i].w)) jm |= jb;
+                    if (__all_sync(kFull, jm & jb)) open &= ~(i < 7 ? 1u << i : 0x780u);
+                    cm &= cm - 1;
+                    cm &= open;
+                }
+            };
+            int t = o0 + src;
+            if (t < C.n_cub) {
+                const float4 *c = S + L.cub + 4 * t;
+                const float4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+                spheres([&](float x, float y, float z, float r) {
+                    return hit_cuboid(c0, c1, c2, c3, x, y, z, __fmul_rn(r, r));
+                });
+            } else if ((t -= C.n_cub) < C.n_zcub) {
+                const float4 *c = S + L.zcub + 4 * t;
+                const float4 c0 = c[0], c1 = c[1], c2 = c[2];
+                spheres([&](float x, float y, float z, float r) {
+                    return hit_zcuboid(c0, c1, c2, x, y, z, __fmul_rn(r, r));
+                });
+            } else if ((t -= C.n_zcub) < C.n_cap) {
+                const float4 *c = S + L.cap + 2 * t;
+                const float4 c0 = c[0], c1 = c[1];
+                spheres([&](float x, float y, float z, float r) { return hit_capsule(c0, c1, x, y, z, r); });
+            } else if ((t -= C.n_cap) < C.n_zcap) {
+                const float4 *c = S + L.zcap + 2 * t;
+                const float4 c0 = c[0], c1 = c[1];
+                spheres([&](float x, float y, float z, float r) { return hit_zcapsule(c0, c1, x, y, z, r); });
+            } else {
+                const float4 c0 = S[L.sph + t - C.n_zcap];
+                spheres([&](float x, float y, float z, float r) {
+                    return hit_sphere_sphere(c0.x, c0.y, c0.z, c0.w, x, y, z, r);
+                });
             }
         }
     }
-}
-
-__device__ __forceinline__ uint32_t env_mask_approx(const float4 *S, const SceneLayout &L, const SceneCounts &C,
-                                                    const float (*sp)[3][32], int lane, const float4 *sw) {
-    uint32_t m = 0;
-    env_class(
-        C.n_cub, lane, sw, sp, m, [&](int o) { return S[L.b_cub + o]; },
-        [&](int o, float4 bs, float4 u) {
-            const float4 *r = S + L.cub + 4 * o;
-            return bs.w > 1e17f || hit_cuboid(r[0], r[1], r[2], r[3], u.x, u.y, u.z, u.w * u.w);
-        },
-        [&](int o, float x, float y, float z, float rad) {
-            const float4 *r = S + L.cub + 4 * o;
-            return hit_cuboid(r[0], r[1], r[2], r[3], x, y, z, __fmul_rn(rad, rad));
-        });
-    env_class(
-        C.n_zcub, lane, sw, sp, m, [&](int o) { return S[L.b_zcub + o]; },
-        [&](int o, float4 bs, float4 u) {
-            const float4 *r = S + L.zcub + 4 * o;
-            return bs.w > 1e17f || hit_zcuboid(r[0], r[1], r[2], u.x, u.y, u.z, u.w * u.w);
-        },
-        [&](int o, float x, float y, float z, float rad) {
-            const float4 *r = S + L.zcub + 4 * o;
-            return hit_zcuboid(r[0], r[1], r[2], x, y, z, __fmul_rn(rad, rad));
-        });
-    env_class(
-        C.n_cap, lane, sw, sp, m, [&](int o) { return S[L.b_cap + o]; }, [&](int, float4, float4) { return true; },
-        [&](int o, float x, float y, float z, float rad) {
-            return hit_capsule(S[L.cap + 2 * o], S[L.cap + 2 * o + 1], x, y, z, rad);
-        });
-    env_class(
-        C.n_zcap, lane, sw, sp, m, [&](int o) { return S[L.b_zcap + o]; }, [&](int, float4, float4) { return true; },
-        [&](int o, float x, float y, float z, float rad) {
-            return hit_zcapsule(S[L.zcap + 2 * o], S[L.zcap + 2 * o + 1], x, y, z, rad);
-        });
-    env_class(
-        C.n_sph, lane, sw, sp, m, [&](int o) { return S[L.sph + o]; }, [&](int, float4, float4) { return true; },
-        [&](int o, float x, float y, float z, float rad) {
-            const float4 c0 = S[L.sph + o];
-            return hit_sphere_sphere(c0.x, c0.y, c0.z, c0.w, x, y, z, rad);
-        });
-    return m;
+    return jm;
 }
 
 // Arm pairs (a < b) in order: pair index of (a, b), and the count.
@@ -550,8 +593,6 @@ static __constant__ uint8_t c_intra_pairs[21][2] = {
     {0, 5}, {0, 6}, {0, 7}, {0, 8}, {0, 9}, {0, 10}, {1, 5}, {1, 6}, {1, 7}, {1, 8}, {1, 9},
     {1, 10}, {2, 5}, {2, 7}, {2, 8}, {2, 9}, {2, 10}, {5, 7}, {5, 8}, {5, 9}, {5, 10}};
 
-// Broad phase of one sample (every lane of the warp calls it; lanes past the
-// segment's last sample evaluate sample g and discard the result).
 // Intra-arm pairs of one arm (panda_four.cuh:140-176): the 21 approx sphere
 // pairs, one per lane, screened by the swept bounds sw of the warp's samples;
 // exact per-sample tests for the survivors.  Returns the lane's flag bits (by
@@ -580,87 +621,111 @@ __device__ __forceinline__ uint32_t intra_flags(const float (*sp)[3][32], const 
     return jm;
 }
 
+// Broad phase of one sample (every lane of the warp calls it; lanes past the
+// segment's last sample evaluate sample g and discard the result).  One loop
+// places arms: arm b, with its env and intra-arm tests and the screen of its
+// sphere pairs with every lower arm by swept bounds (lane (a, i): sphere i of
+// arm a against arm b's 11), then each lower arm that a pair survived with,
+// whose spheres stay in registers for the exact tests against arm b's columns.
+// Flags of an arm pair go to its lower arm (panda_four.cuh:178-214); lane p of
+// pm receives pair p's connected joints, the lower arm's in bits 0..7 and the
+// upper arm's in bits 8..15.
+// Bound by instruction issue.  With one placement loop and one obstacle order
+// (code shared, a lower arm's spheres in registers: half the scratch) the broad
+// kernels run 24 warps per SM: 65536 4-arm edges 467 -> 414 us, 262144 5-arm
+// edges x 64 samples 5.28 -> 3.82 ms, 65536 shortcut edges 2.47 -> 1.92 ms;
+// 30011 one-arm edges, one class of obstacle, 81 -> 83 us.
 template <int A>
-__device__ __forceinline__ void broad_sample(const EdgeParams &P, WarpScratch &W, const float4 *S,
-                                             const SceneLayout &L, int seg, int k, uint64_t &envw, uint64_t &selfw,
+__device__ __forceinline__ void broad_sample(const EdgeParams &P, const EdgeScratch &W, BroadPart &B, const float4 *S,
+                                             const SceneLayout &L, int seg, int k, Flags<A> &envw, Flags<A> &selfw,
                                              uint32_t &pm) {
     const int lane = threadIdx.x & 31;
     envw = 0;
     selfw = 0;
     pm = 0;
     const bool do_env = P.flags & kEnvBit, do_self = P.flags & kSelfBit;
-    auto &cur = W.broad.cur;
-    auto &low = W.broad.low;
+    auto &cur = B.cur;
 #pragma unroll 1
     for (int b = 0; b < A; b++) {
-        MRPOP_PHASE_START();
-        float4 *sw = W.broad.swept[b];
-        const bool reg = fk_approx_lane(P.base[b], W, P.rule, seg, P.single ? 0 : b, k, cur, lane, sw);
-        MRPOP_PHASE(P, 0);
-        if (do_env) {
-            const uint32_t m = env_mask_approx(S, L, P.sc, cur, lane, sw);
-            uint32_t jm = 0;
-#pragma unroll
-            for (int i = 1; i < kNumApprox; i++)
-                if (m >> i & 1u) jm |= 1u << approx_joint(i);
-            envw |= (uint64_t)jm << (8 * b);
-        }
-        MRPOP_PHASE(P, 1);
-        if (!do_self) continue;
-        // intra-arm pairs: one pair per lane screened by swept bounds, exact
-        // per-sample tests for the survivors
-        const bool regular = __all_sync(kFull, reg) && (P.rigid >> b & 1);
-        const uint32_t jm = intra_flags(cur, sw, lane, regular);
-        selfw |= (uint64_t)jm << (8 * b);
-        MRPOP_PHASE(P, 2);
-        if (A == 1) continue;
-        // arm-vs-arm against every lower arm a < b; flags go to arm a
-        // (panda_four.cuh:178-214).  The 121 sphere pairs are screened by
-        // swept bounds, four rounds of one pair per lane; arm a's spheres are
-        // rebuilt only when some pair survives.
+        float4 *sw = B.swept[b];
+        uint32_t xm[2] = {0u, 0u};  // lane 11 * (a & 1) + i of word a >> 1: arm b's spheres that sphere i of arm a meets
+        uint32_t pend = 0;          // lower arms left to test
 #pragma unroll 1
-        for (int a = 0; a < b; a++) {
-            const float4 *swa = W.broad.swept[a];
-            uint32_t bal[4];
+        for (int x = b;;) {
+            MRPOP_PHASE_START();
+            float q[7];
+            sample_q(W, P.rule, seg, P.single ? 0 : x, k, q);
+            ArmSpheres s;
+            fk_approx_arm(P.base[x], q, s);
+            if (A == 1 || x == b) {
+                store_swept(s, cur, lane, sw);
+                MRPOP_PHASE(P, 0);
+                if (do_env) envw |= (Flags<A>)env_joints(S, L, P.sc, cur, lane, sw) << (8 * b);
+                MRPOP_PHASE(P, 1);
+                if (!do_self) break;
+                const bool reg = regular_pose(q);
+                const bool regular = __all_sync(kFull, reg) && (P.rigid >> b & 1);
+                selfw |= (Flags<A>)intra_flags(cur, sw, lane, regular) << (8 * b);
+                MRPOP_PHASE(P, 2);
+                if (A == 1) break;
+                const int la = lane >= kNumApprox ? 1 : 0, i = min(lane - kNumApprox * la, kNumApprox - 1);
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int t = 32 * r + lane;
-                const int i = t / kNumApprox, j = t - kNumApprox * i;
-                bal[r] = __ballot_sync(kFull, t < kNumApprox * kNumApprox &&
-                                                  near3(swa[i].x, swa[i].y, swa[i].z, sw[j], swa[i].w));
-            }
-            if (!(bal[0] | bal[1] | bal[2] | bal[3])) continue;
-            fk_approx_lane(P.base[a], W, P.rule, seg, a, k, low, lane, nullptr);
-            uint32_t am = 0, ja = 0, jb = 0;
+                for (int w = 0; w < (A > 3 ? 2 : 1); w++) {
+                    if (2 * w >= b) break;
+                    const int a = 2 * w + la;
+                    const float4 u = B.swept[a < b ? a : 0][i];
+                    uint32_t m = 0;
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                uint32_t q = bal[r];
-                while (q) {
-                    const int t = 32 * r + __ffs(q) - 1;
-                    q &= q - 1;
-                    const int i = t / kNumApprox, j = t - kNumApprox * i;
-                    ja |= 1u << approx_joint(i);
-                    jb |= 1u << approx_joint(j);
-                    if (hit_sphere_sphere(low[i][0][lane], low[i][1][lane], low[i][2][lane], c_approx[i].w,
-                                          cur[j][0][lane], cur[j][1][lane], cur[j][2][lane], c_approx[j].w))
-                        am |= 1u << approx_joint(i);
+                    for (int j = 0; j < kNumApprox; j++)
+                        if (near3(u.x, u.y, u.z, sw[j], u.w)) m |= 1u << j;
+                    xm[w] = a < b && lane < 2 * kNumApprox ? m : 0u;
+                    const uint32_t nz = __ballot_sync(kFull, xm[w] != 0);
+                    pend |= ((nz & 0x7ffu ? 1u : 0u) | (nz >> kNumApprox ? 2u : 0u)) << (2 * w);
                 }
+            } else {
+                const int a = x;
+                const uint32_t word = A > 3 && a > 1 ? xm[1] : xm[0];
+                uint32_t am = 0, ja = 0, sb = 0;
+#pragma unroll
+                for (int i = 0; i < kNumApprox; i++) {
+                    uint32_t m = __shfl_sync(kFull, word, kNumApprox * (a & 1) + i);
+                    if (!m) continue;
+                    ja |= 1u << approx_joint(i);
+                    sb |= m;
+                    bool h = false;
+#pragma unroll 1
+                    for (; m; m &= m - 1) {
+                        const int j = __ffs(m) - 1;
+                        h |= hit_sphere_sphere(s.x[i], s.y[i], s.z[i], c_approx[i].w, cur[j][0][lane], cur[j][1][lane],
+                                               cur[j][2][lane], c_approx[j].w);
+                    }
+                    if (h) am |= 1u << approx_joint(i);
+                }
+                selfw |= (Flags<A>)am << (8 * a);
+                const uint32_t jb = (sb & 0x7fu) | (sb >> 7 ? 0x80u : 0u);
+                if (lane == pair_index(a, b, A)) pm = ja | jb << 8;
+                MRPOP_PHASE(P, 3);
             }
-            selfw |= (uint64_t)am << (8 * a);
-            if (lane == pair_index(a, b, A)) pm = ja | jb << 8;
+            if (!pend) break;
+            x = __ffs(pend) - 1;
+            pend &= pend - 1;
         }
-        MRPOP_PHASE(P, 3);
+        __syncwarp();  // arm b's columns are read before the next arm's overwrite them
     }
 }
 
-__device__ __forceinline__ int flag_count(uint64_t w) {
-    int n = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const uint64_t col = (w >> j) & 0x0101010101ull; // joint j of arms 0..4
-        n += det_count(j) * __popcll(col);
-    }
-    return n;
+// Detailed spheres on the joints flagged in w (8 bits per arm).  Joints with equal counts share a population count.
+template <int A>
+__device__ __forceinline__ int flag_count(Flags<A> w) {
+    static_assert(det_count(0) == 1 && det_count(1) == 4 && det_count(2) == 4 && det_count(3) == 4 &&
+                      det_count(4) == 4 && det_count(5) == 12 && det_count(6) == 3 && det_count(7) == 27,
+                  "counts per joint");
+    auto bits = [&](uint32_t joints) {
+        int n = __popc((uint32_t)w & 0x01010101u * joints);
+        if constexpr (A > 4) n += __popc((uint32_t)(w >> 32) & joints);
+        return n;
+    };
+    return bits(0x01u) + 4 * bits(0x1eu) + 12 * bits(0x20u) + 3 * bits(0x40u) + 27 * bits(0x80u);
 }
 
 // reference thread split (utils.cuh:478-497): share of 4g threads, truncated
@@ -696,22 +761,6 @@ static __device__ __noinline__ double narrow_flops(const EdgeParams &P, int A, u
 // ---------------------------------------------------------------------------
 // narrow phase
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t joint_sphere_mask(uint32_t jm) {
-    uint64_t m = 0;
-#pragma unroll
-    for (int j = 0; j < kNumJoints; j++)
-        if (jm >> j & 1u) m |= ((1ull << det_count(j)) - 1ull) << det_first(j);
-    return m;
-}
-
-// position of the n-th (0-based) set bit of m
-__device__ __forceinline__ int nth_bit(uint64_t m, int n) {
-    const uint32_t lo = (uint32_t)m;
-    const int pl = __popc(lo);
-    if (n < pl) return (int)__fns(lo, 0, n + 1);
-    return 32 + (int)__fns((uint32_t)(m >> 32), 0, n - pl + 1);
-}
-
 // bit r set: detailed self row r is checked for an arm with self flags sm
 // Rows whose first-read sphere is on joint j (quirk: sphere r, else first(r)).
 __host__ __device__ constexpr uint32_t joint_rows(int j, bool quirk) {
@@ -800,28 +849,6 @@ constexpr int kHandFirst = 37;
 constexpr int kHandParts = 3;
 __host__ __device__ __forceinline__ constexpr uint32_t hand_part(int s) {
     return s == 0 ? 0x3030C3u : s == 1 ? 0x00C30Cu : 0x0F0C30u;
-}
-
-// Exact env test of one sphere against obstacle o (index over all classes in
-// the bound order cuboids, z-cuboids, capsules, z-capsules, spheres).
-__device__ __forceinline__ bool env_exact(const float4 *S, const SceneLayout &L, const SceneCounts &C, int o, float x,
-                                          float y, float z, float r) {
-    if (o < C.n_cub) {
-        const float4 *c = S + L.cub + 4 * o;
-        return hit_cuboid(c[0], c[1], c[2], c[3], x, y, z, __fmul_rn(r, r));
-    }
-    o -= C.n_cub;
-    if (o < C.n_zcub) {
-        const float4 *c = S + L.zcub + 4 * o;
-        return hit_zcuboid(c[0], c[1], c[2], x, y, z, __fmul_rn(r, r));
-    }
-    o -= C.n_zcub;
-    if (o < C.n_cap) return hit_capsule(S[L.cap + 2 * o], S[L.cap + 2 * o + 1], x, y, z, r);
-    o -= C.n_cap;
-    if (o < C.n_zcap) return hit_zcapsule(S[L.zcap + 2 * o], S[L.zcap + 2 * o + 1], x, y, z, r);
-    o -= C.n_zcap;
-    const float4 c0 = S[L.sph + o];
-    return hit_sphere_sphere(c0.x, c0.y, c0.z, c0.w, x, y, z, r);
 }
 
 // Conservative screen of obstacle o (index over all classes, in the order of
@@ -939,9 +966,9 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
         const int r = __ffs(m1) - 1;
         m1 &= m1 - 1;
         const float3 p = place_reg(T, det_tab[c.quirk ? r : det_row_first(r)]);
-        W.lanes.stash[r][0][lane] = p.x;
-        W.lanes.stash[r][1][lane] = p.y;
-        W.lanes.stash[r][2][lane] = p.z;
+        W.stash[r][0][lane] = p.x;
+        W.stash[r][1][lane] = p.y;
+        W.stash[r][2][lane] = p.z;
     }
 #pragma unroll 1
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
@@ -953,7 +980,7 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
         while (rows) {
             const int r = __ffs(rows) - 1;
             rows &= rows - 1;
-            if (near3(W.lanes.stash[r][0][lane], W.lanes.stash[r][1][lane], W.lanes.stash[r][2][lane],
+            if (near3(W.stash[r][0][lane], W.stash[r][1][lane], W.stash[r][2][lane],
                       make_float4(gc.x, gc.y, gc.z, gl.w), det_tab[det_row_first(r)].w))
                 nr |= 1u << r;
         }
@@ -970,7 +997,7 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
                 uint32_t ns = 0;
                 for (uint32_t m = nr; m; m &= m - 1) {
                     const int r = __ffs(m) - 1;
-                    if (near3(W.lanes.stash[r][0][lane], W.lanes.stash[r][1][lane], W.lanes.stash[r][2][lane],
+                    if (near3(W.stash[r][0][lane], W.stash[r][1][lane], W.stash[r][2][lane],
                               make_float4(sc.x, sc.y, sc.z, sl.w), det_tab[det_row_first(r)].w))
                         ns |= 1u << r;
                 }
@@ -980,8 +1007,8 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
                     const float3 p = place_reg(T, sd);
                     for (uint32_t m = ns; m; m &= m - 1) {
                         const int r = __ffs(m) - 1;
-                        h |= hit_sphere_sphere(W.lanes.stash[r][0][lane], W.lanes.stash[r][1][lane],
-                                               W.lanes.stash[r][2][lane], det_tab[det_row_first(r)].w, p.x, p.y,
+                        h |= hit_sphere_sphere(W.stash[r][0][lane], W.stash[r][1][lane],
+                                               W.stash[r][2][lane], det_tab[det_row_first(r)].w, p.x, p.y,
                                                p.z, sd.w);
                     }
                 }
@@ -994,8 +1021,8 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
                 while (m) {
                     const int r = __ffs(m) - 1;
                     m &= m - 1;
-                    h |= hit_sphere_sphere(W.lanes.stash[r][0][lane], W.lanes.stash[r][1][lane],
-                                           W.lanes.stash[r][2][lane], det_tab[det_row_first(r)].w, p.x, p.y, p.z,
+                    h |= hit_sphere_sphere(W.stash[r][0][lane], W.stash[r][1][lane],
+                                           W.stash[r][2][lane], det_tab[det_row_first(r)].w, p.x, p.y, p.z,
                                            sd.w);
                 }
             }
@@ -1099,7 +1126,7 @@ struct RowTargets {
 // Every lane of the warp calls it.  sw: the lane's self flag words (0 for a
 // lane without a self candidate); arms_in: arms to screen.
 template <int A>
-__device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const WarpScratch &W, int seg, int k0, uint64_t sw,
+__device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const EdgeScratch &W, int seg, int k0, Flags<A> sw,
                                                  int quirk, uint32_t arms_in) {
     const int lane = threadIdx.x & 31;
     RowScreen out;
@@ -1107,7 +1134,8 @@ __device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const Warp
     out.arms = 0;
     out.sub = 32;
     const uint32_t lo = __reduce_or_sync(kFull, (uint32_t)sw & 0x1f1f1f1fu);
-    const uint32_t hi = A > 4 ? __reduce_or_sync(kFull, (uint32_t)(sw >> 32) & 0x1fu) : 0u;
+    uint32_t hi = 0;
+    if constexpr (A > 4) hi = __reduce_or_sync(kFull, (uint32_t)(sw >> 32) & 0x1fu);
     uint32_t joints = 0;
 #pragma unroll
     for (int a = 0; a < A; a++) {
@@ -1207,11 +1235,11 @@ __device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const Warp
 
 // Lower arm, joint j (flagged for this lane): its spheres from index `from` on
 // that can reach one of the upper arm's sub-groups gb (bounds, centres in
-// W.lanes.cross.gc) go to the lane's stash with the sub-groups they reach;
+// W.cross.gc) go to the lane's stash with the sub-groups they reach;
 // `next` receives the first sphere left out when the stash is full.
 __device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf &T, uint32_t gb, int from, int &n,
                                             int &next, WarpScratch &W, int lane) {
-    auto &X = W.lanes.cross;
+    auto &X = W.cross;
 #pragma unroll 1
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
         if (grp_first(g + 1) <= from) continue;
@@ -1254,7 +1282,7 @@ __device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf
 // Upper arm, joint j: its spheres against the stashed spheres that reach their
 // sub-group.
 __device__ __forceinline__ void probe_joint(int j, const Xf &T, int n, bool &hit, WarpScratch &W, int lane) {
-    auto &X = W.lanes.cross;
+    auto &X = W.cross;
 #pragma unroll 1
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
         uint32_t em = 0;
@@ -1338,7 +1366,7 @@ constexpr int kStageAll = 0, kStageEnvPairs = 1, kStageRows = 2;
 template <int A, bool ONE = false, int STAGE = kStageAll>
 __device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch &W, const float4 *S,
                                                 const SceneLayout &L, const float4 *det_tab, int seg, int k0,
-                                                uint64_t ew, uint64_t sw, bool dE, bool dS, uint32_t pms,
+                                                Flags<A> ew, Flags<A> sw, bool dE, bool dS, uint32_t pms,
                                                 int one_arm = 0, ArmShare *X = nullptr, int slot = 0) {
     const int lane = threadIdx.x & 31;
     const int k = min(k0 + lane + 1, P.g);
@@ -1446,9 +1474,9 @@ __device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch
 #pragma unroll 1
                         for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
                             const float3 ctr = place_reg(T, P.grp[g]);
-                            W.lanes.cross.gc[g][0][lane] = ctr.x;
-                            W.lanes.cross.gc[g][1][lane] = ctr.y;
-                            W.lanes.cross.gc[g][2][lane] = ctr.z;
+                            W.cross.gc[g][0][lane] = ctr.x;
+                            W.cross.gc[g][1][lane] = ctr.y;
+                            W.cross.gc[g][2][lane] = ctr.z;
                         }
                     } else if (act && !c.hit && n > 0) {
                         probe_joint(j, T, n, c.hit, W, lane);
@@ -1483,7 +1511,7 @@ __device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch
 // Edge set-up: segment start and per-sample / per-segment steps of every dof
 // into warp scratch (call-site formulas, see the rule constants).  Returns
 // the segment count; too_many marks counts beyond kMaxSegments.
-__device__ __forceinline__ int edge_setup(const EdgeParams &P, WarpScratch &W, long long e, int dof, int g, int lane,
+__device__ __forceinline__ int edge_setup(const EdgeParams &P, EdgeScratch &W, long long e, int dof, int g, int lane,
                                           bool &too_many) {
     const float *qa = P.q0 + e * dof, *qb = P.q1 + e * dof;
     float diff0 = 0.f, diff1 = 0.f;
@@ -1524,7 +1552,7 @@ __device__ __forceinline__ int edge_setup(const EdgeParams &P, WarpScratch &W, l
 
 // CONNECT: the segment start of segment `seg` (the caller's loop adds the
 // per-segment step once per finished segment, pop_planner.cu:697).
-__device__ __forceinline__ void connect_advance(WarpScratch &W, int dof, int seg, int lane) {
+__device__ __forceinline__ void connect_advance(EdgeScratch &W, int dof, int seg, int lane) {
     for (int d = lane; d < dof; d += 32) {
         float b = W.base[d];
         for (int s = 0; s < seg; s++) b = __fadd_rn(b, W.delta[d]);
@@ -1583,10 +1611,10 @@ __device__ __forceinline__ void thread_split(bool exact, int g, int lane, const 
 }
 
 template <int A, int SPL>
-__device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W, const float4 *S,
-                                             const SceneLayout &L, int seg, int g, int lane, uint64_t (&envw)[SPL],
-                                             uint64_t (&selfw)[SPL], uint32_t (&pm)[SPL], uint64_t &cand_env,
-                                             uint64_t &cand_self, double &tally) {
+__device__ __forceinline__ bool broad_decide(const EdgeParams &P, const EdgeScratch &W, BroadPart &B, const float4 *S,
+                                             const SceneLayout &L, int seg, int g, int lane, Flags<A> (&envw)[SPL],
+                                             Flags<A> (&selfw)[SPL], uint32_t (&pm)[SPL], uint64_t &cand_env,
+                                             uint64_t &cand_self, long long e, bool first) {
     MRPOP_PHASE_START();
     int envc[SPL], selfc[SPL];
     int tot_env = 0, tot_self = 0;
@@ -1595,11 +1623,11 @@ __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W
 #pragma unroll 1
     for (int s = 0; s < SPL; s++) {
         const int k = lane + 1 + 32 * s;
-        uint64_t ew, sw;
+        Flags<A> ew, sw;
         uint32_t pw;
-        broad_sample<A>(P, W, S, L, seg, k <= g ? k : g, ew, sw, pw);
+        broad_sample<A>(P, W, B, S, L, seg, k <= g ? k : g, ew, sw, pw);
         if (k > g) ew = sw = 0;
-        const int ec = flag_count(ew), sc = flag_count(sw);
+        const int ec = flag_count<A>(ew), sc = flag_count<A>(sw);
         if (s == 0) {
             envw[0] = ew;
             selfw[0] = sw;
@@ -1622,7 +1650,7 @@ __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W
         tot_env += __shfl_xor_sync(kFull, tot_env, o);
         tot_self += __shfl_xor_sync(kFull, tot_self, o);
     }
-    if (P.flops) tally += P.fbp * g;
+    if (P.flops && lane == 0) P.flops[e] = (first ? 0.0 : P.flops[e]) + P.fbp * g;
     cand_env = cand_self = 0;
     if (tot_env == 0 && tot_self == 0) return false;
     MRPOP_PHASE(P, 7);
@@ -1637,7 +1665,7 @@ __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(kFull, f, o);
-        tally += f;
+        if (lane == 0) P.flops[e] += f;
     }
     MRPOP_PHASE(P, 4);
     return true;
@@ -1649,7 +1677,7 @@ __device__ __forceinline__ bool broad_decide(const EdgeParams &P, WarpScratch &W
 template <int A, int SPL, int STAGE = kStageAll>
 __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &W, const float4 *S,
                                               const SceneLayout &L, const float4 *det_tab, int seg, int lane,
-                                              const uint64_t (&envw)[SPL], const uint64_t (&selfw)[SPL],
+                                              const Flags<A> (&envw)[SPL], const Flags<A> (&selfw)[SPL],
                                               const uint32_t (&pm)[SPL], uint64_t cand_env, uint64_t cand_self,
                                               int k0 = 0) {
     MRPOP_PHASE_START();
@@ -1659,7 +1687,7 @@ __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &
     for (int s = 0; s < SPL; s++) {
         const int bit = lane + 32 * s;
         const bool dE = cand_env >> bit & 1ull, dS = cand_self >> bit & 1ull;
-        const uint64_t ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
+        const Flags<A> ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
         const uint32_t hb = narrow_slot<A, false, STAGE>(P, W, S, L, det_tab, seg, k0 + 32 * s, ew, sw, dE, dS,
                                                          s == 0 ? pm[0] : pm[SPL - 1]);
         hits |= (uint64_t)hb << (32 * s);
@@ -1669,15 +1697,15 @@ __device__ __forceinline__ int narrow_segment(const EdgeParams &P, WarpScratch &
 }
 
 // Common kernel prologue: scene staged in shared memory, warp scratch.
-#define MRPOP_KERNEL_PROLOGUE()                                                                        \
+#define MRPOP_KERNEL_PROLOGUE(Scratch)                                                                 \
     extern __shared__ __align__(128) unsigned char smem_raw[];                                         \
     __shared__ __align__(8) uint64_t bar;                                                              \
     __shared__ float4 det_tab[kNumDet];                                                                \
     const SceneLayout L = scene_layout(P.sc);                                                          \
     float4 *S = reinterpret_cast<float4 *>(smem_raw);                                                  \
-    WarpScratch *Wall = reinterpret_cast<WarpScratch *>(smem_raw + (size_t)L.total * sizeof(float4));  \
+    Scratch *Wall = reinterpret_cast<Scratch *>(smem_raw + (size_t)L.total * sizeof(float4));          \
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;                                        \
-    WarpScratch &W = Wall[warp];                                                                       \
+    Scratch &W = Wall[warp];                                                                           \
     for (int i = threadIdx.x; i < kNumDet; i += blockDim.x) det_tab[i] = c_det[i];                     \
     const bool staged = stage_scene(S, P.scene, (uint32_t)(L.total * sizeof(float4)), &bar, P.status); \
     MRPOP_PHASE_BIND(P);                                                                               \
@@ -1707,13 +1735,15 @@ __device__ __forceinline__ void fused_edge(const EdgeParams &P, WarpScratch &W, 
     bool too_many;
     const int nseg = edge_setup(P, W, e, dof, g, lane, too_many);
     int first = 0;
-    double tally = 0.0;
+    if (P.flops && P.seg0 == 0 && lane == 0) P.flops[e] = 0.0;
     const int nseg_run = too_many ? 0 : nseg;
     if (P.rule == kRuleConnect && P.seg0 > 0) connect_advance(W, dof, P.seg0, lane);
     for (int seg = P.seg0; seg < nseg_run && first == 0; seg++) {
-        uint64_t envw[SPL], selfw[SPL], cand_env, cand_self;
+        Flags<A> envw[SPL], selfw[SPL];
+        uint64_t cand_env, cand_self;
         uint32_t pm[SPL];
-        if (broad_decide<A, SPL>(P, W, S, L, seg, g, lane, envw, selfw, pm, cand_env, cand_self, tally)) {
+        if (broad_decide<A, SPL>(P, W, W.broad, S, L, seg, g, lane, envw, selfw, pm, cand_env, cand_self, e,
+                                 false)) {
             const int fb =
                 narrow_segment<A, SPL>(P, W, S, L, det_tab, seg, lane, envw, selfw, pm, cand_env, cand_self);
             if (fb < 64) first = seg * g + fb + 1;
@@ -1728,7 +1758,6 @@ __device__ __forceinline__ void fused_edge(const EdgeParams &P, WarpScratch &W, 
         P.valid[e] = (first == 0 && !too_many) ? 1 : 0;
         P.first_hit[e] = too_many ? -2 : (first ? first : -1);
         if (P.n_seg_out) P.n_seg_out[e] = nseg;
-        if (P.flops) P.flops[e] = P.seg0 > 0 ? P.flops[e] + tally : tally;
     }
     __syncwarp();
 }
@@ -1736,7 +1765,7 @@ __device__ __forceinline__ void fused_edge(const EdgeParams &P, WarpScratch &W, 
 template <int A, int SPL>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     validate_kernel(const __grid_constant__ EdgeParams P) {
-    MRPOP_KERNEL_PROLOGUE()
+    MRPOP_KERNEL_PROLOGUE(WarpScratch)
     for (long long e = (long long)blockIdx.x * kWarpsPerBlock + warp; e < P.n_edges; e += nwarps)
         fused_edge<A, SPL>(P, W, S, L, det_tab, e, dof, g, lane, staged);
 }
@@ -1774,11 +1803,11 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
     const int k = lane + 1 + 32 * half;
     int first = 0;
     for (int seg = 0; seg < nseg_run && first == 0; seg++) {
-        uint64_t ew, sw;
+        Flags<A> ew, sw;
         uint32_t pw;
-        broad_sample<A>(P, W, S, L, seg, k <= g ? k : g, ew, sw, pw);
+        broad_sample<A>(P, W, W.broad, S, L, seg, k <= g ? k : g, ew, sw, pw);
         if (k > g) ew = sw = 0;
-        const int ec = flag_count(ew), sc = flag_count(sw);
+        const int ec = flag_count<A>(ew), sc = flag_count<A>(sw);
         int te = ec, ts = sc;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -1818,7 +1847,7 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
             }
             const uint64_t cand_env = __ballot_sync(kFull, cE), cand_self = __ballot_sync(kFull, cS);
             __syncwarp();
-            const uint64_t envw[1] = {ew}, selfw[1] = {sw};
+            const Flags<A> envw[1] = {ew}, selfw[1] = {sw};
             const uint32_t pm[1] = {pw};
             const int fb = (cand_env | cand_self)
                                ? narrow_segment<A, 1>(P, W, S, L, det_tab, seg, lane, envw, selfw, pm, cand_env,
@@ -1848,7 +1877,7 @@ __device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch
 template <int A>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     pair_kernel(const __grid_constant__ EdgeParams P) {
-    MRPOP_KERNEL_PROLOGUE()
+    MRPOP_KERNEL_PROLOGUE(WarpScratch)
     static_assert(kWarpsPerBlock % 2 == 0, "warps come in pairs");
     __shared__ PairShare X[kWarpsPerBlock / 2];
     const int pair = warp >> 1, half = warp & 1;
@@ -1895,22 +1924,21 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
         }
         __syncthreads();
         // this arm: placement, swept bounds, env and intra-arm screens (the
-        // slots' spheres stay in broad.cur / broad.low for the pair tests)
+        // slots' spheres stay in arm.sp for the pair tests)
 #pragma unroll 1
         for (int s = 0; s < SPL; s++) {
             const int k = lane + 1 + 32 * s;
-            float(*sp)[3][32] = s == 0 ? W.broad.cur : W.broad.low;
-            float4 *sw = W.broad.swept[s];
-            const bool reg =
-                fk_approx_lane(P.base[arm], W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, sp, lane, sw);
+            auto &sp = W.arm.sp[s];
+            float4 *sw = W.arm.swept[s];
+            float q[7];
+            sample_q(W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, q);
+            ArmSpheres as;
+            fk_approx_arm(P.base[arm], q, as);
+            store_swept(as, sp, lane, sw);
+            const bool reg = regular_pose(q);
             const bool regular = __all_sync(kFull, reg) && (P.rigid >> arm & 1);
             uint32_t em = 0, im = 0;
-            if (do_env) {
-                const uint32_t m = env_mask_approx(S, L, P.sc, sp, lane, sw);
-#pragma unroll
-                for (int i = 1; i < kNumApprox; i++)
-                    if (m >> i & 1u) em |= 1u << approx_joint(i);
-            }
+            if (do_env) em = env_joints(S, L, P.sc, sp, lane, sw);
             if (do_self) im = intra_flags(sp, sw, lane, regular);
             if (k <= g) {
                 if (em) atomicOr(&X.env[s][lane], (unsigned long long)em << (8 * arm));
@@ -1930,7 +1958,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
 #pragma unroll 1
                 for (int s = 0; s < SPL; s++) {
                     const int k = lane + 1 + 32 * s;
-                    const float4 *swa = Wa[a].broad.swept[s], *swb = Wa[b].broad.swept[s];
+                    const float4 *swa = Wa[a].arm.swept[s], *swb = Wa[b].arm.swept[s];
                     uint32_t bal[4];
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
@@ -1943,8 +1971,8 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                         if (lane == 0) X.pm[s][p] = 0;
                         continue;
                     }
-                    const float(*low)[3][32] = s == 0 ? Wa[a].broad.cur : Wa[a].broad.low;
-                    const float(*cur)[3][32] = s == 0 ? Wa[b].broad.cur : Wa[b].broad.low;
+                    const auto &low = Wa[a].arm.sp[s];
+                    const auto &cur = Wa[b].arm.sp[s];
                     uint32_t am = 0, ja = 0, jb = 0;
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
@@ -1968,14 +1996,14 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
         }
         __syncthreads();
         // the thread split, from the ORed words (every warp alike)
-        uint64_t envw[SPL], selfw[SPL];
+        Flags<A> envw[SPL], selfw[SPL];
         int envc[SPL], selfc[SPL], tot_env = 0, tot_self = 0;
 #pragma unroll
         for (int s = 0; s < SPL; s++) {
-            envw[s] = X.env[s][lane];
-            selfw[s] = X.self[s][lane];
-            envc[s] = flag_count(envw[s]);
-            selfc[s] = flag_count(selfw[s]);
+            envw[s] = (Flags<A>)X.env[s][lane];
+            selfw[s] = (Flags<A>)X.self[s][lane];
+            envc[s] = flag_count<A>(envw[s]);
+            selfc[s] = flag_count<A>(selfw[s]);
             tot_env += envc[s];
             tot_self += selfc[s];
         }
@@ -1996,7 +2024,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                 if (s > 0 && __shfl_sync(kFull, *(const volatile unsigned int *)&X.hits[0], 0)) break;
                 const int bit = lane + 32 * s;
                 const bool dE = cand_env >> bit & 1ull, dS = cand_self >> bit & 1ull;
-                const uint64_t ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
+                const Flags<A> ew = s == 0 ? envw[0] : envw[SPL - 1], sw = s == 0 ? selfw[0] : selfw[SPL - 1];
                 narrow_slot<A, true>(P, W, S, L, det_tab, seg, 32 * s, ew, sw, dE, dS, 0u, arm, &X, s);
             }
             __syncthreads();
@@ -2051,12 +2079,12 @@ __global__ void __launch_bounds__(32 * A, armwise_min_blocks(A)) armwise_kernel(
 // Staged flag words of sample slot o (= edge * 32 * SPL + sample - 1): 8 flag
 // bits per arm, so 32-bit words hold up to 4 arms.
 template <int A>
-__device__ __forceinline__ void store_flags(const EdgeParams &P, long long o, uint64_t env, uint64_t self) {
+__device__ __forceinline__ void store_flags(const EdgeParams &P, long long o, Flags<A> env, Flags<A> self) {
     if (A <= 4) reinterpret_cast<uint2 *>(P.sflags)[o] = make_uint2((uint32_t)env, (uint32_t)self);
     else reinterpret_cast<ulonglong2 *>(P.sflags)[o] = make_ulonglong2(env, self);
 }
 template <int A>
-__device__ __forceinline__ void load_flags(const EdgeParams &P, long long o, uint64_t &env, uint64_t &self) {
+__device__ __forceinline__ void load_flags(const EdgeParams &P, long long o, Flags<A> &env, Flags<A> &self) {
     if (A <= 4) {
         const uint2 v = reinterpret_cast<const uint2 *>(P.sflags)[o];
         env = v.x;
@@ -2069,7 +2097,7 @@ __device__ __forceinline__ void load_flags(const EdgeParams &P, long long o, uin
 }
 
 template <int A, int SPL, bool SEG>
-__device__ __forceinline__ void broad_edge(const EdgeParams &P, WarpScratch &W, const float4 *S, const SceneLayout &L,
+__device__ __forceinline__ void broad_edge(const EdgeParams &P, BroadScratch &W, const float4 *S, const SceneLayout &L,
                                            long long e, int dof, int g, int lane, bool staged) {
     if (!staged) {
         if (lane == 0) {
@@ -2113,10 +2141,11 @@ __device__ __forceinline__ void broad_edge(const EdgeParams &P, WarpScratch &W, 
     } else {
         (void)nseg;
     }
-    uint64_t envw[SPL], selfw[SPL], cand_env, cand_self;
+    Flags<A> envw[SPL], selfw[SPL];
+    uint64_t cand_env, cand_self;
     uint32_t pm[SPL];
-    double tally = 0.0;
-    const bool any = broad_decide<A, SPL>(P, W, S, L, r, g, lane, envw, selfw, pm, cand_env, cand_self, tally);
+    const bool any = broad_decide<A, SPL>(P, W, W.broad, S, L, r, g, lane, envw, selfw, pm, cand_env, cand_self, e,
+                                          !segmented || r == 0);
     if (any) {
 #pragma unroll
         for (int s = 0; s < SPL; s++) {
@@ -2133,7 +2162,6 @@ __device__ __forceinline__ void broad_edge(const EdgeParams &P, WarpScratch &W, 
             if (segmented) P.sdone[e] = 1;
         }
         if (!segmented && P.n_seg_out) P.n_seg_out[e] = 1;
-        if (P.flops) P.flops[e] = (segmented && r > 0) ? P.flops[e] + tally : tally;
     }
     __syncwarp();
 }
@@ -2159,7 +2187,7 @@ __device__ __forceinline__ void narrow_edge(const EdgeParams &P, WarpScratch &W,
         }
         return;
     }
-    uint64_t envw[SPL], selfw[SPL];
+    Flags<A> envw[SPL], selfw[SPL];
     uint32_t pm[SPL];
     uint32_t any_pair = 0;
 #pragma unroll
@@ -2206,9 +2234,9 @@ __device__ __forceinline__ long long next_edge(unsigned long long *counter, int 
 }
 
 template <int A, int SPL, bool SEG>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, kBroadMinBlocks)
     broad_kernel(const __grid_constant__ EdgeParams P) {
-    MRPOP_KERNEL_PROLOGUE()
+    MRPOP_KERNEL_PROLOGUE(BroadScratch)
     (void)nwarps;
     for (long long e = next_edge(P.work, lane); e < P.n_edges; e = next_edge(P.work, lane))
         broad_edge<A, SPL, SEG>(P, W, S, L, e, dof, g, lane, staged);
@@ -2220,7 +2248,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 template <int A, int SPL, bool SEG>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     narrow_kernel(const __grid_constant__ EdgeParams P) {
-    MRPOP_KERNEL_PROLOGUE()
+    MRPOP_KERNEL_PROLOGUE(WarpScratch)
     (void)nwarps;
     // the scene is staged; wait for the broad kernel (complete, its writes
     // visible) before reading its output
@@ -2296,7 +2324,7 @@ __device__ __forceinline__ bool stage_bulk(float4 *dst, const float4 *src, uint3
 }
 
 template <int A, int SPL, int MODE, bool SEG>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, MODE == kBatchBroad ? kBroadMinBlocks : MRPOP_MIN_BLOCKS)
     batch_kernel(const __grid_constant__ BatchParams B) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
@@ -2344,7 +2372,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
         const EdgeParams &P = Ps;
         const SceneLayout L = scene_layout(P.sc);
         const float4 *S = reinterpret_cast<const float4 *>(smem_raw);
-        WarpScratch &W = reinterpret_cast<WarpScratch *>(smem_raw + (size_t)L.total * sizeof(float4))[warp];
+        using Scratch = std::conditional_t<MODE == kBatchBroad, BroadScratch, WarpScratch>;
+        Scratch &W = reinterpret_cast<Scratch *>(smem_raw + (size_t)L.total * sizeof(float4))[warp];
         const int dof = 7 * (P.single ? 1 : A);
         // ... and its warps take the chunk's edges one at a time
         for (;;) {
@@ -2353,10 +2382,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
             k = __shfl_sync(kFull, k, 0);
             if ((int)k >= ch.z) break;
             const long long e = (long long)ch.y + k;
-            if (MODE == kBatchBroad) broad_edge<A, SPL, SEG>(P, W, S, L, e, dof, P.g, lane, staged);
-            else if (MODE == kBatchNarrow)
+            if constexpr (MODE == kBatchBroad) broad_edge<A, SPL, SEG>(P, W, S, L, e, dof, P.g, lane, staged);
+            else if constexpr (MODE == kBatchNarrow)
                 narrow_edge<A, SPL, SEG, A == 1 ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
-            else if (MODE == kBatchRows)
+            else if constexpr (MODE == kBatchRows)
                 narrow_edge<A, SPL, SEG, kStageRows>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
             else fused_edge<A, SPL>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
         }

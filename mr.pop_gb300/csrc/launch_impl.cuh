@@ -121,7 +121,8 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
         }
         kind = p.g > 32 ? kFusedPair : kFused;
     }
-    // the rows kernel reads no scene
+    // the broad kernel's warps need less scratch; the rows kernel reads no scene
+    if (kind == kBroad) smem_bytes -= (size_t)kWarpsPerBlock * (sizeof(WarpScratch) - sizeof(BroadScratch));
     if (kind == kRows) smem_bytes = (size_t)kWarpsPerBlock * sizeof(WarpScratch);
     const int spl = p.g > 32 ? 2 : 1;
     const bool seg = p.rule != 0;
@@ -161,14 +162,16 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
 // than kWarpsPerBlock (the kernel indexes its per-warp scratch by warp).
 // The arm-per-warp batch kernel runs A warps per CTA whatever `warps` says:
 // its CTA size and shared memory (callers give the size for `warps` warps).
-inline void armwise_shape(int A, size_t &smem_bytes, int &warps) {
-    smem_bytes = smem_bytes - (size_t)warps * sizeof(WarpScratch) + (size_t)A * sizeof(WarpScratch);
-    warps = A;
+// The broad kernels' warps need less scratch.
+inline void batch_shape(int A, int mode, size_t &smem_bytes, int &warps) {
+    smem_bytes -= (size_t)warps * sizeof(WarpScratch);
+    if (mode == kBatchArmwise) warps = A;
+    smem_bytes += (size_t)warps * (mode == kBatchBroad ? sizeof(BroadScratch) : sizeof(WarpScratch));
 }
 
 template <int A>
 cudaError_t batch_occupancy_impl(int mode, bool seg, int spl, size_t smem_bytes, int warps, int *blocks_per_sm) {
-    if (mode == kBatchArmwise) armwise_shape(A, smem_bytes, warps);
+    batch_shape(A, mode, smem_bytes, warps);
     const void *fn = spl == 2 ? batch_fn<A, 2>(mode, seg) : batch_fn<A, 1>(mode, seg);
     cudaError_t err = prepare_kernel(fn, smem_bytes, nullptr);
     if (err != cudaSuccess) return err;
@@ -181,7 +184,7 @@ cudaError_t batch_occupancy_impl(int mode, bool seg, int spl, size_t smem_bytes,
 template <int A>
 cudaError_t launch_batch_impl(int mode, bool seg, int spl, const BatchParams &b, size_t smem_bytes, int grid,
                               int warps, cudaStream_t stream) {
-    if (mode == kBatchArmwise) armwise_shape(A, smem_bytes, warps);
+    batch_shape(A, mode, smem_bytes, warps);
     const void *fn = spl == 2 ? batch_fn<A, 2>(mode, seg) : batch_fn<A, 1>(mode, seg);
     void *args[] = {(void *)&b};
     return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(32 * warps), args, smem_bytes, stream);
