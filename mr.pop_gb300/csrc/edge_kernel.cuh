@@ -421,28 +421,6 @@ __device__ __forceinline__ bool regular_pose(const float (&q)[7]) {
     return sum <= kRegularRad;
 }
 
-// Exact env test of one sphere against obstacle o (index over all classes in
-// the bound order cuboids, z-cuboids, capsules, z-capsules, spheres).
-__device__ __forceinline__ bool env_exact(const float4 *S, const SceneLayout &L, const SceneCounts &C, int o, float x,
-                                          float y, float z, float r) {
-    if (o < C.n_cub) {
-        const float4 *c = S + L.cub + 4 * o;
-        return hit_cuboid(c[0], c[1], c[2], c[3], x, y, z, __fmul_rn(r, r));
-    }
-    o -= C.n_cub;
-    if (o < C.n_zcub) {
-        const float4 *c = S + L.zcub + 4 * o;
-        return hit_zcuboid(c[0], c[1], c[2], x, y, z, __fmul_rn(r, r));
-    }
-    o -= C.n_zcub;
-    if (o < C.n_cap) return hit_capsule(S[L.cap + 2 * o], S[L.cap + 2 * o + 1], x, y, z, r);
-    o -= C.n_cap;
-    if (o < C.n_zcap) return hit_zcapsule(S[L.zcap + 2 * o], S[L.zcap + 2 * o + 1], x, y, z, r);
-    o -= C.n_zcap;
-    const float4 c0 = S[L.sph + o];
-    return hit_sphere_sphere(c0.x, c0.y, c0.z, c0.w, x, y, z, r);
-}
-
 // ---------------------------------------------------------------------------
 // broad phase: approx spheres 1..10 of one arm (lane column `lane` of sp)
 // against the scene.  Returns this lane's joints with a sphere that touches an
@@ -852,7 +830,7 @@ __host__ __device__ __forceinline__ constexpr uint32_t hand_part(int s) {
 }
 
 // Conservative screen of obstacle o (index over all classes, in the order of
-// env_exact) against ball U: the obstacle's bounding sphere, then for cuboids
+// load_obstacle) against ball U: the obstacle's bounding sphere, then for cuboids
 // with orthonormal axes the exact sphere-cuboid test with U's radius.
 __device__ __forceinline__ bool screen_obstacle(const float4 *S, const SceneLayout &L, const SceneCounts &C, int o,
                                                 float4 U) {
@@ -871,13 +849,70 @@ __device__ __forceinline__ bool screen_obstacle(const float4 *S, const SceneLayo
     return true;
 }
 
-// Env test of the spheres of sub-group g (sphere 0 is never env-tested) for
-// the lanes with act set; every lane of the warp calls it.  The active lanes'
-// group bounds are merged into one ball U (box of their centres, half
-// diagonal + group radius); obstacles are screened against U one per lane, 32
-// at a time, and each active lane tests its spheres against the survivors.
+// Lanes 0..lane: a hit on any of them settles the lane's sample.
+__device__ __forceinline__ uint32_t lanes_upto(int lane) { return (2u << lane) - 1u; }
+
+// One obstacle, its record in registers (the same in every lane).  kind: 0
+// cuboid, 1 z-cuboid, 2 capsule, 3 z-capsule, 4 sphere.
+struct Obstacle {
+    float4 c0, c1, c2, c3;
+    float4 bound;  // bounding sphere (+margin); radius 1e18 for a cuboid with skewed axes
+    int kind;
+    // the reference's test of a sphere
+    __device__ __forceinline__ bool hit(float3 p, float r) const {
+        if (kind == 0) return hit_cuboid(c0, c1, c2, c3, p.x, p.y, p.z, __fmul_rn(r, r));
+        if (kind == 1) return hit_zcuboid(c0, c1, c2, p.x, p.y, p.z, __fmul_rn(r, r));
+        if (kind == 2) return hit_capsule(c0, c1, p.x, p.y, p.z, r);
+        if (kind == 3) return hit_zcapsule(c0, c1, p.x, p.y, p.z, r);
+        return hit_sphere_sphere(c0.x, c0.y, c0.z, c0.w, p.x, p.y, p.z, r);
+    }
+    // the test itself bounds what a ball holds (distance to a box)
+    __device__ __forceinline__ bool metric() const { return kind < 2 && bound.w <= 1e17f; }
+};
+
+// Obstacle o over all classes, in the order of the bounds.
+__device__ __forceinline__ Obstacle load_obstacle(const float4 *S, const SceneLayout &L, const SceneCounts &C, int o) {
+    Obstacle b;
+    b.bound = S[L.b_cub + o];
+    const float4 *r;
+    if (o < C.n_cub) {
+        b.kind = 0;
+        r = S + L.cub + 4 * o;
+        b.c3 = r[3];
+    } else if ((o -= C.n_cub) < C.n_zcub) {
+        b.kind = 1;
+        r = S + L.zcub + 4 * o;
+    } else if ((o -= C.n_zcub) < C.n_cap) {
+        b.kind = 2;
+        r = S + L.cap + 2 * o;
+    } else if ((o -= C.n_cap) < C.n_zcap) {
+        b.kind = 3;
+        r = S + L.zcap + 2 * o;
+    } else {
+        b.kind = 4;
+        r = S + L.sph + o - C.n_zcap;
+    }
+    b.c0 = r[0];
+    if (b.kind < 4) b.c1 = r[1];
+    if (b.kind < 2) b.c2 = r[2];
+    return b;
+}
+
+// Env test of the detailed spheres first + (bits of spheres), one sub-group or
+// hand part with bound gl in frame T, for the lanes with act set; every lane of
+// the warp calls it.  The active lanes' bounds are merged into one ball U (box
+// of their centres, half diagonal + bound); obstacles are screened against U one
+// per lane, 32 at a time.  Each survivor then meets the lanes' own bounds (the
+// exact test for boxes with orthonormal axes, the bounding sphere otherwise) and,
+// if some lane's reaches it, its spheres.  A hit settles the lane and those
+// above it.  Returns true for a lane that hit.
+// The slowest edges set the time of calls of up to some ten thousand edges; in
+// those, most survivors of U are near no lane's bound, and every lane tested
+// every sphere of the whole hand against them: the slowest of 30011 one-arm
+// edges takes 94 k cycles in place of 246 k, the kernel 139 -> 81 us; 65536
+// 4-arm edges 457 -> 433 us.
 __device__ __forceinline__ bool env_group_warp(const float4 *S, const SceneLayout &L, const SceneCounts &C,
-                                                   const Xf &T, int g, float4 gl, bool act) {
+                                                   const Xf &T, int first, uint32_t spheres, float4 gl, bool act) {
     const int lane = threadIdx.x & 31;
     const float3 gc = place_reg(T, gl);
     constexpr float kBig = 3.0e38f;
@@ -888,29 +923,40 @@ __device__ __forceinline__ bool env_group_warp(const float4 *S, const SceneLayou
     const float4 U = make_float4(0.5f * (lx + hx), 0.5f * (ly + hy), 0.5f * (lz + hz),
                                  0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + gl.w);
     const int n_obst = C.n_cub + C.n_zcub + C.n_cap + C.n_zcap + C.n_sph;
-    const int i0 = grp_first(g) == 0 ? 1 : grp_first(g), i1 = grp_first(g + 1);
     bool hit = false;
 #pragma unroll 1
     for (int base = 0; base < n_obst; base += 32) {
-        if (__all_sync(kFull, !act || hit)) break;
         const int o = base + lane;
-        const uint32_t m = __ballot_sync(kFull, o < n_obst && screen_obstacle(S, L, C, o, U));
+        uint32_t m = __ballot_sync(kFull, o < n_obst && screen_obstacle(S, L, C, o, U));
         MRPOP_COUNT_W(11, 1);
         MRPOP_COUNT_W(12, __popc(m));
-        MRPOP_COUNT_LANES(13, act && !hit);
-        if (!m || !act || hit) continue;
-        for (int i = i0; i < i1 && !hit; i++) {
-            const float4 sd = c_det[i];
-            const float3 p = place_reg(T, sd);
-            uint32_t mm = m;
-            while (mm) {
-                const int t = __ffs(mm) - 1;
-                mm &= mm - 1;
-                if (near3(p.x, p.y, p.z, S[L.b_cub + base + t], sd.w) &&
-                    env_exact(S, L, C, base + t, p.x, p.y, p.z, sd.w)) {
-                    hit = true;
-                    break;
+        MRPOP_COUNT_LANES(13, act);
+#pragma unroll 1
+        for (; m; m &= m - 1) {
+            const Obstacle b = load_obstacle(S, L, C, base + __ffs(m) - 1);
+            // the bound first, then the spheres: one copy of the tests
+            float4 sd = gl;
+            float3 p = gc;
+            uint32_t rest = spheres;
+            bool reached = false, h = false;
+            for (bool bound = true;; bound = false) {
+                const bool t = bound && !b.metric() ? near3(p.x, p.y, p.z, b.bound, sd.w) : b.hit(p, sd.w);
+                if (bound) {
+                    reached = act && t;
+                    if (!__any_sync(kFull, reached)) break;
+                } else {
+                    h |= t;
                 }
+                if (!rest) break;
+                sd = c_det[first + __ffs(rest) - 1];
+                rest &= rest - 1;
+                p = place_reg(T, sd);
+            }
+            const uint32_t hb = __ballot_sync(kFull, reached && h);
+            if (hb) {
+                hit |= reached && h;
+                act = act && !(hb & lanes_upto(lane));
+                if (!__any_sync(kFull, act)) return hit;
             }
         }
     }
@@ -941,9 +987,6 @@ struct LaneCtx {
     }
 };
 
-// Lanes 0..lane: a hit on any of them settles the lane's sample.
-__device__ __forceinline__ uint32_t lanes_upto(int lane) { return (2u << lane) - 1u; }
-
 // Joint j of one arm, frame T: env tests of an env-flagged joint (lane_env);
 // stash of the first spheres of flagged rows, and the row tests whose targets
 // are here, screened by the target group's bound (lane_rows).
@@ -951,9 +994,18 @@ __device__ __forceinline__ void lane_env(int j, const EdgeParams &P, const Xf &T
                                          const SceneLayout &L) {
     // every lane takes part in the env screening (warp-wide votes inside)
     if (__any_sync(kFull, c.em >> j & 1u)) {
+        // the hand's spheres in its three parts
 #pragma unroll 1
-        for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++)
-            if (env_group_warp(S, L, P.sc, T, g, P.grp[g], c.em >> j & 1u)) c.set_hit();
+        for (int g = jgrp_first(j); g < jgrp_first(j + 1) + (j == 7 ? kHandParts - 1 : 0); g++) {
+            const int part = g - kHandGroup;
+            const int first = part >= 0 ? kHandFirst : grp_first(g);
+            const uint32_t spheres = part >= 0 ? hand_part(part) : (1u << (grp_first(g + 1) - first)) - 1u;
+            if (env_group_warp(S, L, P.sc, T, first, spheres, part >= 0 ? P.hsub[part] : P.grp[g], c.em >> j & 1u))
+                c.set_hit();
+            const uint32_t hb = __ballot_sync(kFull, c.hit);
+            if (hb & lanes_upto(threadIdx.x & 31)) c.em = c.rm = 0;
+            if (!__any_sync(kFull, c.em >> j & 1u)) break;
+        }
     }
 }
 
