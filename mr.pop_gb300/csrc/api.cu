@@ -451,43 +451,6 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
     p.phase = g_phase_counters;
     p.env_test_flops = scene->env_test_flops;
     p.row5 = scene->row5;
-    static const int kGroupFirst[12] = {0, 1, 5, 9, 13, 17, 19, 21, 29, 32, 37, 59};
-    for (int gi = 0; gi < 11; gi++) {
-        double lo[3] = {1e9, 1e9, 1e9}, hi[3] = {-1e9, -1e9, -1e9};
-        for (int i = kGroupFirst[gi]; i < kGroupFirst[gi + 1]; i++) {
-            const double v[3] = {kDet[i].x, kDet[i].y, kDet[i].z};
-            for (int c = 0; c < 3; c++) {
-                lo[c] = std::fmin(lo[c], v[c]);
-                hi[c] = std::fmax(hi[c], v[c]);
-            }
-        }
-        const double cx = 0.5 * (lo[0] + hi[0]), cy = 0.5 * (lo[1] + hi[1]), cz = 0.5 * (lo[2] + hi[2]);
-        double r = 0.0;
-        for (int i = kGroupFirst[gi]; i < kGroupFirst[gi + 1]; i++) {
-            const SphereDef &d = kDet[i];
-            r = std::fmax(r, std::sqrt((d.x - cx) * (d.x - cx) + (d.y - cy) * (d.y - cy) + (d.z - cz) * (d.z - cz)) + d.r);
-        }
-        p.grp[gi] = make_float4((float)cx, (float)cy, (float)cz, (float)(r * 1.001 + kCullMargin));
-    }
-    // the hand group's three parts (bits of hand_part over spheres kHandFirst..)
-    for (int s = 0; s < kHandParts; s++) {
-        double lo[3] = {1e9, 1e9, 1e9}, hi[3] = {-1e9, -1e9, -1e9};
-        for (uint32_t m = hand_part(s); m; m &= m - 1) {
-            const SphereDef &d = kDet[kHandFirst + __builtin_ctz(m)];
-            const double v[3] = {d.x, d.y, d.z};
-            for (int c = 0; c < 3; c++) {
-                lo[c] = std::fmin(lo[c], v[c]);
-                hi[c] = std::fmax(hi[c], v[c]);
-            }
-        }
-        const double cx = 0.5 * (lo[0] + hi[0]), cy = 0.5 * (lo[1] + hi[1]), cz = 0.5 * (lo[2] + hi[2]);
-        double r = 0.0;
-        for (uint32_t m = hand_part(s); m; m &= m - 1) {
-            const SphereDef &d = kDet[kHandFirst + __builtin_ctz(m)];
-            r = std::fmax(r, std::sqrt((d.x - cx) * (d.x - cx) + (d.y - cy) * (d.y - cy) + (d.z - cz) * (d.z - cz)) + d.r);
-        }
-        p.hsub[s] = make_float4((float)cx, (float)cy, (float)cz, (float)(r * 1.001 + kCullMargin));
-    }
     A = arm >= 0 ? 1 : robots->n_arms;
     for (int a = 0; a < A; a++)
         for (int i = 0; i < 12; i++) p.base[a][i] = robots->base[arm >= 0 ? arm : a][i];

@@ -87,7 +87,10 @@ static __device__ unsigned long long *g_dev_phase;
 constexpr int kWarpsPerBlock = 6;
 constexpr int kMaxArms = 5;
 constexpr int kMaxDof = 7 * kMaxArms;
-constexpr int kCrossStash = 8;         // per-lane arm-vs-arm candidate spheres
+// Per-lane arm-vs-arm candidate spheres: a full stash costs another walk of both
+// arms, a larger one scratch.  The arm-per-warp kernels run few CTAs and take as
+// long as their slowest edge; the others fill the SMs.
+constexpr int kCrossStash = 7, kArmCrossStash = 10;
 constexpr float kCullMargin = 1e-3f;   // metres added to every bounding radius
 
 struct SceneCounts {
@@ -150,8 +153,6 @@ struct EdgeParams {
     int32_t *snseg;             // segmented rules: per-edge segment count (-1: too many), from segment 0
     int32_t *sdone;             // segmented rules: per-edge verdict written
     unsigned long long *work;   // split kernels: next-edge counters {broad, narrow, rows}, zero before each launch
-    float4 grp[11];             // detailed sub-group bounds in their joint frame (+margin)
-    float4 hsub[3];             // bounds of the hand group's three parts in the joint-7 frame (+margin)
     const uint32_t *row5;       // forearm-hand rows table (kRow5N6 x kRow5N7 bits), or nullptr
     float base[kMaxArms][12];   // row-major 3x4 per arm of this check
 };
@@ -174,7 +175,9 @@ struct BroadScratch : EdgeScratch {
     BroadPart broad;
 };
 
-struct WarpScratch : EdgeScratch {
+template <int STASH>
+struct WarpScratchT : EdgeScratch {
+    static constexpr int kStash = STASH;
     union {
         BroadPart broad;
         struct {                                // arm-per-warp kernel: the warp's own arm, both slots
@@ -183,12 +186,14 @@ struct WarpScratch : EdgeScratch {
         } arm;
         float stash[kDetRows][3][32];           // first sphere of each detailed self row
         struct {                                // arm-vs-arm test of one arm pair
-            float gc[11][3][32];                // the upper arm's sub-group centres
-            float xs[kCrossStash][4][32];       // the lower arm's candidate spheres {x, y, z, r} ...
-            uint32_t xm[kCrossStash][32];       // ... and the upper arm's sub-groups each can reach
+            float gc[13][3][32];                // the upper arm's sub-group and hand part centres
+            float xs[STASH][4][32];             // the lower arm's candidate spheres {x, y, z, r} ...
+            uint32_t xm[STASH][32];             // ... and the upper arm's sub-groups each can reach
         } cross;
     };
 };
+using WarpScratch = WarpScratchT<kCrossStash>;
+using ArmScratch = WarpScratchT<kArmCrossStash>;  // arm-per-warp kernels
 
 // Flag words of one sample: 8 bits (joints) per arm.
 template <int A>
@@ -807,7 +812,7 @@ __device__ __forceinline__ float3 place_reg(const Xf &T, float4 s) {
 
 // Sub-groups of the detailed spheres (contiguous index ranges within one
 // joint): [0] [1-4] [5-8] [9-12] [13-16] [17-18] [19-20] [21-28] [29-31]
-// [32-36] [37-58].  EdgeParams::grp holds each group's bounding sphere in its
+// [32-36] [37-58].  SetBounds::grp holds each group's bounding sphere in its
 // joint frame; a group's world bound is that centre through the joint frame.
 constexpr int kNumGroups = 11;
 __host__ __device__ __forceinline__ constexpr int grp_first(int g) {
@@ -821,13 +826,55 @@ __host__ __device__ __forceinline__ constexpr int jgrp_first(int j) {
 // The hand group (spheres 37..58: a 6 x 3 grid along the gripper's diagonal
 // plus four finger-tip spheres) is screened in three parts along the diagonal:
 // the two columns and finger tips on each side, and the two middle columns.
-// Bits are sphere index - kHandFirst; EdgeParams::hsub holds each part's bound.
+// Bits are sphere index - kHandFirst; SetBounds::hsub holds each part's bound.
 constexpr int kHandGroup = 10;
 constexpr int kHandFirst = 37;
 constexpr int kHandParts = 3;
 __host__ __device__ __forceinline__ constexpr uint32_t hand_part(int s) {
     return s == 0 ? 0x3030C3u : s == 1 ? 0x00C30Cu : 0x0F0C30u;
 }
+
+// Bounding spheres of the sub-groups and of the hand's parts in their joint
+// frames (+margin): the centre of the box around the spheres' centres.  In
+// constant memory, not in the kernels' parameters: the batch kernels, which keep
+// those in shared memory, read them as operands too.
+struct SetBounds {
+    float4 grp[kNumGroups];
+    float4 hsub[kHandParts];
+};
+constexpr double const_sqrt(double v) {
+    double x = v > 1.0 ? v : 1.0;
+    for (int i = 0; i < 64; i++) x = 0.5 * (x + v / x);
+    return x;
+}
+// the spheres first + (bits of m)
+constexpr float4 set_ball(int first, uint32_t m) {
+    double lo[3] = {1e9, 1e9, 1e9}, hi[3] = {-1e9, -1e9, -1e9}, r = 0.0;
+    for (int i = 0; i < 32; i++) {
+        if (!(m >> i & 1u)) continue;
+        const double v[3] = {kDet[first + i].x, kDet[first + i].y, kDet[first + i].z};
+        for (int c = 0; c < 3; c++) {
+            lo[c] = v[c] < lo[c] ? v[c] : lo[c];
+            hi[c] = v[c] > hi[c] ? v[c] : hi[c];
+        }
+    }
+    const double x = 0.5 * (lo[0] + hi[0]), y = 0.5 * (lo[1] + hi[1]), z = 0.5 * (lo[2] + hi[2]);
+    for (int i = 0; i < 32; i++) {
+        if (!(m >> i & 1u)) continue;
+        const SphereDef &d = kDet[first + i];
+        const double e = const_sqrt((d.x - x) * (d.x - x) + (d.y - y) * (d.y - y) + (d.z - z) * (d.z - z)) + d.r;
+        r = e > r ? e : r;
+    }
+    return float4{(float)x, (float)y, (float)z, (float)(r * 1.001 + kCullMargin)};
+}
+constexpr SetBounds make_set_bounds() {
+    SetBounds b{};
+    for (int g = 0; g < kNumGroups; g++)
+        b.grp[g] = set_ball(grp_first(g), (1u << (grp_first(g + 1) - grp_first(g))) - 1u);
+    for (int s = 0; s < kHandParts; s++) b.hsub[s] = set_ball(kHandFirst, hand_part(s));
+    return b;
+}
+static __constant__ SetBounds c_bounds = make_set_bounds();
 
 // Conservative screen of obstacle o (index over all classes, in the order of
 // load_obstacle) against ball U: the obstacle's bounding sphere, then for cuboids
@@ -987,6 +1034,28 @@ struct LaneCtx {
     }
 };
 
+// Sphere sets of the arm-pair and env tests: the sub-groups, the hand whole as
+// set 10 or (PARTS) in its three parts as sets 10..12.  Sets of joint j:
+// [jgrp_first(j), set_end(j)); the bound of set t; its spheres, first + (bits of
+// set_spheres); the sets of the joints in jm.
+template <bool PARTS>
+__device__ __forceinline__ int set_end(int j) {
+    return jgrp_first(j + 1) + (PARTS && j == 7 ? kHandParts - 1 : 0);
+}
+template <bool PARTS>
+__device__ __forceinline__ float4 set_bound(int t) {
+    return !PARTS || t < kHandGroup ? c_bounds.grp[t] : c_bounds.hsub[t - kHandGroup];
+}
+__device__ __forceinline__ int set_first(int t) { return t < kHandGroup ? grp_first(t) : kHandFirst; }
+template <bool PARTS>
+__device__ __forceinline__ uint32_t set_spheres(int t) {
+    return !PARTS || t < kHandGroup ? (1u << (grp_first(t + 1) - grp_first(t))) - 1u : hand_part(t - kHandGroup);
+}
+template <bool PARTS>
+__device__ __forceinline__ uint32_t joint_sets(uint32_t jm) {
+    return (jm & 0x1fu) | (jm >> 5 & 1u) * 0xe0u | (jm >> 6 & 1u) << 8 | (jm >> 7 & 1u) * (PARTS ? 0x1e00u : 0x600u);
+}
+
 // Joint j of one arm, frame T: env tests of an env-flagged joint (lane_env);
 // stash of the first spheres of flagged rows, and the row tests whose targets
 // are here, screened by the target group's bound (lane_rows).
@@ -996,11 +1065,9 @@ __device__ __forceinline__ void lane_env(int j, const EdgeParams &P, const Xf &T
     if (__any_sync(kFull, c.em >> j & 1u)) {
         // the hand's spheres in its three parts
 #pragma unroll 1
-        for (int g = jgrp_first(j); g < jgrp_first(j + 1) + (j == 7 ? kHandParts - 1 : 0); g++) {
-            const int part = g - kHandGroup;
-            const int first = part >= 0 ? kHandFirst : grp_first(g);
-            const uint32_t spheres = part >= 0 ? hand_part(part) : (1u << (grp_first(g + 1) - first)) - 1u;
-            if (env_group_warp(S, L, P.sc, T, first, spheres, part >= 0 ? P.hsub[part] : P.grp[g], c.em >> j & 1u))
+        for (int g = jgrp_first(j); g < set_end<true>(j); g++) {
+            if (env_group_warp(S, L, P.sc, T, set_first(g), set_spheres<true>(g), set_bound<true>(g),
+                               c.em >> j & 1u))
                 c.set_hit();
             const uint32_t hb = __ballot_sync(kFull, c.hit);
             if (hb & lanes_upto(threadIdx.x & 31)) c.em = c.rm = 0;
@@ -1009,8 +1076,8 @@ __device__ __forceinline__ void lane_env(int j, const EdgeParams &P, const Xf &T
     }
 }
 
-template <int A>
-__device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &T, LaneCtx &c, WarpScratch &W,
+template <int A, typename WS>
+__device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &T, LaneCtx &c, WS &W,
                                           const float4 *det_tab, int lane) {
     if (!c.rm) return;
     uint32_t m1 = c.rm & c_rows.jfirst[c.quirk][j];
@@ -1026,7 +1093,7 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
         uint32_t rows = c.rm & c_rows.cover[grp_first(g)];
         if (!rows) continue;
-        const float4 gl = P.grp[g];
+        const float4 gl = c_bounds.grp[g];
         const float3 gc = place_reg(T, gl);
         uint32_t nr = 0;
         while (rows) {
@@ -1044,7 +1111,7 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
             // more than they save)
 #pragma unroll 1
             for (int s = 0; s < kHandParts; s++) {
-                const float4 sl = P.hsub[s];
+                const float4 sl = c_bounds.hsub[s];
                 const float3 sc = place_reg(T, sl);
                 uint32_t ns = 0;
                 for (uint32_t m = nr; m; m &= m - 1) {
@@ -1158,7 +1225,7 @@ struct RowTargets {
     __device__ __forceinline__ void reach(const EdgeParams &P, float r) {
 #pragma unroll
         for (int t = 0; t < 6; t++) {
-            const float v = P.grp[5 + t].w + r + mv[t];
+            const float v = c_bounds.grp[5 + t].w + r + mv[t];
             rr[t] = v * v;
         }
     }
@@ -1224,7 +1291,7 @@ __device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const Edge
     RowTargets t;
 #pragma unroll
     for (int i = 0; i < 6; i++) {
-        t.c[i] = make_float3(P.grp[5 + i].x, P.grp[5 + i].y, P.grp[5 + i].z);
+        t.c[i] = make_float3(c_bounds.grp[5 + i].x, c_bounds.grp[5 + i].y, c_bounds.grp[5 + i].z);
         t.mv[i] = 0.0f;
     }
     uint32_t rows = quirk ? ~0x1ffffu : ~0x1fffu;
@@ -1286,39 +1353,40 @@ __device__ __forceinline__ RowScreen screen_rows(const EdgeParams &P, const Edge
 }
 
 // Lower arm, joint j (flagged for this lane): its spheres from index `from` on
-// that can reach one of the upper arm's sub-groups gb (bounds, centres in
-// W.cross.gc) go to the lane's stash with the sub-groups they reach;
-// `next` receives the first sphere left out when the stash is full.
+// that can reach one of the upper arm's sets gb (bounds, centres in W.cross.gc)
+// go to the lane's stash with the sets they reach; `next` receives the first
+// sphere left out when the stash is full.
+template <bool PARTS, typename WS>
 __device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf &T, uint32_t gb, int from, int &n,
-                                            int &next, WarpScratch &W, int lane) {
+                                            int &next, WS &W, int lane) {
     auto &X = W.cross;
 #pragma unroll 1
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
         if (grp_first(g + 1) <= from) continue;
-        const float4 gl = P.grp[g];
+        const float4 gl = c_bounds.grp[g];
         const float3 gc = place_reg(T, gl);
         uint32_t near = 0;
         for (uint32_t m = gb; m; m &= m - 1) {
             const int t = __ffs(m) - 1;
-            if (near3(gc.x, gc.y, gc.z, make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], P.grp[t].w),
-                      gl.w))
+            if (near3(gc.x, gc.y, gc.z,
+                      make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], set_bound<PARTS>(t).w), gl.w))
                 near |= 1u << t;
         }
         if (!near) continue;
 #pragma unroll 1
-        for (int i = max(grp_first(g), from); i < grp_first(g + 1); i++) {
-            const float4 sd = c_det[i];
+        for (int at = max(grp_first(g), from); at < grp_first(g + 1); at++) {
+            const float4 sd = c_det[at];
             const float3 p = place_reg(T, sd);
             uint32_t nm = 0;
             for (uint32_t m = near; m; m &= m - 1) {
                 const int t = __ffs(m) - 1;
-                if (near3(p.x, p.y, p.z, make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], P.grp[t].w),
-                          sd.w))
+                if (near3(p.x, p.y, p.z,
+                          make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], set_bound<PARTS>(t).w), sd.w))
                     nm |= 1u << t;
             }
             if (!nm) continue;
-            if (n == kCrossStash) {
-                next = i;
+            if (n == WS::kStash) {
+                next = at;
                 return;
             }
             X.xs[n][0][lane] = p.x;
@@ -1332,17 +1400,18 @@ __device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf
 }
 
 // Upper arm, joint j: its spheres against the stashed spheres that reach their
-// sub-group.
-__device__ __forceinline__ void probe_joint(int j, const Xf &T, int n, bool &hit, WarpScratch &W, int lane) {
+// set.
+template <bool PARTS, typename WS>
+__device__ __forceinline__ void probe_joint(int j, const Xf &T, int n, bool &hit, WS &W, int lane) {
     auto &X = W.cross;
 #pragma unroll 1
-    for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
+    for (int g = jgrp_first(j); g < set_end<PARTS>(j); g++) {
         uint32_t em = 0;
         for (int e = 0; e < n; e++) em |= (X.xm[e][lane] >> g & 1u) << e;
         if (!em) continue;
         bool h = false;
-        for (int i = grp_first(g); i < grp_first(g + 1); i++) {
-            const float4 sd = c_det[i];
+        for (uint32_t rest = set_spheres<PARTS>(g); rest; rest &= rest - 1) {
+            const float4 sd = c_det[set_first(g) + __ffs(rest) - 1];
             const float3 p = place_reg(T, sd);
             for (uint32_t m = em; m; m &= m - 1) {
                 const int e = __ffs(m) - 1;
@@ -1356,11 +1425,6 @@ __device__ __forceinline__ void probe_joint(int j, const Xf &T, int n, bool &hit
             return;
         }
     }
-}
-
-// Sub-groups of the joints in jm.
-__device__ __forceinline__ uint32_t joint_groups(uint32_t jm) {
-    return (jm & 0x1fu) | (jm >> 5 & 1u) * 0xe0u | (jm >> 6 & 1u) << 8 | (jm >> 7 & 1u) * 0x600u;
 }
 
 // Shared words of a CTA whose warps take one arm each (armwise_kernel).
@@ -1395,8 +1459,9 @@ __device__ __forceinline__ int take_pair(unsigned int *c, int lane) {
 //            that some approx sphere pair's swept bounds connect in the slot
 //            (pms: lane p holds pair p's; a joint's detailed spheres lie inside
 //            its approx spheres but for 0.6 mm, and those bounds carry 1 mm
-//            each).  Arm b's sub-group centres are placed first; arm a's
-//            spheres are tested against them by sub-group and one by one, so
+//            each).  Arm b's sub-group centres are placed first (the hand in
+//            its three parts); arm a's spheres are tested against them by
+//            sub-group and one by one, so
 //            that only spheres that can reach arm b are stashed; arm b is
 //            walked again only if some lane stashed any.
 // Bound by instruction issue.  Against the first form of the arm-pair test
@@ -1415,17 +1480,23 @@ __device__ __forceinline__ int take_pair(unsigned int *c, int lane) {
 // are shared through X->hits (a stale read only costs tests).
 constexpr int kStageAll = 0, kStageEnvPairs = 1, kStageRows = 2;
 
-template <int A, bool ONE = false, int STAGE = kStageAll>
-__device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch &W, const float4 *S,
+template <int A, bool ONE = false, int STAGE = kStageAll, typename WS>
+__device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WS &W, const float4 *S,
                                                 const SceneLayout &L, const float4 *det_tab, int seg, int k0,
                                                 Flags<A> ew, Flags<A> sw, bool dE, bool dS, uint32_t pms,
                                                 int one_arm = 0, ArmShare *X = nullptr, int slot = 0) {
     const int lane = threadIdx.x & 31;
     const int k = min(k0 + lane + 1, P.g);
     static_assert(!ONE || STAGE == kStageAll, "the arm-per-warp kernel runs every test");
-    constexpr bool with_env = STAGE != kStageRows, with_rows = STAGE != kStageEnvPairs;
+    constexpr bool with_env = STAGE != kStageRows, with_rows = STAGE == kStageAll || STAGE == kStageRows;
     constexpr bool with_pairs = A > 1 && STAGE != kStageRows;
     constexpr int kArm = 0, kCentres = 1, kStash = 2, kProbe = 3;  // jobs
+    // The upper arm's hand in its three parts: fewer spheres reach it, at more
+    // tests each.  The slowest edges gain (300 5-arm extend checks 92.7 -> 80
+    // us, with a stash of 10 in place of 8), and 65536 4-arm edges (433 -> 411
+    // us); 262144 5-arm edges, most of which collide at their first sample,
+    // took 3.43 in place of 3.27 ms.
+    constexpr bool kParts = ONE || A <= 4;
     const int arm0 = ONE ? one_arm : 0, arm1 = ONE ? one_arm + 1 : A;
     LaneCtx c;
     c.quirk = (!P.single && !(P.flags & kExactBit)) ? 1 : 0;
@@ -1512,7 +1583,7 @@ __device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch
         }
         // walk the arm's chain
         const uint32_t before = __ballot_sync(kFull, c.hit);
-        const uint32_t gb = joint_groups(jb);
+        const uint32_t gb = joint_sets<kParts>(jb);
         Xf T;
         load_base(T, P.base[arm]);
 #pragma unroll 1
@@ -1520,18 +1591,18 @@ __device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch
             if (with_pairs && job != kArm) {
                 if (job == kStash) {
                     if ((sma >> j & 1u) && next == kNumDet && from < det_first(j + 1))
-                        stash_joint(j, P, T, gb, from, n, next, W, lane);
+                        stash_joint<kParts>(j, P, T, gb, from, n, next, W, lane);
                 } else if (jb >> j & 1u) {
                     if (job == kCentres) {
 #pragma unroll 1
-                        for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
-                            const float3 ctr = place_reg(T, P.grp[g]);
+                        for (int g = jgrp_first(j); g < set_end<kParts>(j); g++) {
+                            const float3 ctr = place_reg(T, set_bound<kParts>(g));
                             W.cross.gc[g][0][lane] = ctr.x;
                             W.cross.gc[g][1][lane] = ctr.y;
                             W.cross.gc[g][2][lane] = ctr.z;
                         }
                     } else if (act && !c.hit && n > 0) {
-                        probe_joint(j, T, n, c.hit, W, lane);
+                        probe_joint<kParts>(j, T, n, c.hit, W, lane);
                     }
                 }
             } else {
@@ -1550,6 +1621,7 @@ __device__ __forceinline__ uint32_t narrow_slot(const EdgeParams &P, WarpScratch
         if (ONE) {
             if (lane == 0 && hb != before) atomicOr(&X->hits[slot], hb);
             hb |= *(const volatile unsigned int *)&X->hits[slot];
+            if (slot > 0 && *(const volatile unsigned int *)&X->hits[0]) hb = kFull;  // settles the edge
         }
         act = act && !(hb & lanes_upto(lane));
         if (!__any_sync(kFull, act)) break;
@@ -1950,13 +2022,20 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 // verdicts are those of the one-warp kernels.  The lower arm's spheres of a
 // pair are read from the warp that placed them instead of being placed again.
 // ---------------------------------------------------------------------------
-template <int A, int SPL>
+// G = 2 (64 samples per segment, calls so small that the SMs have room): two
+// warps per arm, each one 32-sample slot of it; a slot's arm pairs are shared by
+// the slot's warps.
+template <int A, int SPL, int G>
 __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char *wbase, const float4 *S,
                                              const SceneLayout &L, const float4 *det_tab, long long e, int dof,
-                                             int g, int lane, int arm, ArmShare &X, bool staged) {
-    WarpScratch &W = reinterpret_cast<WarpScratch *>(wbase)[arm];
+                                             int g, int lane, int warp, ArmShare &X, bool staged) {
+    ArmScratch &W = reinterpret_cast<ArmScratch *>(wbase)[warp];
+    const int arm = G > 1 && warp >= A ? warp - A : warp, grp = G > 1 && warp >= A ? 1 : 0;
+    static_assert(G == 1 || SPL == 2, "a warp per slot");
+    constexpr bool by_slot = G > 1;
+    const int s0 = by_slot ? grp : 0, s1 = by_slot ? grp + 1 : SPL;  // this warp's slots
     if (!staged) {
-        if (arm == 0 && lane == 0) {
+        if (warp == 0 && lane == 0) {
             P.valid[e] = 0;
             P.first_hit[e] = -2;
         }
@@ -1968,7 +2047,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
     const bool do_env = P.flags & kEnvBit, do_self = P.flags & kSelfBit;
     int first = 0;
     for (int seg = 0; seg < nseg_run && first == 0; seg++) {
-        if (arm == 0) {
+        if (warp == 0) {
 #pragma unroll
             for (int t = 0; t < 2; t++) X.env[t][lane] = X.self[t][lane] = 0;
             if (lane < 2) X.hits[lane] = 0;
@@ -1978,7 +2057,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
         // this arm: placement, swept bounds, env and intra-arm screens (the
         // slots' spheres stay in arm.sp for the pair tests)
 #pragma unroll 1
-        for (int s = 0; s < SPL; s++) {
+        for (int s = s0; s < s1; s++) {
             const int k = lane + 1 + 32 * s;
             auto &sp = W.arm.sp[s];
             float4 *sw = W.arm.swept[s];
@@ -2002,15 +2081,19 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
         // they finish (their costs differ): flags go to arm a
         // (panda_four.cuh:178-214); screened by the slot's swept bounds
         if (A > 1 && do_self) {
-            const WarpScratch *Wa = reinterpret_cast<const WarpScratch *>(wbase);
+            const ArmScratch *Wa = reinterpret_cast<const ArmScratch *>(wbase);
 #pragma unroll 1
-            for (int p = take_pair(&X.next[0], lane); p < num_pairs(A); p = take_pair(&X.next[0], lane)) {
+            for (int t = take_pair(&X.next[0], lane); t < num_pairs(A) * (by_slot ? 2 : 1);
+                 t = take_pair(&X.next[0], lane)) {
+                const int p = by_slot && t >= num_pairs(A) ? t - num_pairs(A) : t;
+                const int p0 = by_slot && t >= num_pairs(A) ? 1 : 0, p1 = by_slot ? p0 + 1 : SPL;  // slots
                 int a, b;
                 pair_arms<A>(p, a, b);
 #pragma unroll 1
-                for (int s = 0; s < SPL; s++) {
+                for (int s = p0; s < p1; s++) {
                     const int k = lane + 1 + 32 * s;
-                    const float4 *swa = Wa[a].arm.swept[s], *swb = Wa[b].arm.swept[s];
+                    const ArmScratch &Wl = Wa[(by_slot ? A * s : 0) + a], &Wu = Wa[(by_slot ? A * s : 0) + b];
+                    const float4 *swa = Wl.arm.swept[s], *swb = Wu.arm.swept[s];
                     uint32_t bal[4];
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
@@ -2023,8 +2106,8 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
                         if (lane == 0) X.pm[s][p] = 0;
                         continue;
                     }
-                    const auto &low = Wa[a].arm.sp[s];
-                    const auto &cur = Wa[b].arm.sp[s];
+                    const auto &low = Wl.arm.sp[s];
+                    const auto &cur = Wu.arm.sp[s];
                     uint32_t am = 0, ja = 0, jb = 0;
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
@@ -2069,7 +2152,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
             thread_split<SPL>((P.flags & kExactBit) != 0, g, lane, envc, selfc, tot_env, tot_self, cand_env,
                               cand_self);
 #pragma unroll 1
-            for (int s = 0; s < SPL; s++) {
+            for (int s = s0; s < s1; s++) {
                 // a hit that some warp found in an earlier slot settles the
                 // edge.  Other warps write the word meanwhile, so the branch
                 // takes lane 0's reading for the whole warp
@@ -2090,7 +2173,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
         }
         __syncthreads();  // the shared words are read before the next segment clears them
     }
-    if (arm == 0 && lane == 0) {
+    if (warp == 0 && lane == 0) {
         P.valid[e] = (first == 0 && !too_many) ? 1 : 0;
         P.first_hit[e] = too_many ? -2 : (first ? first : -1);
         if (P.n_seg_out) P.n_seg_out[e] = nseg;
@@ -2098,26 +2181,29 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
 }
 
 // CTAs of the arm-per-warp kernels that fit an SM beside a 51-box scene (their
-// scratch is 11.6 KB per warp).  Given as a launch bound because ptxas, left to
+// scratch is 11.8 KB per warp).  Given as a launch bound because ptxas, left to
 // choose, cuts 5 arms at 64 samples to 72 registers and spills.
-__host__ __device__ constexpr int armwise_min_blocks(int A) { return A >= 5 ? 3 : A == 4 ? 4 : 5; }
+__host__ __device__ constexpr int armwise_min_blocks(int A, int G = 1) {
+    return G > 1 ? (A >= 4 ? 2 : 3) : A >= 5 ? 3 : A == 4 ? 4 : 5;
+}
 
-template <int A, int SPL>
-__global__ void __launch_bounds__(32 * A, armwise_min_blocks(A)) armwise_kernel(const __grid_constant__ EdgeParams P) {
+template <int A, int SPL, int G>
+__global__ void __launch_bounds__(32 * A * G, armwise_min_blocks(A, G))
+    armwise_kernel(const __grid_constant__ EdgeParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ float4 det_tab[kNumDet];
     __shared__ ArmShare X;
     const SceneLayout L = scene_layout(P.sc);
     const float4 *S = reinterpret_cast<const float4 *>(smem_raw);
-    const int arm = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < kNumDet; i += blockDim.x) det_tab[i] = c_det[i];
     const bool staged = stage_scene(reinterpret_cast<float4 *>(smem_raw), P.scene,
                                     (uint32_t)(L.total * sizeof(float4)), &bar, P.status);
     unsigned char *wbase = smem_raw + (size_t)L.total * sizeof(float4);
     const int dof = 7 * (P.single ? 1 : A);
     for (long long e = blockIdx.x; e < P.n_edges; e += gridDim.x)
-        armwise_edge<A, SPL>(P, wbase, S, L, det_tab, e, dof, P.g, lane, arm, X, staged);
+        armwise_edge<A, SPL, G>(P, wbase, S, L, det_tab, e, dof, P.g, lane, warp, X, staged);
 }
 
 // ---------------------------------------------------------------------------
@@ -2490,7 +2576,7 @@ __global__ void __launch_bounds__(32 * A, armwise_min_blocks(A)) batch_armwise_k
         unsigned char *wbase = smem_raw + (size_t)L.total * sizeof(float4);
         const int dof = 7 * (Ps.single ? 1 : A);
         for (int k = 0; k < ch.z; k++)
-            armwise_edge<A, SPL>(Ps, wbase, S, L, det_tab, (long long)ch.y + k, dof, Ps.g, lane, arm, X, staged);
+            armwise_edge<A, SPL, 1>(Ps, wbase, S, L, det_tab, (long long)ch.y + k, dof, Ps.g, lane, arm, X, staged);
         __syncthreads();  // every warp is done with this chunk (and instance)
     }
 }
