@@ -2334,13 +2334,14 @@ __device__ __forceinline__ void narrow_edge(const EdgeParams &P, WarpScratch &W,
         any_pair |= pm[s];
     }
     if (first_stage && !cand_env && !__any_sync(kFull, any_pair)) return; // rows alone
+    // (loaded before the set-up waits for the endpoints, so that both are under way)
+#pragma unroll
+    for (int s = 0; s < SPL; s++) load_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
     const int r = SEG ? P.seg0 : 0;
     constexpr bool segmented = SEG;
     bool too_many;
     const int nseg = edge_setup(P, W, e, dof, g, lane, too_many);
     if (SEG && P.rule == kRuleConnect && r > 0) connect_advance(W, dof, r, lane);
-#pragma unroll
-    for (int s = 0; s < SPL; s++) load_flags<A>(P, e * (32 * SPL) + lane + 32 * s, envw[s], selfw[s]);
     const int fb =
         narrow_segment<A, SPL, STAGE>(P, W, S, L, det_tab, r, lane, envw, selfw, pm, cand_env, cand_self);
     if (lane == 0) {

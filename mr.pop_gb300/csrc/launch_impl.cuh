@@ -77,26 +77,33 @@ const void *kernel_fn(KernelKind kind, bool seg) {
         if constexpr (A > 1) return seg ? (const void *)rows_kernel<A, SPL, true> : (const void *)rows_kernel<A, SPL, false>;
         return nullptr;
     case kFusedPair: return (const void *)pair_kernel<A>;
-    case kArmwise: return (const void *)armwise_kernel<A, SPL, 1>;
     default: return (const void *)validate_kernel<A, SPL>;
     }
 }
 
 template <int A, int SPL>
 const void *batch_fn(int mode, bool seg) {
-    if (mode == kBatchArmwise) return (const void *)batch_armwise_kernel<A, SPL>;
+    // (only groups of 3 to 5 arms run the arm-per-warp kernel, of 2 and more the rows kernel)
+    if (mode == kBatchArmwise) {
+        if constexpr (A >= 3) return (const void *)batch_armwise_kernel<A, SPL>;
+        return nullptr;
+    }
+    if (mode == kBatchRows) {
+        if constexpr (A > 1)
+            return seg ? (const void *)batch_kernel<A, SPL, kBatchRows, true>
+                       : (const void *)batch_kernel<A, SPL, kBatchRows, false>;
+        return nullptr;
+    }
     if (!seg) {
         switch (mode) {
         case kBatchBroad: return (const void *)batch_kernel<A, SPL, kBatchBroad, false>;
         case kBatchNarrow: return (const void *)batch_kernel<A, SPL, kBatchNarrow, false>;
-        case kBatchRows: return (const void *)batch_kernel<A, SPL, kBatchRows, false>;
         default: return (const void *)batch_kernel<A, SPL, kBatchFused, false>;
         }
     }
     switch (mode) {
     case kBatchBroad: return (const void *)batch_kernel<A, SPL, kBatchBroad, true>;
     case kBatchNarrow: return (const void *)batch_kernel<A, SPL, kBatchNarrow, true>;
-    case kBatchRows: return (const void *)batch_kernel<A, SPL, kBatchRows, true>;
     default: return (const void *)batch_kernel<A, SPL, kBatchFused, true>;
     }
 }
@@ -106,33 +113,35 @@ const void *batch_fn(int mode, bool seg) {
 template <int A>
 cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t smem_bytes, cudaStream_t stream) {
     if (kind == kArmwise) {
-        // one edge per CTA at a time, two warps per arm or one; only while
-        // every edge of the call has a CTA of its own (a second round of edges
-        // would double the call's time): then the pair or one-warp kernel.
-        // Two warps per arm against one, 64 samples: 4 arms, 300 connect edges
-        // 113 -> 99 us, 64 shortcut edges 93 -> 66; 3 arms, 300 connect edges
-        // 94 -> 76; 5 arms, 64 shortcut edges 143 -> 121, but 300 connect edges
-        // 151 -> 164 (two 10-warp CTAs per SM at 96 registers), so 5 arms take
-        // them only up to one CTA per SM
-        const size_t scene = smem_bytes - (size_t)kWarpsPerBlock * sizeof(WarpScratch);
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        for (int per_arm = p.g > 32 ? 2 : 1; per_arm >= 1; per_arm--) {
-            const int warps = A * per_arm;
-            const size_t arm_smem = scene + (size_t)warps * sizeof(ArmScratch);
-            if (arm_smem > kMaxDynamicSmem) continue;
-            const void *fn = p.g <= 32      ? (const void *)armwise_kernel<A, 1, 1>
-                             : per_arm == 2 ? (const void *)armwise_kernel<A, 2, 2>
-                                            : (const void *)armwise_kernel<A, 2, 1>;
-            int per_sm = 0;
-            const cudaError_t err = prepare_kernel(fn, arm_smem, &per_sm, 32 * warps);
-            if (err != cudaSuccess) return err;
-            if (per_arm == 2 && A == 5) per_sm = 1;  // (see above)
-            if (p.n_edges <= (long long)sms * (per_sm > 0 ? per_sm : 1)) {
-                void *args[] = {(void *)&p};
-                return cudaLaunchKernel(fn, dim3((unsigned)(p.n_edges > 0 ? p.n_edges : 1)), dim3(32 * warps), args,
-                                        arm_smem, stream);
+        if constexpr (A >= 3) {
+            // one edge per CTA at a time, two warps per arm or one; only while
+            // every edge of the call has a CTA of its own (a second round of edges
+            // would double the call's time): then the pair or one-warp kernel.
+            // Two warps per arm against one, 64 samples: 4 arms, 300 connect edges
+            // 113 -> 99 us, 64 shortcut edges 93 -> 66; 3 arms, 300 connect edges
+            // 94 -> 76; 5 arms, 64 shortcut edges 143 -> 121, but 300 connect edges
+            // 151 -> 164 (two 10-warp CTAs per SM at 96 registers), so 5 arms take
+            // them only up to one CTA per SM
+            const size_t scene = smem_bytes - (size_t)kWarpsPerBlock * sizeof(WarpScratch);
+            int dev = 0, sms = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            for (int per_arm = p.g > 32 ? 2 : 1; per_arm >= 1; per_arm--) {
+                const int warps = A * per_arm;
+                const size_t arm_smem = scene + (size_t)warps * sizeof(ArmScratch);
+                if (arm_smem > kMaxDynamicSmem) continue;
+                const void *fn = p.g <= 32      ? (const void *)armwise_kernel<A, 1, 1>
+                                 : per_arm == 2 ? (const void *)armwise_kernel<A, 2, 2>
+                                                : (const void *)armwise_kernel<A, 2, 1>;
+                int per_sm = 0;
+                const cudaError_t err = prepare_kernel(fn, arm_smem, &per_sm, 32 * warps);
+                if (err != cudaSuccess) return err;
+                if (per_arm == 2 && A == 5) per_sm = 1;  // (see above)
+                if (p.n_edges <= (long long)sms * (per_sm > 0 ? per_sm : 1)) {
+                    void *args[] = {(void *)&p};
+                    return cudaLaunchKernel(fn, dim3((unsigned)(p.n_edges > 0 ? p.n_edges : 1)), dim3(32 * warps), args,
+                                            arm_smem, stream);
+                }
             }
         }
         kind = p.g > 32 ? kFusedPair : kFused;
