@@ -108,7 +108,7 @@ cudaError_t timed_launch(int arms, mrpop::KernelKind kind, const mrpop::EdgePara
     if (!on) return mrpop::launch_validate(arms, kind, p, smem, stream);
     TimedLaunch t{nullptr, nullptr,
                   (int)(kind == mrpop::kFusedPair || kind == mrpop::kArmwise ? mrpop::kFused
-                        : kind == mrpop::kRows                               ? mrpop::kNarrow
+                        : kind == mrpop::kRows || kind == mrpop::kNarrowAll  ? mrpop::kNarrow
                                                                              : kind)};
     cudaError_t e = cudaEventCreate(&t.start);
     if (e == cudaSuccess) e = cudaEventCreate(&t.stop);
@@ -481,6 +481,18 @@ void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int
     p.sdone = p.snseg + n_edges;
 }
 
+// Largest calls whose narrow phase is one kernel (kNarrowAll) instead of
+// kNarrow and kRows.  Up to some edges per resident warp each kernel of a round
+// takes as long as its slowest edge, so a third kernel adds a third tail; above
+// that the larger kernel's instruction fetches cost more (its hot code grows with
+// the arm pairs and passes the SM's instruction cache).  Whole calls, one kernel
+// against two: 4 arms x 32 samples, 4134 edges 130 / 156 us, 9000 270 / 271, 22000
+// 402 / 364; 5 arms x 64, 3000 258 / 350, 6000 401 / 435, 22000 980 / 870; 2 arms x
+// 64, 24990 327 / 335, x 16, 214 / 237.  Segment rounds get emptier one by one, so their call may
+// be twice as large: shortcut, 4 arms x 32, 12000 778 / 882 us, 26000 1257 / 1221;
+// 5 arms x 64, 8000 1304 / 1441, 18000 2161 / 2070.
+constexpr int64_t one_narrow_edges(int A, bool rounds) { return 100000 / (A * A) * (rounds ? 2 : 1); }
+
 // ext_scratch: caller-provided device scratch for the single-segment pipeline
 // (at least split_scratch_bytes(n_edges, g, arms) bytes); nullptr = the
 // library's stream-ordered pool.
@@ -553,8 +565,10 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
             p.seg0 = r;
             err = cudaMemsetAsync(p.work, 0, 3 * sizeof(unsigned long long), stream);
             if (err == cudaSuccess) err = timed_launch(A, kBroad, p, smem, stream);
-            if (err == cudaSuccess) err = timed_launch(A, kNarrow, p, smem, stream);
-            if (err == cudaSuccess && A > 1) err = timed_launch(A, kRows, p, smem, stream);
+            // (one arm has no rows kernel)
+            const bool one = A > 1 && n_edges <= one_narrow_edges(A, rounds > 1);
+            if (err == cudaSuccess) err = timed_launch(A, one ? kNarrowAll : kNarrow, p, smem, stream);
+            if (err == cudaSuccess && A > 1 && !one) err = timed_launch(A, kRows, p, smem, stream);
         }
         if (err == cudaSuccess && rule != MRPOP_RULE_PLAIN) {
             p.seg0 = kSegRounds;

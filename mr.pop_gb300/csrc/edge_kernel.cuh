@@ -2400,7 +2400,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, kBroadMinBlocks)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <int A, int SPL, bool SEG>
+template <int A, int SPL, bool SEG, int STAGE>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     narrow_kernel(const __grid_constant__ EdgeParams P) {
     MRPOP_KERNEL_PROLOGUE(WarpScratch)
@@ -2409,8 +2409,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
     // visible) before reading its output
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (long long e = next_edge(P.work + 1, lane); e < P.n_edges; e = next_edge(P.work + 1, lane))
-        narrow_edge<A, SPL, SEG, A == 1 ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, g, lane, staged);
-    if (A > 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the rows kernel
+        narrow_edge<A, SPL, SEG, STAGE>(P, W, S, L, det_tab, e, dof, g, lane, staged);
+    if (STAGE == kStageEnvPairs) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the rows kernel
 }
 
 // Composite checks: the intra-arm rows, after the narrow kernel.

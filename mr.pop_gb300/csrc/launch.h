@@ -13,7 +13,8 @@ namespace mrpop {
 // kArmwise: the fused kernel with one warp per arm; timed as kFused.
 // kRows: the rows kernel that follows kNarrow for more than one arm; timed as
 // kNarrow.
-enum KernelKind { kFused = 0, kBroad = 1, kNarrow = 2, kFusedPair = 3, kArmwise = 4, kRows = 5 };
+// kNarrowAll: kNarrow and kRows in one kernel; timed as kNarrow.
+enum KernelKind { kFused = 0, kBroad = 1, kNarrow = 2, kFusedPair = 3, kArmwise = 4, kRows = 5, kNarrowAll = 6 };
 
 // Launch a validator kernel for `arms` arms (1..5).  smem_bytes: dynamic
 // shared memory (staged scene + per-warp scratch).  Returns the launch error.

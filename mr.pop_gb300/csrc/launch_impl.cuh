@@ -72,7 +72,12 @@ template <int A, int SPL>
 const void *kernel_fn(KernelKind kind, bool seg) {
     switch (kind) {
     case kBroad: return seg ? (const void *)broad_kernel<A, SPL, true> : (const void *)broad_kernel<A, SPL, false>;
-    case kNarrow: return seg ? (const void *)narrow_kernel<A, SPL, true> : (const void *)narrow_kernel<A, SPL, false>;
+    case kNarrow:
+        return seg ? (const void *)narrow_kernel<A, SPL, true, A == 1 ? kStageAll : kStageEnvPairs>
+                   : (const void *)narrow_kernel<A, SPL, false, A == 1 ? kStageAll : kStageEnvPairs>;
+    case kNarrowAll:
+        return seg ? (const void *)narrow_kernel<A, SPL, true, kStageAll>
+                   : (const void *)narrow_kernel<A, SPL, false, kStageAll>;
     case kRows:
         if constexpr (A > 1) return seg ? (const void *)rows_kernel<A, SPL, true> : (const void *)rows_kernel<A, SPL, false>;
         return nullptr;
@@ -164,7 +169,7 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
     if (need < grid) grid = need;
     if (grid < 1) grid = 1;
     void *args[] = {(void *)&p};
-    if (kind != kNarrow && kind != kRows)
+    if (kind != kNarrow && kind != kRows && kind != kNarrowAll)
         return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(32 * kWarpsPerBlock), args, smem_bytes, stream);
     // the narrow kernel follows the broad one, and the rows kernel the narrow
     // one, as a programmatic dependent: its CTAs start (and stage the scene)
