@@ -245,6 +245,14 @@ def fp32_peak(pkg, torch) -> float:
 KERNEL_NAMES = {"fused": "validate_kernel", "broad": "broad_kernel", "narrow": "narrow_kernel"}
 
 
+def kernel_runs(kt: dict, kind: str) -> float:
+    """Runs of a kind's phase.  The library times the narrow phase's second
+    kernel (rows_kernel, large composite calls) under the narrow kind, so a run
+    of that phase is one or two launches for each broad launch."""
+    launches = kt[kind][0]
+    return kt["broad"][0] if kind == "narrow" and kt["broad"][0] else launches
+
+
 def committed_profile(kernel: str, workload: str) -> dict:
     """Per-launch figures of one kernel from the committed ncu summary
     (profiles/<kernel>_<workload>.json): DRAM bytes and executed FP32 flops."""
@@ -269,7 +277,7 @@ def step_traffic(kt: dict, workload: str, algorithmic_bytes: int, steps: int) ->
         if b is None:
             return {"bytes": None, "algorithmic_bytes": algorithmic_bytes,
                     "basis": f"no committed capture of {KERNEL_NAMES[kind]} on {workload}"}
-        per[KERNEL_NAMES[kind]] = b * launches / steps
+        per[KERNEL_NAMES[kind]] = b * kernel_runs(kt, kind) / steps
     total = sum(per.values())
     return {"bytes": total, "per_kernel": per, "algorithmic_bytes": algorithmic_bytes,
             "ratio": total / algorithmic_bytes,
@@ -283,7 +291,8 @@ def roofline(kt: dict, flops: dict, peak: float, workload: str, arms: int, spl: 
     """Roofline of the kernel with the largest share of device time.
     kt: {kind: (launches, total ms)} from the library's event timing over
     `steps` steps; flops: algorithmic flops per step of each kind (a kind may
-    launch more than once per step: segment rounds); sm_mhz: the median SM
+    launch more than once per step: segment rounds; the narrow kind's figures are
+    those of its phase, narrow_kernel and rows_kernel together); sm_mhz: the median SM
     clock sampled over the timed region.
 
     The kernels are bound by instruction issue (FP32 is about a third of what
@@ -298,7 +307,7 @@ def roofline(kt: dict, flops: dict, peak: float, workload: str, arms: int, spl: 
     total_ms = sum(v[1] for v in ran.values())
     dom = max(ran, key=lambda k: ran[k][1])
     launches, ms = ran[dom]
-    launch_s = ms / launches / 1e3
+    launch_s = ms / kernel_runs(kt, dom) / 1e3
     algorithmic = flops[dom] / (ms / steps / 1e3) / 1e12
     prof = committed_profile(KERNEL_NAMES[dom], workload)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
@@ -340,7 +349,7 @@ def roofline(kt: dict, flops: dict, peak: float, workload: str, arms: int, spl: 
         out["hbm_check"] = {"achieved_gbs": bw, "peak_gbs": hbm, "frac": bw / hbm if hbm else None,
                             "basis": "ncu DRAM bytes of one launch / live launch time, against the measured copy "
                                      "bandwidth (MEASURED_PEAKS.json): HBM is not the bound"}
-    out["kernels"] = {KERNEL_NAMES[k]: {"launches": v[0], "avg_ms": v[1] / v[0], "share": v[1] / total_ms,
+    out["kernels"] = {KERNEL_NAMES[k]: {"launches": v[0], "avg_ms": v[1] / kernel_runs(kt, k), "share": v[1] / total_ms,
                                         "algorithmic_tflops": flops[k] / (v[1] / steps / 1e3) / 1e12}
                       for k, v in ran.items()}
     return out

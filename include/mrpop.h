@@ -124,9 +124,10 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots);
  * sample index of the first sample whose detailed check fired (-1 if valid).
  * Replaces one fkcc_single_buffer* call per edge (see flags above).
  * Launch form: a call of more than the fused-edge limit runs the split
- * pipeline (a broad and a narrow kernel, and for more than one arm a rows
- * kernel; for segmented rules, segment rounds of them and a fused tail); a smaller call runs as one fused launch (both
- * phases per edge in one warp, from segment 0), which saves the launches and
+ * pipeline (a broad and a narrow kernel, and for large composite calls a rows
+ * kernel; for segmented rules, segment rounds of them and a fused tail); a
+ * smaller call runs as one fused launch (both phases of an edge in one kernel,
+ * from segment 0), which saves the launches and
  * the staging that dominate small calls.  Verdicts are the same either way.
  * Segmented calls (mrpop_validate_segments) have 5/2 of the limit.
  * mrpop_set_fused_edges sets the limit for the process (0: the default, 2048
@@ -224,7 +225,8 @@ mrpop_status mrpop_fk_spheres(const mrpop_robotset *robots, int arm, const float
  * (segmented or not)), and keeps the item pointers: their buffers must outlive
  * the batch.
  * mrpop_batch_run launches, per group on `stream`, one persistent broad-phase
- * and one narrow-phase kernel; a segmented group runs them in rounds (one
+ * and one narrow-phase kernel and, for more than one arm, one rows kernel (the
+ * narrow kernel's shape); a segmented group runs them in rounds (one
  * segment of every undecided edge per round) and then one fused kernel for the
  * edges with segments left.  It allocates nothing and reads the inputs as they
  * are at execution time, so a batch can be rerun on refilled buffers.
@@ -607,7 +609,8 @@ mrpop_status mrpop_broad_flops_per_sample(const mrpop_scene *scene, const mrpop_
 #define MRPOP_KERNEL_KINDS 3
 #define MRPOP_KERNEL_FUSED 0  /* segmented rules, segments after the split rounds: both phases in one kernel */
 #define MRPOP_KERNEL_BROAD 1  /* broad phase (single-segment edges, or one segment round) */
-#define MRPOP_KERNEL_NARROW 2 /* narrow phase (single-segment edges, or one segment round) */
+#define MRPOP_KERNEL_NARROW 2 /* narrow phase (single-segment edges, or one segment round): one launch, or two in
+                                 large composite calls */
 mrpop_status mrpop_kernel_timing(int enable);
 mrpop_status mrpop_kernel_times(int64_t *launches, double *ms);
 

@@ -486,16 +486,14 @@ void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int
 // takes as long as its slowest edge, so a third kernel adds a third tail; above
 // that the larger kernel's instruction fetches cost more (its hot code grows with
 // the arm pairs and passes the SM's instruction cache).  Whole calls, one kernel
-// against two: 4 arms x 32 samples, 4134 edges 130 / 156 us, 9000 270 / 271, 22000
-// 402 / 364; 5 arms x 64, 3000 258 / 350, 6000 401 / 435, 22000 980 / 870; 2 arms x
-// 64, 24990 327 / 335, x 16, 214 / 237.  Segment rounds get emptier one by one, so their call may
-// be twice as large: shortcut, 4 arms x 32, 12000 778 / 882 us, 26000 1257 / 1221;
-// 5 arms x 64, 8000 1304 / 1441, 18000 2161 / 2070.
+// against two, us: 4 arms x 32 samples, 4134 edges 164 / 202, 9000 219 / 246, 22000
+// 404 / 363; 5 arms x 64, 3000 237 / 305, 6000 391 / 442, 22000 879 / 849; 5 arms x
+// 32, 4134 206 / 236, 6000 282 / 280; 2 arms x 64, 24990 325 / 328, x 16 221 / 236.
+// Segment rounds get emptier one by one, so their call may be twice as large:
+// shortcut, 4 arms x 32, 12000 778 / 882, 26000 1257 / 1221; 5 arms x 64, 8000
+// 1304 / 1441, 18000 2161 / 2070.
 constexpr int64_t one_narrow_edges(int A, bool rounds) { return 100000 / (A * A) * (rounds ? 2 : 1); }
 
-// ext_scratch: caller-provided device scratch for the single-segment pipeline
-// (at least split_scratch_bytes(n_edges, g, arms) bytes); nullptr = the
-// library's stream-ordered pool.
 // Calls of at most this many edges run as one fused launch (mrpop_set_fused_edges).
 constexpr int64_t kFusedEdgesDefault = 2048;
 constexpr int64_t kMaxFusedEdges = (int64_t)1 << 40;  // (beyond any call; keeps the product below in range)
@@ -512,6 +510,9 @@ constexpr int64_t fused_segment_edges(int64_t limit) { return limit < 0 ? limit 
 
 std::atomic<int64_t> g_fused_edges{kFusedEdgesDefault};
 
+// ext_scratch: caller-provided device scratch for the single-segment pipeline
+// (at least split_scratch_bytes(n_edges, g, arms) bytes); nullptr = the
+// library's stream-ordered pool.
 mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robots, const float *q0,
                            const float *q1, int64_t n_edges, int g, int rule, float range, uint32_t flags,
                            int arm, uint8_t *valid, int32_t *first_hit, int32_t *n_seg_out, double *flops,
@@ -547,8 +548,8 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     }
     // split pipeline: staged flags, masks, bounds and segment state in
     // stream-ordered scratch.  Single-segment edges: one broad and one narrow
-    // launch (and one of rows for more than one arm).  Segmented rules: segment r of every undecided edge per round
-    // (broad + narrow), kSegRounds rounds, then the fused kernel for the edges
+    // launch (and one of rows for large composite calls).  Segmented rules:
+    // segment r of every undecided edge per round (the same), kSegRounds rounds, then the fused kernel for the edges
     // that still have segments left, from segment kSegRounds on.
     void *scratch = ext_scratch;
     if (!scratch) {

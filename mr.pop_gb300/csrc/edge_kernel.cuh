@@ -2,9 +2,10 @@
 //
 // One warp owns one edge at a time; warps take edges from a per-launch work
 // counter (persistent grid).  Lane L evaluates samples k = L+1 (+32) of the
-// edge.  Single-segment edges run as two kernels (broad, then narrow, the
-// narrow kernel a programmatic dependent of the broad one); segmented rules
-// run those two per segment round and a fused kernel for the tail.
+// edge.  Single-segment edges run as a broad and a narrow kernel and, in large
+// composite calls, a rows kernel (each a programmatic dependent of the one
+// before); segmented rules run those per segment round and a fused kernel for
+// the tail; small calls run one fused kernel.
 //   broad phase  per lane: FK of every arm (FP32 FMA, __sinf/__cosf as the
 //                reference), the 11 broad-phase spheres per arm against the
 //                scene staged in shared memory (one bulk-async copy per CTA,
@@ -24,8 +25,8 @@
 //                obstacles that survive a warp-wide screen per sphere group,
 //                the flagged intra-arm rows (the forearm-hand rows skipped
 //                where a (q6, q7) table certifies them apart) and the
-//                arm-vs-arm group pairs that survive a warp-wide screen; the
-//                first hit is the lowest set bit of a warp ballot.
+//                arm-vs-arm groups of the joints the broad phase left
+//                connected; the first hit is the lowest set bit of a warp ballot.
 // Culling: every obstacle carries a bounding sphere (1 mm margin) and every
 // arm / joint group a bounding sphere computed from its own sphere set; an
 // exact test is skipped only where the bounds prove it cannot fire, so the
@@ -2320,8 +2321,8 @@ __device__ __forceinline__ void broad_edge(const EdgeParams &P, BroadScratch &W,
     __syncwarp();
 }
 
-// The detailed phase of edge e.  One arm: all of it, in one kernel.  Composite
-// checks: the obstacles and arm pairs (STAGE kStageEnvPairs, narrow_kernel),
+// The detailed phase of edge e.  One arm, and composite calls of a middle size:
+// all of it (kStageAll), in one kernel.  Larger composite calls: the obstacles and arm pairs (STAGE kStageEnvPairs, narrow_kernel),
 // then the intra-arm rows (kStageRows, rows_kernel) of the samples below the
 // first hit; between the two P.smasks[2 * e] says whether a sample has hit and
 // P.smasks[2 * e + 1] which samples are left.
