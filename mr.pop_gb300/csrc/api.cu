@@ -394,7 +394,9 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots) {
 namespace {
 
 // True for a rotation (rows orthonormal to 1e-4) and a translation within
-// 16 m (FP32 positions then err by a few micrometres).
+// 100 m (FP32 positions of one arm then err by 0.04 mm at most, half an ulp in
+// each of the chain's ten additions; the tightest fact used, the forearm-hand
+// table, leaves 0.2 mm).
 bool rigid_base(const float *m) {
     for (int r = 0; r < 3; r++) {
         for (int c = r; c < 3; c++) {
@@ -402,9 +404,31 @@ bool rigid_base(const float *m) {
             for (int i = 0; i < 3; i++) dot += (double)m[4 * r + i] * m[4 * c + i];
             if (!(std::fabs(dot - (r == c ? 1.0 : 0.0)) < 1e-4)) return false;
         }
-        if (!(std::fabs((double)m[4 * r + 3]) <= 16.0)) return false;
+        if (!(std::fabs((double)m[4 * r + 3]) <= 100.0)) return false;
     }
     return true;
+}
+
+// Metres by which bounds that hold in a joint's own frame have to grow on a base
+// that is not rigid: the frame moves two centres of a joint's spheres apart by
+// up to its stretch (radii do not follow), and FP32 positions err with their
+// size.  Twice the one bound's share, so that a test of two bounds needs it once.
+double base_slack(const float *m) {
+    if (rigid_base(m)) return 0.0;
+    double stretch2 = 0.0, at = 0.0;  // the largest row sum of M^T M bounds its largest eigenvalue
+    for (int r = 0; r < 3; r++) {
+        double sum = 0.0;
+        for (int c = 0; c < 3; c++) {
+            double dot = 0.0;
+            for (int i = 0; i < 3; i++) dot += (double)m[4 * i + r] * m[4 * i + c];
+            sum += std::fabs(dot);
+        }
+        stretch2 = std::fmax(stretch2, sum);
+        at = std::fmax(at, std::fabs((double)m[4 * r + 3]));
+    }
+    const double stretch = std::sqrt(stretch2);
+    const double slack = 2.0 * mrpop::kJointSpan * std::fmax(0.0, stretch - 1.0) + 4e-6 * (at + 2.0 * stretch);
+    return slack < 1e18 ? slack : 1e18;  // (its square stays finite; NaN too)
 }
 
 }  // namespace
@@ -450,11 +474,17 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
     p.status = scene->d_status;
     p.phase = g_phase_counters;
     p.env_test_flops = scene->env_test_flops;
-    p.row5 = scene->row5;
     A = arm >= 0 ? 1 : robots->n_arms;
     for (int a = 0; a < A; a++)
         for (int i = 0; i < 12; i++) p.base[a][i] = robots->base[arm >= 0 ? arm : a][i];
-    for (int a = 0; a < A; a++) p.rigid |= (int)rigid_base(p.base[a]) << a;
+    double slack = 0.0;
+    for (int a = 0; a < A; a++) {
+        p.rigid |= (int)rigid_base(p.base[a]) << a;
+        slack = std::fmax(slack, base_slack(p.base[a]));
+    }
+    p.slack = (float)slack;
+    p.cull = kCullMargin + p.slack;
+    p.row5 = slack == 0.0 ? scene->row5 : nullptr;
     p.fbp = broad_flops_per_sample(A, scene->env_test_flops, flags);
     smem = (size_t)scene->total_f4 * sizeof(float4) + block_scratch_bytes();
     return MRPOP_OK;

@@ -135,6 +135,8 @@ struct EdgeParams {
     int flags;       // MRPOP_CHECK_* | MRPOP_MODE_EXACT
     int single;      // 1: single-arm (fkcc_single_buffer_mr) semantics
     int rigid;       // bit a: arm a's base is a rigid transform near the origin (see kRegularRad)
+    float cull;      // margin of the broad phase's swept bounds: kCullMargin + slack
+    float slack;     // metres added to bounds of detailed spheres (0 if every base is rigid; see base_slack)
     int rule;        // MRPOP_RULE_*
     int seg0;        // segmented rules: the segment this launch checks (split kernels) or starts at (fused)
     float range;
@@ -154,7 +156,7 @@ struct EdgeParams {
     int32_t *snseg;             // segmented rules: per-edge segment count (-1: too many), from segment 0
     int32_t *sdone;             // segmented rules: per-edge verdict written
     unsigned long long *work;   // split kernels: next-edge counters {broad, narrow, rows}, zero before each launch
-    const uint32_t *row5;       // forearm-hand rows table (kRow5N6 x kRow5N7 bits), or nullptr
+    const uint32_t *row5;       // forearm-hand rows table (kRow5N6 x kRow5N7 bits), or nullptr (a base is not rigid)
     float base[kMaxArms][12];   // row-major 3x4 per arm of this check
 };
 
@@ -373,10 +375,11 @@ constexpr float kRegularRad = 64.0f;
 // The approx spheres s of one arm for this lane's sample go to column `lane` of
 // dst, and a bound of every sphere over the warp's 32 samples to swept: the
 // centre of the box around its 32 centres, radius = half the box diagonal
-// (+0.4 %) + sphere radius + cull margin.  If the sphere touches something at
-// any of the samples, its swept bound touches it too (the margin covers FP
-// rounding).
-__device__ __forceinline__ void store_swept(const ArmSpheres &s, float (*dst)[3][32], int lane, float4 *swept) {
+// (+0.4 %) + sphere radius + cull (EdgeParams::cull).  If the sphere touches
+// something at any of the samples, its swept bound touches it too (the margin
+// covers FP rounding).
+__device__ __forceinline__ void store_swept(const ArmSpheres &s, float (*dst)[3][32], int lane, float4 *swept,
+                                            float cull) {
 #pragma unroll
     for (int i = 0; i < kNumApprox; i++) {
         dst[i][0][lane] = s.x[i];
@@ -414,7 +417,7 @@ __device__ __forceinline__ void store_swept(const ArmSpheres &s, float (*dst)[3]
         const float az = own ? lz : s.z[0], bz = own ? hz : s.z[0];
         const float dx = bx - ax, dy = by - ay, dz = bz - az;
         swept[i] = make_float4(0.5f * (ax + bx), 0.5f * (ay + by), 0.5f * (az + bz),
-                               0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + c_approx[i].w + kCullMargin);
+                               0.5f * sqrtf(dx * dx + dy * dy + dz * dz) * 1.004f + c_approx[i].w + cull);
     }
     __syncwarp();
 }
@@ -588,6 +591,20 @@ constexpr bool approx_cover_detailed() {
 }
 static_assert(kCullMargin >= 1e-3f && approx_cover_detailed(), "approx spheres cover the detailed ones");
 
+// Largest distance between two sphere centres of one joint, approx or detailed.
+constexpr double kJointSpan = 0.25;
+constexpr bool joint_span_holds() {
+    auto at = [](int i) { return i < kNumDet ? kDet[i] : kApprox[i - kNumDet]; };
+    auto joint = [](int i) { return i < kNumDet ? det_joint(i) : approx_joint(i - kNumDet); };
+    for (int i = 0; i < kNumDet + kNumApprox; i++)
+        for (int k = 0; k < i; k++) {
+            const double x = (double)at(i).x - at(k).x, y = (double)at(i).y - at(k).y, z = (double)at(i).z - at(k).z;
+            if (joint(i) == joint(k) && x * x + y * y + z * z > kJointSpan * kJointSpan) return false;
+        }
+    return true;
+}
+static_assert(joint_span_holds(), "span of a joint's spheres");
+
 // Broad-phase intra-arm rows (panda_multi_geometry.cuh:133-139) as 21 pairs.
 static __constant__ uint8_t c_intra_pairs[21][2] = {
     {0, 5}, {0, 6}, {0, 7}, {0, 8}, {0, 9}, {0, 10}, {1, 5}, {1, 6}, {1, 7}, {1, 8}, {1, 9},
@@ -658,7 +675,7 @@ __device__ __forceinline__ void broad_sample(const EdgeParams &P, const EdgeScra
             ArmSpheres s;
             fk_approx_arm(P.base[x], q, s);
             if (A == 1 || x == b) {
-                store_swept(s, cur, lane, sw);
+                store_swept(s, cur, lane, sw, P.cull);
                 MRPOP_PHASE(P, 0);
                 if (do_env) envw |= (Flags<A>)env_joints<A == 1>(S, L, P.sc, cur, lane, sw) << (8 * b);
                 MRPOP_PHASE(P, 1);
@@ -1083,9 +1100,9 @@ __device__ __forceinline__ void lane_env(int j, const EdgeParams &P, const Xf &T
         // the hand's spheres in its three parts
 #pragma unroll 1
         for (int g = jgrp_first(j); g < set_end<true>(j); g++) {
-            if (env_group_warp(S, L, P.sc, T, set_first(g), set_spheres<true>(g), set_bound<true>(g),
-                               c.em >> j & 1u))
-                c.set_hit();
+            float4 gl = set_bound<true>(g);
+            gl.w += P.slack;
+            if (env_group_warp(S, L, P.sc, T, set_first(g), set_spheres<true>(g), gl, c.em >> j & 1u)) c.set_hit();
             const uint32_t hb = __ballot_sync(kFull, c.hit);
             if (hb & lanes_upto(threadIdx.x & 31)) c.em = c.rm = 0;
             if (!__any_sync(kFull, c.em >> j & 1u)) break;
@@ -1110,7 +1127,8 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
     for (int g = jgrp_first(j); g < jgrp_first(j + 1); g++) {
         uint32_t rows = c.rm & c_rows.cover[grp_first(g)];
         if (!rows) continue;
-        const float4 gl = c_bounds.grp[g];
+        float4 gl = c_bounds.grp[g];
+        gl.w += P.slack;
         const float3 gc = place_reg(T, gl);
         uint32_t nr = 0;
         while (rows) {
@@ -1128,7 +1146,8 @@ __device__ __forceinline__ void lane_rows(int j, const EdgeParams &P, const Xf &
             // more than they save)
 #pragma unroll 1
             for (int s = 0; s < kHandParts; s++) {
-                const float4 sl = c_bounds.hsub[s];
+                float4 sl = c_bounds.hsub[s];
+                sl.w += P.slack;
                 const float3 sc = place_reg(T, sl);
                 uint32_t ns = 0;
                 for (uint32_t m = nr; m; m &= m - 1) {
@@ -1393,11 +1412,12 @@ __device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf
         if (grp_first(g + 1) <= from) continue;
         const float4 gl = c_bounds.grp[g];
         const float3 gc = place_reg(T, gl);
+        const float gr = gl.w + P.slack;  // (covers both sets)
         uint32_t near = 0;
         for (uint32_t m = gb; m; m &= m - 1) {
             const int t = __ffs(m) - 1;
             if (near3(gc.x, gc.y, gc.z,
-                      make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], set_bound<PARTS>(t).w), gl.w))
+                      make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], set_bound<PARTS>(t).w), gr))
                 near |= 1u << t;
         }
         if (!near) continue;
@@ -1405,11 +1425,12 @@ __device__ __forceinline__ void stash_joint(int j, const EdgeParams &P, const Xf
         for (int at = max(grp_first(g), from); at < grp_first(g + 1); at++) {
             const float4 sd = c_det[at];
             const float3 p = place_reg(T, sd);
+            const float sr = sd.w + P.slack;
             uint32_t nm = 0;
             for (uint32_t m = near; m; m &= m - 1) {
                 const int t = __ffs(m) - 1;
                 if (near3(p.x, p.y, p.z,
-                          make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], set_bound<PARTS>(t).w), sd.w))
+                          make_float4(X.gc[t][0][lane], X.gc[t][1][lane], X.gc[t][2][lane], set_bound<PARTS>(t).w), sr))
                     nm |= 1u << t;
             }
             if (!nm) continue;
@@ -2093,7 +2114,7 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
             sample_q(W, P.rule, seg, P.single ? 0 : arm, k <= g ? k : g, q);
             ArmSpheres as;
             fk_approx_arm(P.base[arm], q, as);
-            store_swept(as, sp, lane, sw);
+            store_swept(as, sp, lane, sw, P.cull);
             const bool reg = regular_pose(q);
             const bool regular = __all_sync(kFull, reg) && (P.rigid >> arm & 1);
             uint32_t em = 0, im = 0;
