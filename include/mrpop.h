@@ -129,9 +129,10 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots);
  * smaller call runs as one fused launch (both phases of an edge in one kernel,
  * from segment 0), which saves the launches and
  * the staging that dominate small calls.  Verdicts are the same either way.
- * Segmented calls (mrpop_validate_segments) have 5/2 of the limit.
- * mrpop_set_fused_edges sets the limit for the process (0: the default, 2048
- * edges; -1: every call split) and returns the previous one.
+ * mrpop_set_fused_edges sets the limit of every call of the process (-1: every
+ * call split) and returns the previous one.  0, or 2048, is the default: 2048
+ * edges, and 5120 for segmented calls (mrpop_validate_segments), whose split
+ * form has more launches.
  */
 int64_t mrpop_set_fused_edges(int64_t max_edges);
 mrpop_status mrpop_validate_edges(const mrpop_scene *scene, const mrpop_robotset *robots,

@@ -526,17 +526,20 @@ constexpr int64_t one_narrow_edges(int A, bool rounds) { return 100000 / (A * A)
 
 // Calls of at most this many edges run as one fused launch (mrpop_set_fused_edges).
 constexpr int64_t kFusedEdgesDefault = 2048;
-constexpr int64_t kMaxFusedEdges = (int64_t)1 << 40;  // (beyond any call; keeps the product below in range)
 
-// The limit of segmented calls: the split pipeline runs 4 rounds of two or
+// The default limit of segmented calls: the split pipeline runs 4 rounds of two or
 // three launches and a fused tail, each as long as its slowest edge, so one
 // fused launch is the faster form up to about two edges per resident warp.
 // Measured, split against fused in us: 3 arms x 24 B-spline 2800 edges 609 /
 // 250, 4096 569 / 422, 8000 641 / 750; 5 arms x 64 shortcut 4096 edges 1058 /
 // 773, 8000 1251 / 1480; 4 arms x 32 connect 4096 576 / 381, 8000 737 / 763.
 // (Single-segment calls, 4 arms x 32: 2000 edges 171 / 207, 2800 224 / 191,
-// 4096 240 / 322; 5 arms x 64: 2000 327 / 246, 4096 395 / 463.)
-constexpr int64_t fused_segment_edges(int64_t limit) { return limit < 0 ? limit : limit * 5 / 2; }
+// 4096 240 / 322; 5 arms x 64: 2000 327 / 246, 4096 395 / 463.)  A limit set by
+// the caller holds for every call.
+constexpr int64_t kFusedSegmentEdges = 5120;
+constexpr int64_t fused_limit(int64_t limit, int rule) {
+    return limit == kFusedEdgesDefault && rule != MRPOP_RULE_PLAIN ? kFusedSegmentEdges : limit;
+}
 
 std::atomic<int64_t> g_fused_edges{kFusedEdgesDefault};
 
@@ -567,8 +570,7 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     // more arms one warp per arm, else above 32 samples per segment two warps
     // per edge (one per 32-sample slot), unless the flop tally is wanted
     cudaError_t err;
-    const int64_t limit = g_fused_edges.load(std::memory_order_relaxed);
-    if (n_edges <= (rule == MRPOP_RULE_PLAIN || limit > kMaxFusedEdges ? limit : fused_segment_edges(limit))) {
+    if (n_edges <= fused_limit(g_fused_edges.load(std::memory_order_relaxed), rule)) {
         p.seg0 = 0;
         err = timed_launch(A, flops ? kFused : A >= 3 ? kArmwise : g > 32 ? kFusedPair : kFused, p, smem, stream);
         if (tmp_valid) cudaFreeAsync(tmp_valid, stream);

@@ -1,0 +1,52 @@
+"""The largest calls that run as one fused launch: a limit set by
+mrpop_set_fused_edges holds for calls of every rule, the default one lets
+segmented calls be larger.  The launch form shows in the kernel times (a split
+call launches broad kernels)."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _is_fused(cuda, pkg, arms, n, rule):
+    import numpy as np
+    W = pkg.workloads
+    bases = W.bases_facing_centre(arms, 0.71)
+    q0, q1 = W.random_edges(np.random.default_rng(n), n, arms, 2.0)
+    scene, robots = pkg.Scene(W.scene_config2(3)), pkg.RobotSet(arms, bases)
+    a, b = cuda.from_numpy(q0).cuda(), cuda.from_numpy(q1).cuda()
+    cuda.cuda.synchronize()
+    pkg.kernel_timing(True)
+    try:
+        pkg.kernel_times()
+        pkg.validate(scene, robots, a, b, 4, rule=rule, range_=1.0 if rule else 0.0)
+        cuda.cuda.synchronize()
+        t = pkg.kernel_times()
+    finally:
+        pkg.kernel_timing(False)
+    assert t["broad"][0] or t["fused"][0]
+    return t["broad"][0] == 0
+
+
+@pytest.mark.parametrize("rule", [0, 1, 2, 3])
+@pytest.mark.parametrize("limit", [1, 700, 2049])
+def test_a_limit_set_holds_for_every_rule(cuda, pkg, limit, rule):
+    lib = pkg.library()
+    prev = lib.mrpop_set_fused_edges(limit)
+    try:
+        assert _is_fused(cuda, pkg, 2, limit, rule)
+        assert not _is_fused(cuda, pkg, 2, limit + 1, rule)
+        assert not _is_fused(cuda, pkg, 2, 2 * limit, rule)
+    finally:
+        assert lib.mrpop_set_fused_edges(prev) == limit
+
+
+@pytest.mark.parametrize("setting", [0, 2048])
+def test_default_limits(cuda, pkg, setting):
+    lib = pkg.library()
+    prev = lib.mrpop_set_fused_edges(setting)
+    try:
+        for rule, limit in ((0, 2048), (1, 5120), (2, 5120), (3, 5120)):
+            assert _is_fused(cuda, pkg, 2, limit, rule)
+            assert not _is_fused(cuda, pkg, 2, limit + 1, rule)
+    finally:
+        assert lib.mrpop_set_fused_edges(prev) == 2048
