@@ -511,34 +511,25 @@ void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int
     p.sdone = p.snseg + n_edges;
 }
 
-// Largest calls whose narrow phase is one kernel (kNarrowAll) instead of
-// kNarrow and kRows.  Up to some edges per resident warp each kernel of a round
-// takes as long as its slowest edge, so a third kernel adds a third tail; above
-// that the larger kernel's instruction fetches cost more (its hot code grows with
-// the arm pairs and passes the SM's instruction cache).  Whole calls, one kernel
-// against two, us: 4 arms x 32 samples, 4134 edges 164 / 202, 9000 219 / 246, 22000
-// 404 / 363; 5 arms x 64, 3000 237 / 305, 6000 391 / 442, 22000 879 / 849; 5 arms x
-// 32, 4134 206 / 236, 6000 282 / 280; 2 arms x 64, 24990 325 / 328, x 16 221 / 236.
-// Segment rounds get emptier one by one, so their call may be twice as large:
-// shortcut, 4 arms x 32, 12000 778 / 882, 26000 1257 / 1221; 5 arms x 64, 8000
-// 1304 / 1441, 18000 2161 / 2070.
-constexpr int64_t one_narrow_edges(int A, bool rounds) { return 100000 / (A * A) * (rounds ? 2 : 1); }
-
 // Calls of at most this many edges run as one fused launch (mrpop_set_fused_edges).
 constexpr int64_t kFusedEdgesDefault = 2048;
 
 // The default limit of segmented calls: the split pipeline runs 4 rounds of two or
 // three launches and a fused tail, each as long as its slowest edge, so one
-// fused launch is the faster form up to about two edges per resident warp.
-// Measured, split against fused in us: 3 arms x 24 B-spline 2800 edges 609 /
-// 250, 4096 569 / 422, 8000 641 / 750; 5 arms x 64 shortcut 4096 edges 1058 /
-// 773, 8000 1251 / 1480; 4 arms x 32 connect 4096 576 / 381, 8000 737 / 763.
+// fused launch is the faster form up to one to two edges per resident warp, the
+// fewer the more arms (an edge's warp walks them all).  Whole calls, split against
+// fused in us: 3 arms x 24 B-spline 2800 edges 609 / 250, 4096 569 / 422, 8000
+// 641 / 750; 4 arms x 32 connect, mixed cell, 3500 441 / 393, 4100 465 / 468, 5100
+// 480 / 557, bin table 560 / 475, 546 / 408, 598 / 501; 5 arms x 32 connect, mixed
+// cell, 2600 574 / 452, 3072 619 / 568, 4100 666 / 747, shelf 385 / 336, 434 /
+// 448, 450 / 549; 5 arms x 64, mixed cell, 3072 917 / 676, 5100 1090 / 1046,
+// shelf 571 / 526, 682 / 784.
 // (Single-segment calls, 4 arms x 32: 2000 edges 171 / 207, 2800 224 / 191,
 // 4096 240 / 322; 5 arms x 64: 2000 327 / 246, 4096 395 / 463.)  A limit set by
 // the caller holds for every call.
-constexpr int64_t kFusedSegmentEdges = 5120;
-constexpr int64_t fused_limit(int64_t limit, int rule) {
-    return limit == kFusedEdgesDefault && rule != MRPOP_RULE_PLAIN ? kFusedSegmentEdges : limit;
+constexpr int64_t fused_segment_edges(int A) { return A <= 3 ? 5120 : A == 4 ? 4096 : 3072; }
+constexpr int64_t fused_limit(int64_t limit, int rule, int A) {
+    return limit == kFusedEdgesDefault && rule != MRPOP_RULE_PLAIN ? fused_segment_edges(A) : limit;
 }
 
 std::atomic<int64_t> g_fused_edges{kFusedEdgesDefault};
@@ -570,7 +561,7 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     // more arms one warp per arm, else above 32 samples per segment two warps
     // per edge (one per 32-sample slot), unless the flop tally is wanted
     cudaError_t err;
-    if (n_edges <= fused_limit(g_fused_edges.load(std::memory_order_relaxed), rule)) {
+    if (n_edges <= fused_limit(g_fused_edges.load(std::memory_order_relaxed), rule, A)) {
         p.seg0 = 0;
         err = timed_launch(A, flops ? kFused : A >= 3 ? kArmwise : g > 32 ? kFusedPair : kFused, p, smem, stream);
         if (tmp_valid) cudaFreeAsync(tmp_valid, stream);

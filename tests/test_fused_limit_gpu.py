@@ -50,3 +50,15 @@ def test_default_limits(cuda, pkg, setting):
             assert not _is_fused(cuda, pkg, 2, limit + 1, rule)
     finally:
         assert lib.mrpop_set_fused_edges(prev) == 2048
+
+
+@pytest.mark.parametrize("arms,limit", [(1, 5120), (3, 5120), (4, 4096), (5, 3072)])
+def test_default_limit_of_segmented_calls_by_arms(cuda, pkg, arms, limit):
+    lib = pkg.library()
+    prev = lib.mrpop_set_fused_edges(0)
+    try:
+        for rule in (1, 2, 3):
+            assert _is_fused(cuda, pkg, arms, limit, rule)
+            assert not _is_fused(cuda, pkg, arms, limit + 1, rule)
+    finally:
+        lib.mrpop_set_fused_edges(prev)
