@@ -78,6 +78,24 @@ constexpr size_t split_scratch_bytes(int64_t n_edges, int g, [[maybe_unused]] in
 }
 void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int A);
 
+// Largest calls whose narrow phase is one kernel (kNarrowAll) instead of
+// kNarrow and kRows.  Up to some edges per resident warp each kernel of a round
+// takes as long as its slowest edge, so a third kernel adds a third tail; above
+// that the larger kernel's instruction fetches cost more (its hot code grows with
+// the arm pairs and passes the SM's instruction cache).  Whole calls, one kernel
+// against two, us: 4 arms x 32 samples, 4134 edges 164 / 202, 9000 219 / 246, 22000
+// 404 / 363; 5 arms x 64, 3000 237 / 305, 6000 391 / 442, 22000 879 / 849; 5 arms x
+// 32, 4134 206 / 236, 6000 282 / 280; 2 arms x 64, 24990 325 / 328, x 16 221 / 236.
+// Segment rounds get emptier one by one, so their call may be twice as large:
+// shortcut, 4 arms x 32, 12000 778 / 882, 26000 1257 / 1221; 5 arms x 64, 8000
+// 1304 / 1441, 18000 2161 / 2070.
+// Service waves, whose kernels read the endpoints from host memory (the rows kernel
+// once more), device time of a wave: 2 arms x 64 connect, 4500 edges 529 / 697,
+// 20000 975 / 1059; 4 arms x 64, connect 4500 738 / 941, shortcut 7200 in 12
+// steps 527 / 613; above the limit, plain x 64, 20000 edges, 4 arms 715 / 662, 5
+// arms 783 / 701.
+constexpr int64_t one_narrow_edges(int A, bool rounds) { return 100000 / (A * A) * (rounds ? 2 : 1); }
+
 // The dRRT / AO-x planner (drrt.cu) with any validator (validate_many, if
 // not null, takes the groups of checks of the roadmap rounds in one call);
 // device_nn: tree searches as a kernel on the current device, else on the host.
