@@ -2490,6 +2490,8 @@ constexpr int kBatchBroad = 0, kBatchNarrow = 1, kBatchFused = 2;
 constexpr int kBatchArmwise = 3;
 // The rows kernel of composite groups, after kBatchNarrow.
 constexpr int kBatchRows = 4;
+// kBatchNarrow and kBatchRows in one kernel (service waves).
+constexpr int kBatchNarrowAll = 5;
 
 // One bulk copy of `bytes` from global to shared memory, completed on `bar`
 // in phase `parity`; bounded wait.  Every thread of the CTA calls it after a
@@ -2571,8 +2573,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MODE == kBatchBroad ? kBr
             if ((int)k >= ch.z) break;
             const long long e = (long long)ch.y + k;
             if constexpr (MODE == kBatchBroad) broad_edge<A, SPL, SEG>(P, W, S, L, e, dof, P.g, lane, staged);
-            else if constexpr (MODE == kBatchNarrow)
-                narrow_edge<A, SPL, SEG, A == 1 ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
+            else if constexpr (MODE == kBatchNarrow || MODE == kBatchNarrowAll)
+                narrow_edge<A, SPL, SEG, A == 1 || MODE == kBatchNarrowAll ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
             else if constexpr (MODE == kBatchRows)
                 narrow_edge<A, SPL, SEG, kStageRows>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
             else fused_edge<A, SPL>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);

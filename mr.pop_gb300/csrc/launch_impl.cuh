@@ -93,6 +93,12 @@ const void *batch_fn(int mode, bool seg) {
         if constexpr (A >= 3) return (const void *)batch_armwise_kernel<A, SPL>;
         return nullptr;
     }
+    if (mode == kBatchNarrowAll) {
+        if constexpr (A > 1)
+            return seg ? (const void *)batch_kernel<A, SPL, kBatchNarrowAll, true>
+                       : (const void *)batch_kernel<A, SPL, kBatchNarrowAll, false>;
+        return nullptr;
+    }
     if (mode == kBatchRows) {
         if constexpr (A > 1)
             return seg ? (const void *)batch_kernel<A, SPL, kBatchRows, true>

@@ -293,13 +293,14 @@ cudaError_t launch_wave(mrpop_server *s, mrpop_server::Slot &slot) {
             continue;
         }
         const int rounds = seg ? mrpop::kSegRounds : 1;
+        const bool one = arms > 1 && r.edges <= mrpop::one_narrow_edges(arms, seg);
         for (int rd = 0; rd < rounds && err == cudaSuccess; rd++) {
             err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchBroad, rd, items, chunks, r.nc, work + 3 * rd,
                              slot.stream);
             if (err == cudaSuccess)
-                err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchNarrow, rd, items, chunks, r.nc,
-                                 work + 3 * rd + 1, slot.stream);
-            if (err == cudaSuccess && arms > 1)
+                err = launch_one(s, arms, seg, spl, r.smem, one ? mrpop::kBatchNarrowAll : mrpop::kBatchNarrow, rd, items,
+                                 chunks, r.nc, work + 3 * rd + 1, slot.stream);
+            if (err == cudaSuccess && arms > 1 && !one)
                 err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchRows, rd, items, chunks, r.nc,
                                  work + 3 * rd + 2, slot.stream);
         }
