@@ -15,7 +15,10 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
+# device code uncompressed: nvcc compresses some of the units and not others, and a
+# compressed one takes ten times as long to load (an arm count's first call 1.3 ->
+# 10 to 13 ms)
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--no-compress", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 SOURCES = ["api.cu", "batch.cu", "server.cu", "planner.cu", "drrt.cu", "peak_probe.cu", "no_alloc.cu"] + \
     [f"validate_a{a}.cu" for a in range(1, 6)]
 # the planners' host arithmetic is written with explicit fmaf where the
