@@ -32,6 +32,7 @@
 // exact test is skipped only where the bounds prove it cannot fire, so the
 // set of tests that can fire -- and therefore every verdict -- is unchanged.
 #pragma once
+#include <cstddef>
 #include <type_traits>
 
 #include "panda_model.cuh"
@@ -196,6 +197,11 @@ struct WarpScratchT : EdgeScratch {
     };
 };
 using WarpScratch = WarpScratchT<kCrossStash>;
+// store_swept reads the sphere columns 16 bytes at a time, and the scratch of the
+// warps follows the scene (16-byte records)
+static_assert(offsetof(BroadPart, cur) % 16 == 0 && alignof(BroadPart) >= 16 && sizeof(BroadScratch) % 16 == 0 &&
+                  sizeof(WarpScratch) % 16 == 0,
+              "sphere columns on 16 bytes");
 using ArmScratch = WarpScratchT<kArmCrossStash>;  // arm-per-warp kernels
 
 // Flag words of one sample: 8 bits (joints) per arm.
@@ -610,6 +616,24 @@ static __constant__ uint8_t c_intra_pairs[21][2] = {
     {0, 5}, {0, 6}, {0, 7}, {0, 8}, {0, 9}, {0, 10}, {1, 5}, {1, 6}, {1, 7}, {1, 8}, {1, 9},
     {1, 10}, {2, 5}, {2, 7}, {2, 8}, {2, 9}, {2, 10}, {5, 7}, {5, 8}, {5, 9}, {5, 10}};
 
+constexpr double const_sqrt(double v) {
+    double x = v > 1.0 ? v : 1.0;
+    for (int i = 0; i < 64; i++) x = 0.5 * (x + v / x);
+    return x;
+}
+constexpr double const_hypot(double x, double y) { return const_sqrt(x * x + y * y); }
+
+// Approx spheres 5 and 8 overlap in every pose.  Joint 6's axis is the y axis of
+// joint 5's frame, through its origin; sphere 8 is at F_7 Rz(q7) x from joint 6.
+constexpr bool spheres_5_8_overlap() {
+    const SphereDef &a = kApprox[5], &b = kApprox[8];
+    const double out = const_hypot(kJointK.v[5][1] + const_hypot(b.x, b.y), b.z);  // from joint 6's axis, at most
+    const double along = (a.y > 0 ? a.y : -a.y) + const_hypot(b.x, b.y);           // along it
+    const double far = const_hypot(out + const_hypot(a.x, a.z), along);
+    return kJointK.v[4][1] == 0.f && kJointK.v[4][2] == 0.f && far < (double)a.r + b.r - 2e-3;
+}
+static_assert(spheres_5_8_overlap(), "pair (5, 8) overlaps in every pose");
+
 // Intra-arm pairs of one arm (panda_four.cuh:140-176): the 21 approx sphere
 // pairs, one per lane, screened by the swept bounds sw of the warp's samples;
 // exact per-sample tests for the survivors.  Returns the lane's flag bits (by
@@ -876,11 +900,6 @@ struct SetBounds {
     float4 grp[kNumGroups];
     float4 hsub[kHandParts];
 };
-constexpr double const_sqrt(double v) {
-    double x = v > 1.0 ? v : 1.0;
-    for (int i = 0; i < 64; i++) x = 0.5 * (x + v / x);
-    return x;
-}
 // the spheres first + (bits of m)
 constexpr float4 set_ball(int first, uint32_t m) {
     double lo[3] = {1e9, 1e9, 1e9}, hi[3] = {-1e9, -1e9, -1e9}, r = 0.0;
@@ -1230,6 +1249,45 @@ __host__ __device__ __forceinline__ constexpr float row_reach(int t, int j) {
         {0.981f, 0.664f, 0.581f, 0.188f, 0.188f, 0.002f}}; // 10
     return kReach[t][j - 2];
 }
+// The table against the model's numbers, by the argument above.
+constexpr bool row_reach_holds() {
+    constexpr int kJoint[6] = {5, 5, 5, 6, 7, 7};
+    const double fold = const_hypot(kJointK.v[3][1], kJointK.v[3][2]);  // joint 6's origin in frame 4
+    for (int t = 0; t < 6; t++) {
+        const float4 c = set_ball(grp_first(5 + t), (1u << (grp_first(6 + t) - grp_first(5 + t))) - 1u);
+        const double rho = const_hypot(c.x, c.y), z = c.z > 0 ? c.z : -c.z;
+        // from joint 6's origin, at most
+        const double wrist = kJoint[t] == 7 ? const_hypot(kJointK.v[5][1] + rho, z) : const_hypot(rho, z);
+        double need[6] = {};  // joints 2..7
+        if (kJoint[t] == 7) need[5] = rho;
+        if (kJoint[t] >= 6) need[4] = kJoint[t] == 6 ? rho : wrist;
+        need[3] = kJoint[t] == 5 ? rho : wrist;
+        need[2] = kJoint[t] == 5 ? const_hypot(kJointK.v[3][1], kJointK.v[3][2] + c.z) + rho : fold + wrist;
+        need[1] = need[2] + kJointK.v[2][1];
+        need[0] = need[1] - kJointK.v[1][2];
+        for (int j = 2; j <= 7; j++)
+            if (row_reach(t, j) < need[j - 2] || (j <= kJoint[t] && row_reach(t, j) == 0.0f)) return false;
+    }
+    return kJointK.v[0][1] == 0.f && kJointK.v[0][2] == 0.f && kJointK.v[1][1] == 0.f && kJointK.v[2][2] == 0.f &&
+           kJointK.v[4][1] == 0.f && kJointK.v[4][2] == 0.f && kJointK.v[5][2] == 0.f;
+}
+static_assert(row_reach_holds(), "reach of the rows' targets");
+
+// The rows as screen_rows reads them: radii of their first spheres, and targets
+// that are the sub-groups 5..10, 5..7 or 9..10.
+constexpr bool low_rows_as_screened() {
+    if (kDet[0].r > 0.08f || kDet[0].x != 0.f || kDet[0].y != 0.f) return false;
+    for (int r = 1; r <= 16; r++)
+        if (kDet[det_row_first(r)].r > 0.06f) return false;
+    for (int r = 0; r <= 16; r++) {
+        const int lo = r <= 4 ? 5 : r <= 12 && r % 2 == 1 ? 5 : 9, hi = lo == 5 && r > 4 ? 7 : 10;
+        if (det_row_lo(r) < grp_first(lo) || det_row_hi(r) >= grp_first(hi + 1)) return false;
+    }
+    for (int r = 5; r <= 12; r++)
+        if (det_row_first(r) != 5 + (r - 5) / 2) return false;
+    return det_joint(4) == 1 && det_joint(8) == 2 && det_joint(12) == 3 && det_joint(16) == 4;
+}
+static_assert(low_rows_as_screened(), "rows of the screen");
 
 // Target centre p through joint J: F_J Rz(q) p (see joint_step for F_J).
 template <int J>

@@ -215,15 +215,19 @@ __device__ __forceinline__ void joint_step(Xf &T, float q) {
 //   n3 = t3 + (t0*tx + t1*ty)
 // where a zero translation term contributes an exact signed zero, exactly as
 // the reference's zero products do.  {A, tx, ty} per joint 2..7:
-static __constant__ float c_joint_k[6][3] = {{-1.f, 0.f, 0.f},      {1.f, 0.f, -0.316f}, {1.f, 0.0825f, 0.f},
-                                             {-1.f, -0.0825f, 0.384f}, {1.f, 0.f, 0.f},     {1.f, 0.088f, 0.f}};
+struct JointK {
+    float v[6][3];
+};
+constexpr JointK kJointK = {{{-1.f, 0.f, 0.f},      {1.f, 0.f, -0.316f}, {1.f, 0.0825f, 0.f},
+                             {-1.f, -0.0825f, 0.384f}, {1.f, 0.f, 0.f},     {1.f, 0.088f, 0.f}}};
+static __constant__ JointK c_joint_k = kJointK;
 
 __device__ __forceinline__ void joint_step_rt(Xf &T, float q, int j) {
     if (j == 1) {
         joint_step<1>(T, q);
         return;
     }
-    const float A = c_joint_k[j - 2][0], tx = c_joint_k[j - 2][1], ty = c_joint_k[j - 2][2];
+    const float A = c_joint_k.v[j - 2][0], tx = c_joint_k.v[j - 2][1], ty = c_joint_k.v[j - 2][2];
     const float c = __cosf(q);
     const float s = __sinf(q);
 #pragma unroll
