@@ -2287,12 +2287,16 @@ __device__ __forceinline__ void armwise_edge(const EdgeParams &P, unsigned char 
     }
 }
 
-// CTAs of the arm-per-warp kernels that fit an SM beside a 51-box scene (their
-// scratch is 11.8 KB per warp).  Given as a launch bound because ptxas, left to
-// choose, cuts 5 arms at 64 samples to 72 registers and spills.
+// CTAs of the arm-per-warp kernels that fit an SM (228 KB) by their warps' scratch,
+// 3 KB of static shared memory and the 1 KB that the system takes of each, beside
+// a scene of some boxes.  Given as a launch bound because ptxas, left to choose,
+// cuts 5 arms at 64 samples to 72 registers and spills.
 __host__ __device__ constexpr int armwise_min_blocks(int A, int G = 1) {
-    return G > 1 ? (A >= 4 ? 2 : 3) : A >= 5 ? 3 : A == 4 ? 4 : 5;
+    return (int)(228 * 1024 / (A * G * sizeof(ArmScratch) + 4096));
 }
+static_assert(armwise_min_blocks(3) == 5 && armwise_min_blocks(4) == 4 && armwise_min_blocks(5) == 3 &&
+                  armwise_min_blocks(3, 2) == 3 && armwise_min_blocks(4, 2) == 2 && armwise_min_blocks(5, 2) == 1,
+              "CTAs per SM");
 
 template <int A, int SPL, int G>
 __global__ void __launch_bounds__(32 * A * G, armwise_min_blocks(A, G))

@@ -130,9 +130,8 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
             // would double the call's time): then the pair or one-warp kernel.
             // Two warps per arm against one, 64 samples: 4 arms, 300 connect edges
             // 113 -> 99 us, 64 shortcut edges 93 -> 66; 3 arms, 300 connect edges
-            // 94 -> 76; 5 arms, 64 shortcut edges 143 -> 121, but 300 connect edges
-            // 151 -> 164 (two 10-warp CTAs per SM at 96 registers), so 5 arms take
-            // them only up to one CTA per SM
+            // 94 -> 76; 5 arms (one 10-warp CTA fills an SM's shared memory), 64
+            // shortcut edges 143 -> 121
             const size_t scene = smem_bytes - (size_t)kWarpsPerBlock * sizeof(WarpScratch);
             int dev = 0, sms = 0;
             cudaGetDevice(&dev);
@@ -147,7 +146,6 @@ cudaError_t launch_validate_impl(KernelKind kind, const EdgeParams &p, size_t sm
                 int per_sm = 0;
                 const cudaError_t err = prepare_kernel(fn, arm_smem, &per_sm, 32 * warps);
                 if (err != cudaSuccess) return err;
-                if (per_arm == 2 && A == 5) per_sm = 1;  // (see above)
                 if (p.n_edges <= (long long)sms * (per_sm > 0 ? per_sm : 1)) {
                     void *args[] = {(void *)&p};
                     return cudaLaunchKernel(fn, dim3((unsigned)(p.n_edges > 0 ? p.n_edges : 1)), dim3(32 * warps), args,
