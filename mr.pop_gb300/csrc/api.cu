@@ -428,7 +428,7 @@ double base_slack(const float *m) {
     }
     const double stretch = std::sqrt(stretch2);
     const double slack = 2.0 * mrpop::kJointSpan * std::fmax(0.0, stretch - 1.0) + 4e-6 * (at + 2.0 * stretch);
-    return slack < 1e18 ? slack : 1e18;  // (its square stays finite; NaN too)
+    return slack < 1e18 ? slack : 1e18;  // (its square stays finite)
 }
 
 }  // namespace
@@ -496,8 +496,7 @@ mrpop_status make_params(const mrpop_scene *scene, const mrpop_robotset *robots,
 // of their slice (which keeps its 64-bit size).
 int robotset_arms(const mrpop_robotset *robots) { return robots ? robots->n_arms : 0; }
 
-void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int A) {
-    (void)A;
+void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g) {
     const int spl = g > 32 ? 2 : 1;
     const size_t flag_bytes = (size_t)n_edges * 32 * spl * 2 * sizeof(uint64_t);
     const size_t mask_bytes = (size_t)n_edges * 2 * sizeof(uint64_t);
@@ -535,7 +534,7 @@ constexpr int64_t fused_limit(int64_t limit, int rule, int A) {
 std::atomic<int64_t> g_fused_edges{kFusedEdgesDefault};
 
 // ext_scratch: caller-provided device scratch for the single-segment pipeline
-// (at least split_scratch_bytes(n_edges, g, arms) bytes); nullptr = the
+// (at least split_scratch_bytes(n_edges, g) bytes); nullptr = the
 // library's stream-ordered pool.
 mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robots, const float *q0,
                            const float *q1, int64_t n_edges, int g, int rule, float range, uint32_t flags,
@@ -578,12 +577,12 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     if (!scratch) {
         cudaMemPool_t pool;
         err = scratch_pool(&pool);
-        if (err == cudaSuccess) err = cudaMallocFromPoolAsync(&scratch, split_scratch_bytes(n_edges, g, A), pool, stream);
+        if (err == cudaSuccess) err = cudaMallocFromPoolAsync(&scratch, split_scratch_bytes(n_edges, g), pool, stream);
     } else {
         err = cudaSuccess;
     }
     if (err == cudaSuccess) {
-        set_split_scratch(p, scratch, n_edges, g, A);
+        set_split_scratch(p, scratch, n_edges, g);
         const int rounds = rule == MRPOP_RULE_PLAIN ? 1 : kSegRounds;
         for (int r = 0; r < rounds && err == cudaSuccess; r++) {
             p.seg0 = r;

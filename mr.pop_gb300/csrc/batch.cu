@@ -174,7 +174,7 @@ mrpop_status mrpop_batch_create(const mrpop_batch_item *items, int64_t n_items, 
         if (it.n_edges == 0) continue;
         e.spl = it.granularity > 32 ? 2 : 1;
         e.seg = it.rule != MRPOP_RULE_PLAIN;
-        e.scratch = (mrpop::split_scratch_bytes(it.n_edges, it.granularity, e.arms) + 255) & ~(size_t)255;
+        e.scratch = (mrpop::split_scratch_bytes(it.n_edges, it.granularity) + 255) & ~(size_t)255;
         scratch_total += e.scratch;
         ent.push_back(e);
     }
@@ -186,7 +186,7 @@ mrpop_status mrpop_batch_create(const mrpop_batch_item *items, int64_t n_items, 
     }
     size_t off = 0;
     for (Entry &e : ent) {
-        mrpop::set_split_scratch(e.p, (char *)b->d_scratch + off, e.p.n_edges, e.p.g, e.arms);
+        mrpop::set_split_scratch(e.p, (char *)b->d_scratch + off, e.p.n_edges, e.p.g);
         off += e.scratch;
     }
     for (int key = 0; key < 4 * MRPOP_MAX_ARMS; key++) {

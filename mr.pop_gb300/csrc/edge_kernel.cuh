@@ -802,7 +802,6 @@ static __device__ __noinline__ double narrow_flops(const EdgeParams &P, int A, u
 // ---------------------------------------------------------------------------
 // narrow phase
 // ---------------------------------------------------------------------------
-// bit r set: detailed self row r is checked for an arm with self flags sm
 // Rows whose first-read sphere is on joint j (quirk: sphere r, else first(r)).
 __host__ __device__ constexpr uint32_t joint_rows(int j, bool quirk) {
     uint32_t m = 0;
@@ -811,6 +810,7 @@ __host__ __device__ constexpr uint32_t joint_rows(int j, bool quirk) {
     return m;
 }
 
+// bit r set: detailed self row r is checked for an arm with self flags sm
 __device__ __forceinline__ uint32_t row_mask(uint32_t sm, bool quirk) {
     uint32_t m = 0;
 #pragma unroll
@@ -828,31 +828,21 @@ constexpr uint32_t forearm_rows() {
 }
 constexpr uint32_t kForearmRows = forearm_rows();
 
-// Row bookkeeping of the detailed self check, per sphere index i:
-//   first[q][i]  rows whose first-read sphere is i (q = 1: the composite
+// Row bookkeeping of the detailed self check:
+//   cover[i]     rows whose target range lo..hi contains sphere i
+//   jfirst[q][j] rows whose first-read sphere is on joint j (q = 1: the composite
 //                robots' reading, sphere r; q = 0: sphere first(r))
-//   cover[i]     rows whose target range lo..hi contains i
-// and the same ORed over the spheres of each joint.
 struct RowTab {
-    uint32_t first[2][kNumDet];
     uint32_t cover[kNumDet];
     uint32_t jfirst[2][kNumJoints];
-    uint32_t jcover[kNumJoints];
 };
 
 __host__ __device__ constexpr RowTab make_row_tab() {
     RowTab t{};
-    for (int r = 0; r < kDetRows; r++) {
-        t.first[0][det_row_first(r)] |= 1u << r;
-        t.first[1][r] |= 1u << r;
+    for (int r = 0; r < kDetRows; r++)
         for (int i = det_row_lo(r); i <= det_row_hi(r); i++) t.cover[i] |= 1u << r;
-    }
-    for (int i = 0; i < kNumDet; i++) {
-        const int j = det_joint(i);
-        t.jfirst[0][j] |= t.first[0][i];
-        t.jfirst[1][j] |= t.first[1][i];
-        t.jcover[j] |= t.cover[i];
-    }
+    for (int q = 0; q < 2; q++)
+        for (int j = 0; j < kNumJoints; j++) t.jfirst[q][j] = joint_rows(j, q != 0);
     return t;
 }
 
@@ -1792,9 +1782,6 @@ __device__ __forceinline__ void connect_advance(EdgeScratch &W, int dof, int seg
     __syncwarp();
 }
 
-// Broad phase of one segment for this lane's samples plus the decision: which
-// samples get the detailed check (the reference's thread split, or every
-// flagged sample in EXACT mode).  Returns false when no sample is flagged.
 // The candidate masks of a segment from its samples' flag counts (totals over
 // the segment given): every flagged sample in EXACT mode, else the samples the
 // reference's proportional 4g-thread split gives at least one thread
@@ -1841,6 +1828,9 @@ __device__ __forceinline__ void thread_split(bool exact, int g, int lane, const 
     }
 }
 
+// Broad phase of one segment for this lane's samples plus the decision: which
+// samples get the detailed check (the reference's thread split, or every
+// flagged sample in EXACT mode).  Returns false when no sample is flagged.
 template <int A, int SPL>
 __device__ __forceinline__ bool broad_decide(const EdgeParams &P, const EdgeScratch &W, BroadPart &B, const float4 *S,
                                              const SceneLayout &L, int seg, int g, int lane, Flags<A> (&envw)[SPL],
@@ -2018,9 +2008,9 @@ struct PairShare {
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
 template <int A>
-__device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch &W, const float4 *S, const SceneLayout &L, const float4 *det_tab,
-                                                long long e, int dof, int g, int lane, int half, PairShare &X,
-                                                int bar_id, bool staged) {
+__device__ __forceinline__ void fused_edge_pair(const EdgeParams &P, WarpScratch &W, const float4 *S,
+                                                const SceneLayout &L, const float4 *det_tab, long long e, int dof, int g,
+                                                int lane, int half, PairShare &X, int bar_id, bool staged) {
     if (!staged) {
         if (half == 0 && lane == 0) {
             P.valid[e] = 0;
@@ -2119,11 +2109,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, MRPOP_MIN_BLOCKS)
 }
 
 // ---------------------------------------------------------------------------
-// fused kernel, one warp per arm (small calls of 2 to 5 arms): a CTA of A
+// fused kernel, one warp per arm (small calls of 3 to 5 arms): a CTA of A
 // warps takes one edge at a time and warp a does arm a's share of it -- its
 // forward kinematics, env and intra-arm screens and exact tests, its detailed
-// chain walk -- and every A-th arm pair of the arm-vs-arm screens and tests,
-// each over every slot of the segment.  Flag words are ORed together in
+// chain walk -- over every slot of the segment; the arm pairs of the arm-vs-arm
+// screens and tests go to whichever warp is free.  Flag words are ORed together in
 // shared memory, the thread split is evaluated from them by every warp (the
 // same integers), and a sample collides when any warp's tests fire: the
 // verdicts are those of the one-warp kernels.  The lower arm's spheres of a
@@ -2416,8 +2406,8 @@ __device__ __forceinline__ void broad_edge(const EdgeParams &P, BroadScratch &W,
 }
 
 // The detailed phase of edge e.  One arm, and composite calls of a middle size:
-// all of it (kStageAll), in one kernel.  Larger composite calls: the obstacles and arm pairs (STAGE kStageEnvPairs, narrow_kernel),
-// then the intra-arm rows (kStageRows, rows_kernel) of the samples below the
+// all of it (kStageAll), in one kernel.  Larger composite calls: the obstacles and
+// arm pairs (STAGE kStageEnvPairs, narrow_kernel), then the intra-arm rows (kStageRows, rows_kernel) of the samples below the
 // first hit; between the two P.smasks[2 * e] says whether a sample has hit and
 // P.smasks[2 * e + 1] which samples are left.
 template <int A, int SPL, bool SEG, int STAGE>
@@ -2645,7 +2635,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, batch_min_blocks(MODE))
             const long long e = (long long)ch.y + k;
             if constexpr (MODE == kBatchBroad) broad_edge<A, SPL, SEG>(P, W, S, L, e, dof, P.g, lane, staged);
             else if constexpr (MODE == kBatchNarrow || MODE == kBatchNarrowAll)
-                narrow_edge<A, SPL, SEG, A == 1 || MODE == kBatchNarrowAll ? kStageAll : kStageEnvPairs>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
+                narrow_edge<A, SPL, SEG, A == 1 || MODE == kBatchNarrowAll ? kStageAll : kStageEnvPairs>(
+                    P, W, S, L, det_tab, e, dof, P.g, lane, staged);
             else if constexpr (MODE == kBatchRows)
                 narrow_edge<A, SPL, SEG, kStageRows>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
             else fused_edge<A, SPL>(P, W, S, L, det_tab, e, dof, P.g, lane, staged);
@@ -2658,7 +2649,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, batch_min_blocks(MODE))
 // launch's counter, stages each instance's parameters and scene as
 // batch_kernel does, and runs the arm-per-warp body on every edge of the chunk.
 template <int A, int SPL>
-__global__ void __launch_bounds__(32 * A, armwise_min_blocks(A)) batch_armwise_kernel(const __grid_constant__ BatchParams B) {
+__global__ void __launch_bounds__(32 * A, armwise_min_blocks(A))
+    batch_armwise_kernel(const __grid_constant__ BatchParams B) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ float4 det_tab[kNumDet];

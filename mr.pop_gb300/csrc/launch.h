@@ -71,12 +71,12 @@ size_t warp_scratch_bytes();
 // masks, kPairSlots arm-pair words and the segment state.
 constexpr size_t kSplitScratchHead = 128;
 constexpr int kPairSlots = 2 * num_pairs(kMaxArms);
-constexpr size_t split_scratch_bytes(int64_t n_edges, int g, [[maybe_unused]] int A) {
+constexpr size_t split_scratch_bytes(int64_t n_edges, int g) {
     return kSplitScratchHead +
            (size_t)n_edges * (32 * (g > 32 ? 2 : 1) * 2 * sizeof(uint64_t) + 2 * sizeof(uint64_t) +
                               kPairSlots * sizeof(uint16_t) + 2 * sizeof(int32_t));
 }
-void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g, int A);
+void set_split_scratch(EdgeParams &p, void *scratch, int64_t n_edges, int g);
 
 // Largest calls whose narrow phase is one kernel (kNarrowAll) instead of
 // kNarrow and kRows.  Up to some edges per resident warp each kernel of a round

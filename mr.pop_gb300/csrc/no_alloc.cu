@@ -6,16 +6,20 @@
 // whole device-memory budget when it starts and admits work against it (an
 // allocation inside a call could fail, or change the budget it accounts for),
 // or a planner loop that must not enter the allocator while it runs.  This file
-// gives them mrpop_validate_edges_noalloc, which runs the same two kernels with
-// their scratch in a fixed array that lives in the library's own device memory.
+// gives them mrpop_validate_edges_noalloc, which runs the same kernels (a fused one
+// without scratch for a small call, else the split ones) with their scratch in a
+// fixed array that lives in the library's own device memory.
 //
 // The array: kNoAllocBytes bytes per device (MRPOP_NOALLOC_MAX_EDGES edges at
 // the largest granularity), held by every GPU that loads the library until
 // the process exits.  Every call uses the same array, so calls that overlap on
 // the GPU (for example on two streams at once) race on it and must be ordered
 // by the caller.  The array keeps the previous call's contents; nothing in it
-// needs to start at zero, because each call's first kernel writes every word of
-// scratch that its second kernel reads.
+// needs to start at zero: the work counters are zeroed in stream order, the broad
+// kernel writes every edge's candidate masks, and the flag words and arm-pair
+// joints of every edge with a candidate, which are all that the narrow kernel
+// reads; that one rewrites the masks that the rows kernel reads, but of edges that
+// need no narrow test, whose masks stay the broad kernel's.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -25,9 +29,9 @@
 namespace {
 
 // The scratch of the largest call allowed: MRPOP_NOALLOC_MAX_EDGES edges at
-// granularity 64 with 5 arms (the same size function the pool path uses).
-constexpr size_t kNoAllocBytes = mrpop::split_scratch_bytes(MRPOP_NOALLOC_MAX_EDGES, 64, mrpop::kMaxArms);
-static_assert(kNoAllocBytes >= mrpop::split_scratch_bytes(MRPOP_NOALLOC_MAX_EDGES, 32, mrpop::kMaxArms),
+// granularity 64, any arm count (the same size function the pool path uses).
+constexpr size_t kNoAllocBytes = mrpop::split_scratch_bytes(MRPOP_NOALLOC_MAX_EDGES, 64);
+static_assert(kNoAllocBytes >= mrpop::split_scratch_bytes(MRPOP_NOALLOC_MAX_EDGES, 32),
               "the array must hold the largest call at every granularity");
 
 // Host code must not use this name as a device address (on the host it is only

@@ -526,7 +526,7 @@ mrpop_status mrpop_session_open(mrpop_server *s, int arms, int64_t max_edges, in
     // scratch of max_edges edges at the largest arm count and granularity, and
     // room for the per-item header and alignment of a multi-item submission
     const size_t bytes =
-        round_up(mrpop::split_scratch_bytes(max_edges, max_granularity, arms) + 2 * MRPOP_SESSION_MAX_ITEMS * kAlign);
+        round_up(mrpop::split_scratch_bytes(max_edges, max_granularity) + 2 * MRPOP_SESSION_MAX_ITEMS * kAlign);
     const size_t qbytes = round_up((size_t)max_edges * 7 * arms * sizeof(float));
     const size_t host_bytes = 2 * qbytes + round_up((size_t)max_edges) + round_up((size_t)max_edges * sizeof(int32_t));
     if ((int64_t)bytes > s->stats.budget_bytes || host_bytes > round_up((size_t)s->cfg.host_bytes))
@@ -593,14 +593,14 @@ mrpop_status mrpop_session_submit_many(mrpop_session *ss, const mrpop_batch_item
             return fail(MRPOP_ERR_INVALID_ARGUMENT, "session_submit: step larger than the session was opened for");
         edges += it->n_edges;
         if (it->n_edges == 0) continue;
-        const size_t need = mrpop::split_scratch_bytes(it->n_edges, it->granularity, A);
+        const size_t need = mrpop::split_scratch_bytes(it->n_edges, it->granularity);
         if (off + need > ss->bytes)
             return fail(MRPOP_ERR_INVALID_ARGUMENT, "session_submit: the steps' scratch exceeds the session's");
         st.arms = A;
         st.spl = it->granularity > 32 ? 2 : 1;
         st.seg = it->rule != MRPOP_RULE_PLAIN;
         st.n_chunks = (int)((it->n_edges + kChunkEdges - 1) / kChunkEdges);
-        mrpop::set_split_scratch(st.p, s->d_arena + ss->offset + off, it->n_edges, it->granularity, A);
+        mrpop::set_split_scratch(st.p, s->d_arena + ss->offset + off, it->n_edges, it->granularity);
         off = round_up(off + need);
         n_steps++;
     }
