@@ -132,7 +132,7 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots);
  * mrpop_set_fused_edges sets the limit of every call of the process (-1: every
  * call split) and returns the previous one.  0, or 2048, is the default: 2048
  * edges, and for segmented calls (mrpop_validate_segments), whose split form has
- * more launches, 5120 edges up to 3 arms, 4096 of 4 arms, 3072 of 5.
+ * more launches, 5120 edges, 4096 with 5 arms.
  */
 int64_t mrpop_set_fused_edges(int64_t max_edges);
 mrpop_status mrpop_validate_edges(const mrpop_scene *scene, const mrpop_robotset *robots,

@@ -515,18 +515,18 @@ constexpr int64_t kFusedEdgesDefault = 2048;
 
 // The default limit of segmented calls: the split pipeline runs 4 rounds of two or
 // three launches and a fused tail, each as long as its slowest edge, so one
-// fused launch is the faster form up to one to two edges per resident warp, the
-// fewer the more arms (an edge's warp walks them all).  Whole calls, split against
-// fused in us: 3 arms x 24 B-spline 2800 edges 609 / 250, 4096 569 / 422, 8000
-// 641 / 750; 4 arms x 32 connect, mixed cell, 3500 441 / 393, 4100 465 / 468, 5100
-// 480 / 557, bin table 560 / 475, 546 / 408, 598 / 501; 5 arms x 32 connect, mixed
-// cell, 2600 574 / 452, 3072 619 / 568, 4100 666 / 747, shelf 385 / 336, 434 /
-// 448, 450 / 549; 5 arms x 64, mixed cell, 3072 917 / 676, 5100 1090 / 1046,
-// shelf 571 / 526, 682 / 784.
+// fused launch is the faster form up to about two edges per resident warp, fewer
+// with 5 arms (an edge's warp walks them all) and where few edges collide early.
+// Whole calls, split against fused in us: 3 arms x 24 B-spline 2800 edges 609 /
+// 250, 4096 569 / 422, 8000 641 / 750; 4 arms x 32 connect, mixed cell, 3500 441 /
+// 393, 4100 465 / 468, 5100 480 / 557, bin table 560 / 475, 546 / 408, 598 / 501;
+// 5 arms x 32 connect, mixed cell, 2600 574 / 452, 4100 666 / 747, 5100 702 / 834,
+// shelf 385 / 336, 450 / 549, 505 / 735; 5 arms x 64, mixed cell, 4100 989 / 863,
+// 5100 1090 / 1046, shelf 646 / 646, 682 / 784.
 // (Single-segment calls, 4 arms x 32: 2000 edges 171 / 207, 2800 224 / 191,
 // 4096 240 / 322; 5 arms x 64: 2000 327 / 246, 4096 395 / 463.)  A limit set by
 // the caller holds for every call.
-constexpr int64_t fused_segment_edges(int A) { return A <= 3 ? 5120 : A == 4 ? 4096 : 3072; }
+constexpr int64_t fused_segment_edges(int A) { return A <= 4 ? 5120 : 4096; }
 constexpr int64_t fused_limit(int64_t limit, int rule, int A) {
     return limit == kFusedEdgesDefault && rule != MRPOP_RULE_PLAIN ? fused_segment_edges(A) : limit;
 }

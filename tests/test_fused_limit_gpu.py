@@ -52,7 +52,7 @@ def test_default_limits(cuda, pkg, setting):
         assert lib.mrpop_set_fused_edges(prev) == 2048
 
 
-@pytest.mark.parametrize("arms,limit", [(1, 5120), (3, 5120), (4, 4096), (5, 3072)])
+@pytest.mark.parametrize("arms,limit", [(1, 5120), (3, 5120), (4, 5120), (5, 4096)])
 def test_default_limit_of_segmented_calls_by_arms(cuda, pkg, arms, limit):
     lib = pkg.library()
     prev = lib.mrpop_set_fused_edges(0)
