@@ -131,8 +131,9 @@ mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots);
  * the staging that dominate small calls.  Verdicts are the same either way.
  * mrpop_set_fused_edges sets the limit of every call of the process (-1: every
  * call split) and returns the previous one.  0, or 2048, is the default: 2048
- * edges, and for segmented calls (mrpop_validate_segments), whose split form has
- * more launches, 5120 edges, 4096 with 5 arms.
+ * edges (at up to 32 samples 1280 with 4 arms and 512 with 5), and for segmented
+ * calls (mrpop_validate_segments), whose split form has more launches, 5120 edges,
+ * 4096 with 5 arms.
  */
 int64_t mrpop_set_fused_edges(int64_t max_edges);
 mrpop_status mrpop_validate_edges(const mrpop_scene *scene, const mrpop_robotset *robots,

@@ -523,12 +523,23 @@ constexpr int64_t kFusedEdgesDefault = 2048;
 // 5 arms x 32 connect, mixed cell, 2600 574 / 452, 4100 666 / 747, 5100 702 / 834,
 // shelf 385 / 336, 450 / 549, 505 / 735; 5 arms x 64, mixed cell, 4100 989 / 863,
 // 5100 1090 / 1046, shelf 646 / 646, 682 / 784.
-// (Single-segment calls, 4 arms x 32: 2000 edges 171 / 207, 2800 224 / 191,
-// 4096 240 / 322; 5 arms x 64: 2000 327 / 246, 4096 395 / 463.)  A limit set by
-// the caller holds for every call.
 constexpr int64_t fused_segment_edges(int A) { return A <= 4 ? 5120 : 4096; }
-constexpr int64_t fused_limit(int64_t limit, int rule, int A) {
-    return limit == kFusedEdgesDefault && rule != MRPOP_RULE_PLAIN ? fused_segment_edges(A) : limit;
+
+// The default limit of single-segment calls: two launches, each with code that the
+// instruction cache holds, against one.  Above 32 samples the fused form has two
+// warps an edge and wins throughout (5 arms x 64: 2048 edges 129 / 118 to 288 /
+// 254); up to 32, with one warp an edge, the more arms the earlier the split form
+// (4 arms x 32: 700 edges 97 / 96, 87 / 96 and 128 / 123 on three scenes, 2048
+// 128 / 130, 126 / 150, 130 / 150; 5 arms x 32: 700 92 / 101, 152 / 166, 153 / 168,
+// 2048 102 / 128, 182 / 217, 170 / 194; 3 arms 2048 94 / 103, 90 / 94, 108 / 94).
+// Calls whose edges all have resident CTAs (456 edges of 5 arms, 608 of 4) run one
+// warp per arm.
+constexpr int64_t fused_plain_edges(int A, int g) { return g > 32 || A <= 3 ? kFusedEdgesDefault : A == 4 ? 1280 : 512; }
+
+// A limit set by the caller holds for every call.
+constexpr int64_t fused_limit(int64_t limit, int rule, int A, int g) {
+    if (limit != kFusedEdgesDefault) return limit;
+    return rule != MRPOP_RULE_PLAIN ? fused_segment_edges(A) : fused_plain_edges(A, g);
 }
 
 std::atomic<int64_t> g_fused_edges{kFusedEdgesDefault};
@@ -560,7 +571,7 @@ mrpop_status run_validator(const mrpop_scene *scene, const mrpop_robotset *robot
     // more arms one warp per arm, else above 32 samples per segment two warps
     // per edge (one per 32-sample slot), unless the flop tally is wanted
     cudaError_t err;
-    if (n_edges <= fused_limit(g_fused_edges.load(std::memory_order_relaxed), rule, A)) {
+    if (n_edges <= fused_limit(g_fused_edges.load(std::memory_order_relaxed), rule, A, g)) {
         p.seg0 = 0;
         err = timed_launch(A, flops ? kFused : A >= 3 ? kArmwise : g > 32 ? kFusedPair : kFused, p, smem, stream);
         if (tmp_valid) cudaFreeAsync(tmp_valid, stream);
