@@ -319,7 +319,8 @@ mrpop_status mrpop_batch_destroy(mrpop_batch *batch);
  * A session also reserves page-locked host buffers for its steps in a host
  * arena of host_bytes (mrpop_session_host_buffers).  Zero in a config field
  * selects the default: 1 GiB, 4 streams, 1024 steps, 16384 chunks, 256 MiB,
- * 4096 fused edges.
+ * 4096 fused edges (2048 in groups of 3 to 5 arms whose steps have one segment,
+ * 3072 in segmented ones of 5 arms).
  */
 typedef struct {
     int64_t budget_bytes;    /* device arena for the sessions' step scratch            */

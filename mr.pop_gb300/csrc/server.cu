@@ -42,12 +42,20 @@ constexpr int kChunkEdges = 96;    // largest chunk (the batch entry points' chu
 // dozen edges then spreads over several CTAs instead of running through one
 // CTA's warps in turn.
 constexpr int kWaveCtasPerSm = 3;
-// Groups of at most this many edges in a wave (mrpop_server_config.fused_edges)
-// run as one fused launch -- broad and narrow phase per edge in one warp, from
+// Groups of at most this many edges in a wave (mrpop_server_config.fused_edges, if
+// set) run as one fused launch -- broad and narrow phase per edge in one warp, from
 // segment 0 -- instead of the split kernels (1 launch instead of 2, or of
 // 2 * kSegRounds + 1 for segmented rules): launch latency and the serial
-// dependency between the split kernels dominate small waves.
+// dependency between the split kernels dominate small waves.  Groups of 3 to 5 arms
+// whose steps have one segment split earlier: a step of 3 arms x 32, fused against
+// split, 2000 edges 186 / 217 us, 3000 194 / 170, 4000 305 / 245; 4 arms 219 / 211,
+// 247 / 205, 322 / 238; 5 arms 183 / 176, 271 / 219, 350 / 256.  5 arms' segmented
+// steps too: 3000 edges 275 / 292, 4000 370 / 329 (4 arms 4000 474 / 598).
 constexpr int64_t kFusedEdgesDefault = 4096;
+int64_t wave_fused_edges(int64_t set, int arms, bool seg) {
+    if (set != 0) return set;
+    return arms >= 3 && !seg ? 2048 : arms == 5 ? 3072 : kFusedEdgesDefault;
+}
 // Groups of 3 to 5 arms with at most this many edges in a wave run the
 // arm-per-warp kernel (a CTA of A warps per edge; about as many edges as its
 // CTAs resident on the device at 5 arms).
@@ -255,7 +263,8 @@ cudaError_t launch_wave(mrpop_server *s, mrpop_server::Slot &slot) {
         left -= at_chunk;
         // a small group of 3 to 5 arms runs one warp per arm, one edge per
         // CTA: its chunks are single edges, if the table has room for them
-        r.armwise = arms >= 3 && edges <= kArmwiseEdges && edges <= s->cfg.fused_edges &&
+        const int64_t fused = wave_fused_edges(s->cfg.fused_edges, arms, seg);
+        r.armwise = arms >= 3 && edges <= kArmwiseEdges && edges <= fused &&
                     nc + edges + left <= s->cfg.max_wave_chunks;
         const int cs = r.armwise ? 1 : chunk;
         for (const auto &st : slot.steps) {
@@ -288,7 +297,7 @@ cudaError_t launch_wave(mrpop_server *s, mrpop_server::Slot &slot) {
             err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchArmwise, 0, items, chunks, r.nc, work, slot.stream);
             continue;
         }
-        if (r.edges <= s->cfg.fused_edges) {
+        if (r.edges <= wave_fused_edges(s->cfg.fused_edges, arms, seg)) {
             err = launch_one(s, arms, seg, spl, r.smem, mrpop::kBatchFused, 0, items, chunks, r.nc, work, slot.stream);
             continue;
         }
@@ -453,7 +462,6 @@ mrpop_status mrpop_server_create(const mrpop_server_config *cfg, mrpop_server **
     if (c.max_wave_steps <= 0) c.max_wave_steps = 1024;
     if (c.max_wave_chunks <= 0) c.max_wave_chunks = 16384;
     if (c.host_bytes <= 0) c.host_bytes = (int64_t)256 << 20;
-    if (c.fused_edges == 0) c.fused_edges = kFusedEdgesDefault;
     if (c.streams > 16 || c.max_wave_steps > (1 << 20) || c.max_wave_chunks > (1 << 24))
         return fail(MRPOP_ERR_INVALID_ARGUMENT, "server_create: streams <= 16, max_wave_steps <= 2^20, "
                                                 "max_wave_chunks <= 2^24");

@@ -29,3 +29,24 @@ def test_steps_around_the_limit(cuda, pkg, rule, g, n):
         assert np.array_equal(x, out[0].cpu().numpy())
         assert np.array_equal(y, out[1].cpu().numpy())
     assert scene.status() == 0
+
+
+@pytest.mark.parametrize("arms,rule,limit", [(1, 0, 4096), (2, 0, 4096), (3, 0, 2048), (5, 0, 2048), (4, 2, 4096),
+                                             (5, 3, 3072)])
+def test_default_limit_of_fused_groups(cuda, pkg, arms, rule, limit):
+    """A wave of one fused group is one launch; above the limit, or above one set, it is several."""
+    W = pkg.workloads
+    bases = W.bases_facing_centre(arms, 0.71)
+    q0, q1 = W.random_edges(np.random.default_rng(limit), limit + 1, arms, 2.0)
+    scene, robots = pkg.Scene(W.scene_config2(3)), pkg.RobotSet(arms, bases)
+    for setting in (0, 1000):
+        server = pkg.Server(budget_bytes=256 << 20, streams=1, fused_edges=setting)
+        sess = server.session(arms, limit + 1, 8)
+        bound, launches = setting or limit, []
+        for n in (bound, bound + 1):
+            before = server.stats()["kernel_launches"]
+            sess.validate(scene, robots, q0[:n], q1[:n], 8, rule=rule, range_=1.0 if rule else 0.0)
+            launches.append(server.stats()["kernel_launches"] - before)
+        sess.close()
+        server.close()
+        assert launches[0] == 1 and launches[1] > 1
