@@ -2545,13 +2545,14 @@ constexpr int kBatchRows = 4;
 // kBatchNarrow and kBatchRows in one kernel (service waves).
 constexpr int kBatchNarrowAll = 5;
 
-// CTAs per SM of the batch kernels.  The fused ones, whose groups are small (a
-// wave's, or the edges that segment rounds leave), are built for 2: at 3, their
-// 96 registers spill 112 bytes at 64 samples.  Whole wave of fused steps, 3
+// CTAs per SM of the batch kernels.  The fused composite ones, whose groups are
+// small (a wave's, or the edges that segment rounds leave), are built for 2: at 3,
+// their 96 registers spill 112 bytes at 64 samples.  Whole wave of fused steps, 3
 // against 2: 2 arms x 64 connect, 300 edges 192 -> 169 us on the device, 3000 351
-// -> 309; 3 arms x 64 connect, 3000 edges 471 -> 401.
-constexpr int batch_min_blocks(int mode) {
-    return mode == kBatchBroad ? kBroadMinBlocks : mode == kBatchFused ? 2 : MRPOP_MIN_BLOCKS;
+// -> 309; 3 arms x 64 connect, 3000 edges 471 -> 401; one arm, which does not
+// spill, 4000 x 64 79 -> 101.
+constexpr int batch_min_blocks(int arms, int mode) {
+    return mode == kBatchBroad ? kBroadMinBlocks : mode == kBatchFused && arms > 1 ? 2 : MRPOP_MIN_BLOCKS;
 }
 
 // One bulk copy of `bytes` from global to shared memory, completed on `bar`
@@ -2575,7 +2576,7 @@ __device__ __forceinline__ bool stage_bulk(float4 *dst, const float4 *src, uint3
 }
 
 template <int A, int SPL, int MODE, bool SEG>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, batch_min_blocks(MODE))
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, batch_min_blocks(A, MODE))
     batch_kernel(const __grid_constant__ BatchParams B) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
