@@ -111,7 +111,9 @@ mrpop_status mrpop_scene_status(const mrpop_scene *scene, uint32_t *status_out);
  * (panda.cuh:78-83), quad_franka_base_transform for 4 (panda.cuh:16-40 ==
  * panda_four.cuh:17-41), five_franka_base_transform for 5 (panda.cuh:42-73 ==
  * panda_five.cuh:17-46).  The arms are Franka Pandas with the reference's
- * sphere model (panda_multi_geometry.cuh). */
+ * sphere model (panda_multi_geometry.cuh).  Any frame is taken: sphere centres
+ * follow it and radii do not, as in the reference; frames that are not rigid
+ * transforms within 100 m of the origin make checks slower (wider screens). */
 mrpop_status mrpop_robotset_create(int n_arms, const float *base_T, mrpop_robotset **out);
 mrpop_status mrpop_robotset_destroy(mrpop_robotset *robots);
 
